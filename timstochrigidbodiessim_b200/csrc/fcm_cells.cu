@@ -173,6 +173,35 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_chunks(const int* __restrict__ 
   }
 }
 
+// One launch for inputs of a few chunks: every CTA sums the entries before its
+// chunk itself (at most 8 x 8192 of them, from L2), then scans its chunk.  The
+// 32,768 tile counts of a 256^3 grid took 15.4 us in the three launches above
+// (most of it launches of one to four CTAs).
+constexpr int SCAN_DIRECT = 8 * SCAN_CH;
+__global__ void __launch_bounds__(SCAN_T) k_scan_direct(const int* __restrict__ in, int* __restrict__ out, int n) {
+  __shared__ int warp_sums[32];
+  const int c0 = blockIdx.x * SCAN_CH;
+  int before = 0;
+  for (int i = threadIdx.x; i < c0; i += SCAN_T) before += in[i];
+  const int i0 = c0 + threadIdx.x * SCAN_IPT;
+  int v[SCAN_IPT], tot = 0;
+#pragma unroll
+  for (int k = 0; k < SCAN_IPT; ++k) {
+    v[k] = (i0 + k < n) ? in[i0 + k] : 0;
+    tot += v[k];
+  }
+  int offset = 0, total = 0;
+  block_exclusive(before, warp_sums, &offset);
+  __syncthreads();  // warp_sums is used again
+  int run = offset + block_exclusive(tot, warp_sums, &total);
+#pragma unroll
+  for (int k = 0; k < SCAN_IPT; ++k) {
+    if (i0 + k < n) out[i0 + k] = run;
+    run += v[k];
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = offset + total;
+}
+
 __global__ void k_cell_scatter(const int* __restrict__ cell, int Nb, int ncell, const int* __restrict__ start,
                                int* __restrict__ cursor, int* __restrict__ sorted) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -447,6 +476,11 @@ int launch_exclusive_scan(const int* in, int* out, int n, cudaStream_t s) {
     return FCM_OK;
   }
   const int nchunks = (n + SCAN_CH - 1) / SCAN_CH;
+  if (n <= SCAN_DIRECT) {
+    k_scan_direct<<<nchunks, SCAN_T, 0, s>>>(in, out, n);
+    FCM_LAUNCH_CHECK();
+    return FCM_OK;
+  }
   k_scan_chunk_sums<<<nchunks, SCAN_T, 0, s>>>(in, out, n);
   FCM_LAUNCH_CHECK();
   k_scan_chunk_offsets<<<1, SCAN_T, 0, s>>>(out, n, nchunks);

@@ -160,7 +160,6 @@ struct BlobTable {
   T* wc = nullptr;                // [n][3][4][8] weights on the 8-aligned grid chunks a stencil meets
   int* tile_count = nullptr;      // [ntiles]
   int* tile_offset = nullptr;     // [ntiles+1] exclusive offsets
-  int* tile_cursor = nullptr;     // [ntiles]
   unsigned long long* tile_list = nullptr;  // [cap] (blob << 32) | chunk indices, j and half masks
   long long tile_cap = 0;
   T* partial = nullptr;           // [n][64][3] per-(blob, tile) interpolation partials
