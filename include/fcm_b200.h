@@ -298,7 +298,7 @@ int fcm_interp(fcm_ctx* ctx, int32_t precision, double* V);
 /* Kernel variants of the grid stages (no reference counterpart).
  * variants[FCM_NUM_VARIANTS]:
  *   [0] FP64 spread, [2] FP32 spread: 0 = the persistent software-pipelined tile
- *       kernel, 1 / 2 / 3 = one CTA per 8^3 tile staging 16 / 8 / 32 blobs per
+ *       kernel (FP64: by one warp on the FP64 tensor cores, FP32: FMAs), 1 / 2 / 3 = one CTA per 8^3 tile staging 16 / 8 / 32 blobs per
  *       round, 4 = one warp per tile staging 16 blobs per round, two y-rows per
  *       lane.  All sum every grid point's blobs in the same order with the same
  *       products, so the grids are the same bit for bit.  FP32 only: 5 = one warp
@@ -310,8 +310,9 @@ int fcm_interp(fcm_ctx* ctx, int32_t precision, double* V);
  *       (FP32 only).  FP64 defaults to 0 beyond 256 points along x.  The solves
  *       agree within rounding.
  *   [4] FP64 interpolation, [5] FP32 interpolation: 0 = 64 threads per 8^3 tile
- *       with a warp shuffle reduction, 1 = one warp per tile (two y-rows per
- *       lane, added in the lane) with the shuffle reduction, 2 = one warp per tile
+ *       with a warp shuffle reduction, 1 = one warp per tile (FP64: on the FP64
+ *       tensor cores; FP32: two y-rows per lane, added in the lane, with the shuffle
+ *       reduction), 2 = one warp per tile
  *       (two y-rows per thread) with a shared-memory reduction; FP32 only: 3 = one
  *       warp per tile on the tensor cores (3xTF32).  They agree within rounding.
  * Defaults: spread 0 (FP64) and 4 (FP32), solve 1 (FP64 up to 256 points along

@@ -585,12 +585,13 @@ __global__ void __launch_bounds__(32) k_spread_warp(const T* __restrict__ wc, co
 
 // ------------------------------------------------------------------ persistent pipelined tiles
 // Work items of a persistent CTA: its tiles blockIdx.x, +gridDim.x, ..., each cut
-// into staging rounds of SCB blobs (one empty round for a tile without blobs).
+// into staging rounds of RB blobs (one empty round for a tile without blobs).
 // The tile offsets are loaded two tiles ahead, so the generator never waits.
 struct TileItem {
   int tile, c0, nc, last;
 };
 
+template <int RB = SCB>
 struct ItemGen {
   const int* __restrict__ offset;
   int ntiles, stride;
@@ -615,8 +616,8 @@ struct ItemGen {
     return true;
   }
   __device__ __forceinline__ bool next() {
-    if (c0 + SCB < b1) {
-      c0 += SCB;
+    if (c0 + RB < b1) {
+      c0 += RB;
       return true;
     }
     tile += stride;
@@ -629,7 +630,7 @@ struct ItemGen {
     return true;
   }
   __device__ __forceinline__ TileItem item() const {
-    return TileItem{tile, c0, min(SCB, b1 - c0), (c0 + SCB >= b1) ? 1 : 0};
+    return TileItem{tile, c0, min(RB, b1 - c0), (c0 + RB >= b1) ? 1 : 0};
   }
 };
 
@@ -665,7 +666,7 @@ __global__ void __launch_bounds__(64) k_spread_pipe(const T* __restrict__ wc, co
   __shared__ unsigned sflag[2][SCB];
   const int t = threadIdx.x, k = t >> 2, d = t & 3;
   const int z = t & 7, y = t >> 3, yh = t >> 5;
-  ItemGen gen{offset, ntiles, (int)gridDim.x, 0, 0, 0, 0, 0, 0, 0};
+  ItemGen<> gen{offset, ntiles, (int)gridDim.x, 0, 0, 0, 0, 0, 0, 0};
   if (!gen.first()) return;  // uniform over the CTA
   TileItem cur = gen.item();
   bool v1 = gen.next();
@@ -1386,7 +1387,7 @@ __global__ void __launch_bounds__(32) k_interp_mma(const float* __restrict__ wc,
   __shared__ __align__(16) float sw[2][SCB][3][TE];
   __shared__ unsigned sflag[2][SCB], sblob[2][SCB];
   __shared__ __align__(16) float sg[2][3 * TE * SGX];
-  ItemGen gen{offset, ntiles, (int)gridDim.x, 0, 0, 0, 0, 0, 0, 0};
+  ItemGen<> gen{offset, ntiles, (int)gridDim.x, 0, 0, 0, 0, 0, 0, 0};
   if (!gen.first()) return;  // uniform over the warp
   TileItem cur = gen.item();
   grid_tile_async(grid, g, G, cur.tile, sg[0]);
@@ -1501,6 +1502,290 @@ __global__ void __launch_bounds__(32) k_interp_mma(const float* __restrict__ wc,
     v1 = v2;
     nx2 = nx3;
     v2 = v3;
+    buf ^= 1;
+  }
+  cp_async_wait_all();  // no copy outlives the kernel
+}
+
+// ------------------------------------------------------------------ tensor-core tiles (FP64 grids)
+// FP64 spreading and interpolation of one 8x8x8 tile by one warp with the FP64
+// mma.sync m8n8k4.  It runs at the rate of the FP64 FMA units (18.4 TFMA/s measured,
+// against 16.0 for plain FMAs) and sums its products in ascending k with one FMA
+// rounding each (checked against a chain of fma), so nothing is lost in precision;
+// what it saves is everything around the FMAs.  The FMA kernels issued an operand load
+// for every few FMAs and, in the interpolation, a 16-value shuffle reduction per four
+// blobs; here one instruction does 256 FMAs on operands in registers.
+// Both are bound by the FP64 pipe: 1536 FMAs per (blob, tile) pair, at 512^3 cluster
+// density (15.1M pairs) 1.27 ms at the measured rate, plus the operand products.
+//
+// Fragments of m8n8k4 (g = lane / 4, t = lane % 4): A (8 x 4) a (g, t); B (4 x 8)
+// b (t, g); C (8 x 8) c0 (g, 2t), c1 (g, 2t + 1).
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// Copies of 16 or 8 bytes that fill with zeros instead of reading when !live.
+__device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_addr(dst)), "l"(src), "r"(live ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async8_or_zero(void* dst, const void* src, bool live) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_addr(dst)), "l"(src), "r"(live ? 8 : 0)
+               : "memory");
+}
+
+// A staged blob: its three 8-weight chunks, rows padded to 28 doubles so that the
+// fragment reads (four blobs, eight weights) fall in different banks.
+constexpr int SBL = 28;
+
+// Part d (0-2: weight chunk d; 3: the force, if given) of one list entry to shared
+// memory; a slot past the round's blobs (!live) becomes zeros, which add nothing.
+__device__ __forceinline__ void stage_part64(double* sw, double* sF, const double* __restrict__ wc,
+                                             const double* __restrict__ F, unsigned long long e, int d, bool live) {
+  const unsigned b = (unsigned)(e >> 32), lo = (unsigned)e;
+  if (d < 3) {
+    const double* src = wc + (live ? ((size_t)(3 * b + d) * NCH + ((lo >> (2 * d)) & 3u)) * TE : 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cp_async16_or_zero(sw + d * TE + 2 * i, src + 2 * i, live);
+  } else if (sF) {
+    const double* src = F + (live ? 3 * (size_t)b : 0);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) cp_async8_or_zero(sF + i, src + i, live);
+  }
+}
+
+// Spreading: C[(c, y, z), x] = sum over blobs k of (F_kc wy_k[y] wz_k[z]) wx_k[x], 24
+// fragments (c, y) of 8 z by 8 x in registers, four blobs per k-step.  Every grid
+// point adds the products of k_spread_tiled in the same order, so the grids are the
+// same bit for bit.  Persistent: the next round's chunks are copied while this round's
+// k-steps run, the entries of the one after are being loaded, across tiles.
+// 24 MMAs (16 cycles each on a quarter SM) bound a k-step; with the 32 operand products
+// the loop alone measured 21 cycles per MMA (the products share the FP64 path), the
+// kernel 24 (283 us at 256^3 with 57.7 blobs per tile, 2048 rods 111 us; the 64-thread
+// pipelined FMA kernel took 362 and 126 us).  Two warps per tile (a y-half each, twice
+// the warps per SM) measured level, so the chip is not short of warps here.
+__global__ void __launch_bounds__(32) k_spread_mma64(const double* __restrict__ wc, const double* __restrict__ F,
+                                                     TileGeom g, const int* __restrict__ offset,
+                                                     const unsigned long long* __restrict__ list, long long G,
+                                                     double* __restrict__ grid, int ntiles) {
+  constexpr int RB = 8;
+  __shared__ __align__(16) double sw[2][RB * SBL];
+  __shared__ __align__(16) double sF[2][RB][3];
+  const int lane = threadIdx.x, gq = lane >> 2, tq = lane & 3;
+  ItemGen<RB> gen{offset, ntiles, (int)gridDim.x, 0, 0, 0, 0, 0, 0, 0};
+  if (!gen.first()) return;  // uniform over the warp
+  TileItem cur = gen.item();
+  bool v1 = gen.next();
+  TileItem nx1 = v1 ? gen.item() : TileItem{0, 0, 0, 0};
+  auto entry = [&](const TileItem& it) { return gq < it.nc ? list_entry(list, it.c0 + gq, g) : 0ull; };
+  stage_part64(sw[0] + gq * SBL, sF[0][gq], wc, F, entry(cur), tq, gq < cur.nc);
+  cp_async_commit();
+  unsigned long long e1 = v1 ? entry(nx1) : 0ull;
+  double acc[3][TE][2];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int y = 0; y < TE; ++y) acc[c][y][0] = acc[c][y][1] = 0.0;
+  int buf = 0;
+  while (true) {
+    cp_async_wait_all();
+    __syncwarp();
+    bool v2 = false;
+    TileItem nx2{0, 0, 0, 0};
+    unsigned long long e2 = 0ull;
+    if (v1) {
+      stage_part64(sw[buf ^ 1] + gq * SBL, sF[buf ^ 1][gq], wc, F, e1, tq, gq < nx1.nc);
+      cp_async_commit();
+      v2 = gen.next();
+      if (v2) {
+        nx2 = gen.item();
+        e2 = entry(nx2);
+      }
+    }
+#pragma unroll 1
+    for (int k0 = 0; k0 < cur.nc; k0 += 4) {  // uniform over the warp
+      const double* sb = sw[buf] + (k0 + tq) * SBL;
+      const double wx = sb[gq], wz = sb[2 * TE + gq];
+      const double f0 = sF[buf][k0 + tq][0], f1 = sF[buf][k0 + tq][1], f2 = sF[buf][k0 + tq][2];
+#pragma unroll
+      for (int y = 0; y < TE; ++y) {
+        const double wyz = sb[TE + y] * wz;
+        mma_f64(acc[0][y], f0 * wyz, wx);
+        mma_f64(acc[1][y], f1 * wyz, wx);
+        mma_f64(acc[2][y], f2 * wyz, wx);
+      }
+    }
+    if (cur.last) {  // the tile is complete: every point written once
+      const int tz = cur.tile % g.ntz, ty = (cur.tile / g.ntz) % g.nty, tx = cur.tile / (g.ntz * g.nty);
+      const long long xs = (long long)g.ny * g.nz;
+      const long long i0 = ((long long)(tx * TE + 2 * tq) * g.ny + ty * TE) * g.nz + tz * TE + gq;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int y = 0; y < TE; ++y)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const long long idx = i0 + h * xs + (long long)y * g.nz;
+            if (FCM_INB(idx, G, BS_GRID)) grid[c * G + idx] = acc[c][y][h];
+            acc[c][y][h] = 0.0;
+          }
+    }
+    if (!v1) break;
+    cur = nx1;
+    nx1 = nx2;
+    v1 = v2;
+    e1 = e2;
+    buf ^= 1;
+  }
+}
+
+// Interpolation: P_c[k, x] = sum over (y, z) of (wy_k[y] wz_k[z]) u_c[x][y][z], 16 k-steps
+// of four (y, z) with the tile's velocities as B fragments in registers (48 doubles per
+// lane), for two groups of eight blobs; then partial_kc = sum over x of P_c[k, x] wx_k[x].
+// Persistent and pipelined as the spread; the next tile's grid is copied to shared
+// memory while this tile's rounds run.  48 MMAs and 16 products per eight blobs; the 252
+// registers (the grid in fragments) leave eight warps per SM, and half the cycles have no
+// MMA in flight (350 us at 256^3 with 57.7 blobs per tile, 138 us with 2048 rods; the
+// shuffle-reduced warp kernel took 499 and 178 us).  A warp per component (a third of the
+// registers, but the operand products and the round's overhead three times) took 403 us,
+// register caps for ten or eleven warps per SM 385 us and more (spills).
+constexpr int SGX64 = TE * TE + 4;  // padded x-plane: the fragment reads fall in different banks
+
+__device__ __forceinline__ void grid_tile_async64(const double* __restrict__ grid, const TileGeom& g, long long G,
+                                                  int tile, double* sg) {
+  const int tz = tile % g.ntz, ty = (tile / g.ntz) % g.nty, tx = tile / (g.ntz * g.nty);
+#pragma unroll
+  for (int q = 0; q < 24; ++q) {  // 3 x 8 x 8 rows of four 16-byte parts
+    const int i = threadIdx.x + 32 * q, row = i >> 2, part = i & 3;
+    const int c = row >> 6, x = (row >> 3) & 7, y = row & 7;
+    const long long idx = ((long long)(tx * TE + x) * g.ny + ty * TE + y) * g.nz + tz * TE + 2 * part;
+    cp_async16_or_zero(sg + (c * TE + x) * SGX64 + y * TE + 2 * part, grid + c * G + idx, FCM_INB(idx + 1, G, BS_GRID));
+  }
+}
+
+__global__ void __launch_bounds__(32) k_interp_mma64(const double* __restrict__ wc, const double* __restrict__ grid,
+                                                     TileGeom g, const int* __restrict__ offset,
+                                                     const unsigned long long* __restrict__ list, long long G,
+                                                     double* __restrict__ partial, int ntiles) {
+  constexpr int RB = 16;
+  __shared__ __align__(16) double sw[2][RB * SBL];
+  __shared__ unsigned long long sent[2][RB];
+  __shared__ __align__(16) double sg[3 * TE * SGX64];
+  const int lane = threadIdx.x, gq = lane >> 2, tq = lane & 3;
+  ItemGen<RB> gen{offset, ntiles, (int)gridDim.x, 0, 0, 0, 0, 0, 0, 0};
+  if (!gen.first()) return;  // uniform over the warp
+  TileItem cur = gen.item();
+  bool v1 = gen.next();
+  TileItem nx1 = v1 ? gen.item() : TileItem{0, 0, 0, 0};
+  unsigned long long e1[2];
+  auto entries = [&](const TileItem& it, unsigned long long (&e)[2]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) e[i] = gq + 8 * i < it.nc ? list_entry(list, it.c0 + gq + 8 * i, g) : 0ull;
+  };
+  auto stage = [&](int b, const TileItem& it, const unsigned long long (&e)[2]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int k = gq + 8 * i;
+      stage_part64(sw[b] + k * SBL, nullptr, wc, nullptr, e[i], tq, k < it.nc);
+      if (tq == 3) sent[b][k] = e[i];
+    }
+  };
+  grid_tile_async64(grid, g, G, cur.tile, sg);
+  entries(cur, e1);
+  stage(0, cur, e1);
+  cp_async_commit();
+  if (v1) entries(nx1, e1);
+  double u[2 * TE][3];  // B fragments: (y, z) = (j / 2, 4 (j % 2) + tq), x = gq
+  bool first = true;    // cur is the first round of its tile
+  int buf = 0;
+  while (true) {
+    cp_async_wait_all();
+    __syncwarp();
+    if (first) {
+      const int ty = (cur.tile / g.ntz) % g.nty;
+#pragma unroll
+      for (int j = 0; j < 2 * TE; ++j) {
+        const bool live = ty * TE + (j >> 1) < g.ycut;  // rows at or above the slip channel's upper wall read as 0
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double v = sg[(c * TE + gq) * SGX64 + 4 * j + tq];
+          u[j][c] = live ? v : 0.0;
+        }
+      }
+      __syncwarp();  // every lane has its fragments: the buffer takes the next tile
+      const int nt = cur.tile + (int)gridDim.x;
+      if (nt < ntiles) grid_tile_async64(grid, g, G, nt, sg);
+    }
+    bool v2 = false;
+    TileItem nx2{0, 0, 0, 0};
+    unsigned long long e2[2] = {0ull, 0ull};
+    if (v1) {
+      stage(buf ^ 1, nx1, e1);
+      v2 = gen.next();
+      if (v2) {
+        nx2 = gen.item();
+        entries(nx2, e2);
+      }
+    }
+    cp_async_commit();
+    if (cur.nc > 0) {  // uniform over the warp
+      const bool two = cur.nc > 8;
+      const double* sa = sw[buf] + gq * SBL;
+      const double* sb = sa + 8 * SBL;
+      double pa[3][2], pb[3][2];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) pa[c][0] = pa[c][1] = pb[c][0] = pb[c][1] = 0.0;
+      const double za0 = sa[2 * TE + tq], za1 = sa[2 * TE + 4 + tq];
+      if (two) {
+        const double zb0 = sb[2 * TE + tq], zb1 = sb[2 * TE + 4 + tq];
+#pragma unroll
+        for (int j = 0; j < 2 * TE; ++j) {
+          const double aa = sa[TE + (j >> 1)] * (j & 1 ? za1 : za0), ab = sb[TE + (j >> 1)] * (j & 1 ? zb1 : zb0);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            mma_f64(pa[c], aa, u[j][c]);
+            mma_f64(pb[c], ab, u[j][c]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 2 * TE; ++j) {
+          const double aa = sa[TE + (j >> 1)] * (j & 1 ? za1 : za0);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) mma_f64(pa[c], aa, u[j][c]);
+        }
+      }
+      // contract x (lane tq holds x = 2 tq, 2 tq + 1 of blob gq or gq + 8), then lane tq
+      // < 3 writes component tq
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (h == 1 && !two) break;
+        const double2 w = *reinterpret_cast<const double2*>((h ? sb : sa) + 2 * tq);
+        double v[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          v[c] = h ? pb[c][0] * w.x + pb[c][1] * w.y : pa[c][0] * w.x + pa[c][1] * w.y;
+          v[c] += __shfl_xor_sync(0xffffffffu, v[c], 1);
+          v[c] += __shfl_xor_sync(0xffffffffu, v[c], 2);
+        }
+        const int k = gq + 8 * h;
+        if (tq < 3 && k < cur.nc) {
+          const unsigned long long e = sent[buf][k];
+          const unsigned b = (unsigned)(e >> 32), jt = ((unsigned)e >> EJ) & 63u;
+          if (FCM_INB((long long)b * 64 + jt, (long long)g.nblobs * 64, BS_PARTIAL))
+            partial[((size_t)b * 64 + jt) * 3 + tq] = tq == 0 ? v[0] : tq == 1 ? v[1] : v[2];
+        }
+      }
+    }
+    first = cur.last != 0;
+    if (!v1) break;
+    cur = nx1;
+    nx1 = nx2;
+    v1 = v2;
+    e1[0] = e2[0];
+    e1[1] = e2[1];
     buf ^= 1;
   }
   cp_async_wait_all();  // no copy outlives the kernel
@@ -1751,14 +2036,19 @@ int launch_set_up_gaussians(const Ctx& c, BlobTable<T>& t, const double* dY, cud
 template <typename T>
 int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid, cudaStream_t s) {
   if (t.tiled) {
-    // by default FP64 takes the persistent pipelined kernel (its staging latency is
-    // the limit), FP32 one CTA per tile staging 16 blobs per round; fcm_autotune may
-    // choose another (one CTA per tile with 8 or 32 blobs per round)
+    // by default FP64 takes the tensor-core kernel (variant 0; the persistent pipelined
+    // FMA kernel is FP32's variant 0), FP32 one warp per tile; fcm_autotune may choose
+    // another (one CTA per tile with 8, 16 or 32 blobs per round)
     const int v = c.spread_variant[sizeof(T) == 8 ? 0 : 1];
     const TileGeom tg = tile_geom(c.g, t);
     if (v == 0) {
-      const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_pipe<T>, 64, c.device));
-      k_spread_pipe<T><<<ctas, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid, t.ntiles);
+      if constexpr (sizeof(T) == 8) {
+        const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_mma64, 32, c.device));
+        k_spread_mma64<<<ctas, 32, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid, t.ntiles);
+      } else {
+        const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_pipe<T>, 64, c.device));
+        k_spread_pipe<T><<<ctas, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid, t.ntiles);
+      }
     } else if (v == 2) {
       k_spread_tiled<T, 8><<<t.ntiles, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid);
     } else if (v == 3) {
@@ -1790,6 +2080,18 @@ int launch_interp(const Ctx& c, const BlobTable<T>& t, const T* grid, double* dV
     TileGeom g = tile_geom(c.g, t);
     g.ycut = ycut;
     const int v = c.interp_variant[sizeof(T) == 8 ? 0 : 1];
+    if constexpr (sizeof(T) == 8) {
+      // FP64 variant 1; the kernel copies 16-byte parts of the grid's rows (every caller's
+      // grid is an allocation of its own, so aligned; otherwise the 64-thread kernel)
+      if (v == 1 && (reinterpret_cast<uintptr_t>(grid) & 15u) == 0) {
+        k_interp_mma64<<<std::min(t.ntiles, persistent_ctas(k_interp_mma64, 32, c.device)), 32, 0, s>>>(
+            t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles);
+        FCM_LAUNCH_CHECK();
+        k_interp_reduce8<T><<<(t.n + 15) / 16, 128, 0, s>>>(t.base, t.partial, t.n, g, dx3, dV);
+        FCM_LAUNCH_CHECK();
+        return FCM_OK;
+      }
+    }
     if constexpr (sizeof(T) == 4) {
       // the tensor-core kernel copies 16-byte rows of the grid asynchronously
       if (v == 3 && (reinterpret_cast<uintptr_t>(grid) & 15u) == 0) {
@@ -1803,7 +2105,7 @@ int launch_interp(const Ctx& c, const BlobTable<T>& t, const T* grid, double* dV
     }
     if (v == 2)
       k_interp_rows<T, 2><<<t.ntiles, 32, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
-    else if (v == 1)
+    else if (sizeof(T) == 4 && v == 1)
       k_interp_warp<T><<<t.ntiles, 32, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
     else
       k_interp_tiled<T><<<t.ntiles, 64, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
