@@ -305,9 +305,11 @@ int fcm_interp(fcm_ctx* ctx, int32_t precision, double* V);
  *       per tile on the tensor cores (mma.sync with TF32 operands split in two,
  *       3xTF32, FP32 accumulators), equal to the others to FP32 rounding.
  *   [1] FP64 Stokes solve, [3] FP32 Stokes solve: 0 = cuFFT 3D transforms and the
- *       projection kernel, 1 = cuFFT (y, z) transforms around the fused x-transform
- *       + projection kernel, 2 = the library's own (y, z) transforms around it
- *       (FP32 only).  FP64 defaults to 0 beyond 256 points along x.  The solves
+ *       projection kernel (FP64 beyond 256 points along x with three supported lengths:
+ *       the library's transforms of variant 1), 1 = the projection fused into the
+ *       x-transform, in FP64 with the library's own transforms where all three lengths
+ *       are supported, else between cuFFT (y, z) transforms, 2 = the library's own
+ *       transforms in FP32.  FP64 defaults to 0 beyond 256 points along x.  The solves
  *       agree within rounding.
  *   [4] FP64 interpolation, [5] FP32 interpolation: 0 = 64 threads per 8^3 tile
  *       with a warp shuffle reduction, 1 = one warp per tile (FP64: on the FP64

@@ -1,0 +1,49 @@
+"""The Stokes solve on the packed half spectrum (FP64 solve variant 1, FP32 variant 2; the
+default where all three lengths are supported) on the shapes where it can go wrong: the
+smallest lengths (tiles padded beyond H/2 columns, fewer columns than a tile), lengths that
+are not whole numbers of tile columns, planes by one CTA and by separate passes, both tile
+shapes (256 points along x and more), the longest lengths, and narrow Gaussians (ngauss 4,
+sigma = 0.56 dx), whose spectrum is far from zero in the Nyquist rows and planes where the
+projection is symmetrised.  The whole velocity field is compared with the oracle's: norm-wise
+1e-12 in FP64 (a few hundred roundings), 1e-6 in FP32 as the rest of the suite."""
+import numpy as np
+import pytest
+
+from tests.conftest import rel_err
+from tests.oracle_lib import Oracle
+from timstochrigidbodiessim_b200.fcm import Suspension
+from timstochrigidbodiessim_b200.params import FcmParams
+
+pytestmark = pytest.mark.gpu
+
+
+def _params(n, nb, **kw):
+    return FcmParams.defaults(nx=n[0], ny=n[1], nz=n[2], ngauss=4, dx=1.0, num_bodies=nb, blobs_per_body=1, ncells=3,
+                              precision=1, **kw)
+
+
+@pytest.mark.parametrize("n", [(8, 8, 8), (12, 8, 12), (8, 12, 16), (16, 8, 12), (24, 16, 8), (24, 24, 24),
+                               (48, 12, 16), (64, 32, 24), (96, 8, 48), (192, 16, 12), (256, 12, 8), (256, 16, 96),
+                               (8, 384, 16), (8, 16, 384), (12, 512, 512), (384, 8, 8), (384, 16, 24), (512, 8, 12),
+                               (512, 12, 16), (16, 48, 48), (8, 96, 96)])
+def test_velocity_field(gpu, n):
+    nb = 30
+    rng = np.random.default_rng(sum(n))
+    Y = (rng.uniform(0, 1, (nb, 3)) * np.array(n)).ravel()
+    F = rng.standard_normal(3 * nb)
+    p = _params(n, nb)
+    g, o = Suspension(p, [0, 0, 0]), Oracle(p.copy(precision=0), [0, 0, 0])
+    for s in (g, o):
+        s.set_up_gaussians(Y)
+        s.set_up_force_distribution(F)
+        s.produce_deterministic_velocity_field()
+    assert g.get_variants()[3] == 2
+    ug = g.get_velocity_field(0)
+    for c in range(3):
+        a, b = (np.asarray(u).reshape(n[0], n[1], -1)[:, :, :n[2]] for u in (ug[c], o.get_grid(3 + c)))
+        assert rel_err(a, b) < 1e-12, c
+    Vo = o.calculate_deterministic_blob_velocities()
+    g.spread(F, 1)
+    g.stokes_solve(1)
+    assert rel_err(g.interp(1), Vo) < 1e-6
+

@@ -411,25 +411,38 @@ int setup_xfft(Ctx* c) {
   c->d_xtw32 = d32;
   FCM_CUDA(cudaMemcpy(d64, wd.data(), sizeof(double2) * n, cudaMemcpyHostToDevice));
   FCM_CUDA(cudaMemcpy(d32, wf.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
-  // FP32 (y, z) transforms by the library's kernels, where they beat cuFFT's 2D
-  // plans: 64^3, 96^3 (the 64-suspension ensemble ran 11% faster), 256^3 (328
-  // against 364 us per solve) and, with 16 kz per y CTA, 512^3 (the whole FP32 solve
-  // 4091 against 4477 us)
-  c->yz32_cap = xfft_factor(c->g.ny, &n1, &n2) && xfft_factor(c->g.nz, &n1, &n2) && 3 * c->g.nx <= 65535;
-  c->yz32 = c->yz32_cap;
-  if (c->yz32_cap) {
+  // all three lengths supported: the packed half-spectrum solve and its twiddles along y, z
+  c->packed_cap = xfft_factor(c->g.ny, &n1, &n2) && xfft_factor(c->g.nz, &n1, &n2);
+  c->packed32 = c->packed_cap;
+  if (c->packed_cap) {
+    FCM_TRY(packed_tables_init());
     for (int d = 0; d < 2; ++d) {
       const int m = d == 0 ? c->g.ny : c->g.nz;
-      std::vector<float2> w(m);
-      for (int j = 0; j < m; ++j)
-        w[j] = make_float2((float)std::cos(2.0 * PI * j / m), (float)-std::sin(2.0 * PI * j / m));
-      float2* dw = nullptr;
-      FCM_TRY(dev_alloc(&dw, (size_t)m));
-      (d == 0 ? c->d_ytw32 : c->d_ztw32) = dw;
-      FCM_CUDA(cudaMemcpy(dw, w.data(), sizeof(float2) * m, cudaMemcpyHostToDevice));
+      std::vector<double2> w64(m);
+      std::vector<float2> w32(m);
+      for (int j = 0; j < m; ++j) {
+        w64[j] = make_double2(std::cos(2.0 * PI * j / m), -std::sin(2.0 * PI * j / m));
+        w32[j] = make_float2((float)w64[j].x, (float)w64[j].y);
+      }
+      double2* t64 = nullptr;
+      float2* t32 = nullptr;
+      FCM_TRY(dev_alloc(&t64, (size_t)m));
+      (d == 0 ? c->d_ytw64 : c->d_ztw64) = t64;
+      FCM_TRY(dev_alloc(&t32, (size_t)m));
+      (d == 0 ? c->d_ytw32 : c->d_ztw32) = t32;
+      FCM_CUDA(cudaMemcpy(t64, w64.data(), sizeof(double2) * m, cudaMemcpyHostToDevice));
+      FCM_CUDA(cudaMemcpy(t32, w32.data(), sizeof(float2) * m, cudaMemcpyHostToDevice));
     }
   }
   return FCM_OK;
+}
+
+// Complex values of a grid's spectrum: cuFFT's three half spectra or the packed layout,
+// whichever is larger (the packed one for 8 and 12 points along z, padded to whole tiles).
+template <typename T>
+size_t spectrum_size(const Ctx& c) {
+  const size_t n = 3 * (size_t)c.g.Gc;
+  return c.packed_cap ? std::max(n, (size_t)packed_spectrum_size<T>(c)) : n;
 }
 
 template <typename T>
@@ -437,7 +450,7 @@ int ensure_grid(Ctx* c) {
   GridBufs<T>& gb = grid_of<T>(c);
   if (gb.ready) return FCM_OK;
   FCM_TRY(dev_alloc(&gb.r, 3 * (size_t)c->g.G));
-  FCM_TRY(dev_alloc(&gb.c, 3 * (size_t)c->g.Gc));
+  FCM_TRY(dev_alloc(&gb.c, spectrum_size<T>(*c)));
   FCM_TRY(dev_alloc(&gb.urand, 3 * (size_t)c->g.G));
   FCM_CUDA(cudaMemsetAsync(gb.urand, 0, sizeof(T) * 3 * (size_t)c->g.G, c->stream));
   int n[3] = {c->g.nx, c->g.ny, c->g.nz};
@@ -445,7 +458,9 @@ int ensure_grid(Ctx* c) {
   FCM_CUFFT(cufftPlanMany(&gb.c2r, 3, n, nullptr, 1, (int)c->g.Gc, nullptr, 1, (int)c->g.G, c2r_type<T>(), 3));
   FCM_CUFFT(cufftSetStream(gb.r2c, c->stream));
   FCM_CUFFT(cufftSetStream(gb.c2r, c->stream));
-  if (c->xfft_cap[sizeof(T) == 8 ? 0 : 1]) {  // (y, z) transforms of the 3 nx planes of each component
+  // cuFFT's (y, z) transforms of the 3 nx planes, for the fused x-transform on grids
+  // without the packed solve and for FP32 variant 1
+  if (c->xfft_cap[sizeof(T) == 8 ? 0 : 1] && !(sizeof(T) == 8 && c->packed_cap)) {
     int n2[2] = {c->g.ny, c->g.nz};
     const int planes = 3 * c->g.nx;
     FCM_CUFFT(cufftPlanMany(&gb.r2c2d, 2, n2, nullptr, 1, c->g.ny * c->g.nz, nullptr, 1, c->g.ny * c->g.nzh,
@@ -517,14 +532,13 @@ template <typename T>
 int stokes_t(Ctx* c) {
   NvtxRange r(sizeof(T) == 8 ? "fcm stokes solve fp64" : "fcm stokes solve fp32");
   GridBufs<T>& gb = grid_of<T>(c);
-  if (c->xfft[sizeof(T) == 8 ? 0 : 1]) {  // (y, z) transforms, then x + projection + inverse x
-    if constexpr (sizeof(T) == 4) {
-      if (c->yz32) {
-        FCM_TRY(launch_yz_forward(*c, gb.r, gb.c, 1, c->stream));
-        FCM_TRY(launch_xfft_project<T>(*c, gb.c, c->stream));
-        return launch_yz_inverse(*c, gb.c, gb.r, 1, c->stream);
-      }
-    }
+  constexpr int P = sizeof(T) == 8 ? 0 : 1;
+  if (use_packed(*c, P)) {
+    FCM_TRY(launch_packed_forward<T>(*c, gb.r, gb.c, 1, c->stream));
+    FCM_TRY(launch_packed_project<T>(*c, gb.c, c->stream));
+    return launch_packed_inverse<T>(*c, gb.c, gb.r, 1, c->stream);
+  }
+  if (c->xfft[P]) {  // (y, z) transforms, then x + projection + inverse x
     FCM_CUFFT(exec_r2c(gb.r2c2d, gb.r, gb.c));
     FCM_TRY(launch_xfft_project<T>(*c, gb.c, c->stream));
     FCM_CUFFT(exec_c2r(gb.c2r2d, gb.c, gb.r));
@@ -1298,6 +1312,8 @@ void destroy_ctx(Ctx* c) {
   cudaFree(c->d_xtw32);
   cudaFree(c->d_ytw32);
   cudaFree(c->d_ztw32);
+  cudaFree(c->d_ytw64);
+  cudaFree(c->d_ztw64);
   cudaFree(c->d_ushear);
   cudaFree(c->d_vshear);
   cudaFree(c->d_mcmc);
@@ -1931,27 +1947,28 @@ template <typename T>
 int batch_saddle(Batch* B, int in, int out, int mask, cudaStream_t s) {
   constexpr int P = sizeof(T) == 8 ? 0 : 1;
   FCM_TRY(b_spread<T>(B->geom, in, mask, s));
-  bool any3d = false;  // groups without the fused x-transform
+  bool any3d = false;  // groups without a projection in their x transforms
   for (BatchGroup& g : B->groups) {
-    const bool fused = g.r2c2d[P] != 0;
-    any3d = any3d || !fused;
     const Ctx& c0 = *B->m[g.idx[0]];
     const int k = (int)g.idx.size();
-    if (P == 1 && fused && c0.yz32 && 3LL * c0.g.nx * k <= 65535) {  // the library's (y, z) transforms
-      FCM_TRY(launch_yz_forward(c0, (const float*)g.r[P], (cufftComplex*)g.c[P], k, s));
-    } else {
-      const cufftHandle h = fused ? g.r2c2d[P] : g.r2c[P];
-      FCM_CUFFT(cufftSetStream(h, s));
-      FCM_CUFFT(exec_r2c(h, (T*)g.r[P], (typename cplx_t<T>::type*)g.c[P]));
+    if (use_packed(c0, P)) {
+      FCM_TRY(launch_packed_forward<T>(c0, (const T*)g.r[P], (typename cplx_t<T>::type*)g.c[P], k, s));
+      FCM_TRY(b_packed_project<T>(B->geom, c0, g.d_gidx, k, mask, s));
+      continue;
     }
+    const bool fused = g.r2c2d[P] != 0;
+    any3d = any3d || !fused;
+    const cufftHandle h = fused ? g.r2c2d[P] : g.r2c[P];
+    FCM_CUFFT(cufftSetStream(h, s));
+    FCM_CUFFT(exec_r2c(h, (T*)g.r[P], (typename cplx_t<T>::type*)g.c[P]));
     if (fused) FCM_TRY(b_xfft_project<T>(B->geom, c0, g.d_gidx, k, mask, s));
   }
   if (any3d) FCM_TRY(b_project<T>(B->geom, mask, s));  // members of the other groups
   for (BatchGroup& g : B->groups) {
     const Ctx& c0 = *B->m[g.idx[0]];
     const int k = (int)g.idx.size();
-    if (P == 1 && g.c2r2d[P] && c0.yz32 && 3LL * c0.g.nx * k <= 65535) {
-      FCM_TRY(launch_yz_inverse(c0, (cufftComplex*)g.c[P], (float*)g.r[P], k, s));
+    if (use_packed(c0, P)) {
+      FCM_TRY(launch_packed_inverse<T>(c0, (typename cplx_t<T>::type*)g.c[P], (T*)g.r[P], k, s));
       continue;
     }
     const cufftHandle h = g.c2r2d[P] ? g.c2r2d[P] : g.c2r[P];
@@ -2144,6 +2161,23 @@ int build_batch_graph(Batch* B) {
 
 // The members' grids of precision T moved into one contiguous array per group
 // of equal grids, with one cuFFT plan per group over all of them.
+// Whether a solve of precision P projects inside its x-transform kernel.
+bool projects_in_x(const Ctx& c, int P) { return c.xfft[P] || use_packed(c, P); }
+
+// Member i's spectrum in the batched kernels: its own part of the group's array, or, on
+// the packed half spectrum (all of a group's grids transformed as one array), its share
+// of that.
+template <typename T>
+void* batch_spec(const Batch* B, Ctx* c, int i) {
+  constexpr int P = sizeof(T) == 8 ? 0 : 1;
+  if (!use_packed(*c, P)) return grid_of<T>(c).c;
+  for (const BatchGroup& g : B->groups)
+    for (size_t j = 0; j < g.idx.size(); ++j)
+      if (g.idx[j] == i)
+        return (typename cplx_t<T>::type*)g.c[P] + j * (size_t)packed_spectrum_size<T>(*c);
+  return nullptr;
+}
+
 template <typename T>
 int rehome_grids(Batch* B, int P) {
   for (BatchGroup& grp : B->groups) {
@@ -2153,7 +2187,7 @@ int rehome_grids(Batch* B, int P) {
     typename cplx_t<T>::type* sp = nullptr;
     T* ur = nullptr;
     FCM_TRY(dev_alloc(&r, 3 * G * k));
-    FCM_TRY(dev_alloc(&sp, 3 * Gc * k));
+    FCM_TRY(dev_alloc(&sp, spectrum_size<T>(*c0) * k));
     FCM_TRY(dev_alloc(&ur, 3 * G * k));
     grp.r[P] = r;
     grp.c[P] = sp;
@@ -2167,22 +2201,23 @@ int rehome_grids(Batch* B, int P) {
         cudaFree(gb.urand);
       }
       gb.r = r + 3 * G * j;
-      gb.c = sp + 3 * Gc * j;
+      gb.c = sp + spectrum_size<T>(*c0) * j;
       gb.urand = ur + 3 * G * j;
       gb.borrowed = true;
     }
     int nn[3] = {grp.nx, grp.ny, grp.nz};
     FCM_CUFFT(cufftPlanMany(&grp.r2c[P], 3, nn, nullptr, 1, (int)G, nullptr, 1, (int)Gc, r2c_type<T>(), (int)(3 * k)));
     FCM_CUFFT(cufftPlanMany(&grp.c2r[P], 3, nn, nullptr, 1, (int)Gc, nullptr, 1, (int)G, c2r_type<T>(), (int)(3 * k)));
-    if (c0->xfft[P]) {
+    const bool packed = use_packed(*c0, P);
+    if (c0->xfft[P] && !packed) {
       int n2[2] = {grp.ny, grp.nz};
       const int pz = grp.ny * grp.nz, pc = grp.ny * (grp.nz / 2 + 1), planes = (int)(3 * grp.nx * k);
       FCM_CUFFT(cufftPlanMany(&grp.r2c2d[P], 2, n2, nullptr, 1, pz, nullptr, 1, pc, r2c_type<T>(), planes));
       FCM_CUFFT(cufftPlanMany(&grp.c2r2d[P], 2, n2, nullptr, 1, pc, nullptr, 1, pz, c2r_type<T>(), planes));
-      if (!grp.d_gidx) {
-        FCM_TRY(dev_alloc(&grp.d_gidx, k));
-        FCM_CUDA(cudaMemcpy(grp.d_gidx, grp.idx.data(), sizeof(int) * k, cudaMemcpyHostToDevice));
-      }
+    }
+    if ((c0->xfft[P] || packed) && !grp.d_gidx) {
+      FCM_TRY(dev_alloc(&grp.d_gidx, k));
+      FCM_CUDA(cudaMemcpy(grp.d_gidx, grp.idx.data(), sizeof(int) * k, cudaMemcpyHostToDevice));
     }
   }
   return FCM_OK;
@@ -2295,7 +2330,7 @@ int create_batch(int n, const fcm_params* params, const double* const* refs, Bat
     G.red_blocks = std::max(G.red_blocks, c->red_blocks);
     G.md_blocks = std::max(G.md_blocks, c->md_blocks);
     G.total_tiles += c->g64.blobs.ntiles;
-    if (!(c->xfft[0] && c->xfft[1])) G.total_kblocks += (int)((c->g.Gc + 255) / 256);  // k_b_project's share
+    if (!(projects_in_x(*c, 0) && projects_in_x(*c, 1))) G.total_kblocks += (int)((c->g.Gc + 255) / 256);  // k_b_project's share
   }
   G.max_sys_blocks = (int)((max_sys + 255) / 256);
   G.max_blob_blocks = (int)((max_Nb + 127) / 128);
@@ -2371,7 +2406,7 @@ int create_batch(int n, const fcm_params* params, const double* const* refs, Bat
     m.tlist[0] = c->g64.blobs.tile_list;
     m.base[0] = c->g64.blobs.base;
     m.grid[0] = c->g64.r;
-    m.spec[0] = c->g64.c;
+    m.spec[0] = batch_spec<double>(B, c, i);
     m.partial[0] = c->g64.blobs.partial;
     if (B->precision == 1) {
       m.wc[1] = c->g32.blobs.wc;
@@ -2379,17 +2414,17 @@ int create_batch(int n, const fcm_params* params, const double* const* refs, Bat
       m.tlist[1] = c->g32.blobs.tile_list;
       m.base[1] = c->g32.blobs.base;
       m.grid[1] = c->g32.r;
-      m.spec[1] = c->g32.c;
+      m.spec[1] = batch_spec<float>(B, c, i);
       m.partial[1] = c->g32.blobs.partial;
     }
     m.tg[0] = tile_geom(c->g, c->g64.blobs);
     m.tg[1] = B->precision == 1 ? tile_geom(c->g, c->g32.blobs) : tile_geom(c->g, c->g64.blobs);
     m.kp = make_kparams(*c);
     m.dx3 = c->g.dx * c->g.dx * c->g.dx;
-    m.xfft[0] = c->xfft[0] ? 1 : 0;
-    m.xfft[1] = c->xfft[1] ? 1 : 0;
+    m.xfft[0] = projects_in_x(*c, 0) ? 1 : 0;
+    m.xfft[1] = projects_in_x(*c, 1) ? 1 : 0;
     for (int t = 0; t < c->g64.blobs.ntiles; ++t) tmap.push_back(make_int2(i, t));
-    const int kb = (c->xfft[0] && c->xfft[1]) ? 0 : (int)((c->g.Gc + 255) / 256);
+    const int kb = (projects_in_x(*c, 0) && projects_in_x(*c, 1)) ? 0 : (int)((c->g.Gc + 255) / 256);
     for (int t = 0; t < kb; ++t) kmap.push_back(make_int2(i, t));
   }
   if (cudaMemcpy(B->d_mem, hm.data(), sizeof(BMember) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -2509,11 +2544,11 @@ struct fcm_batch {
 using namespace fcm;
 
 // ------------------------------------------------------------------ kernel variants
-// Solve variant of precision P: 0 = 3D transforms, 1 = fused x-transform with
-// cuFFT's (y, z) plans, 2 = with the library's (y, z) kernels.
+// Solve variant of precision P: 0 = 3D transforms, 1 = the projection fused into the
+// x-transform (FP32: around cuFFT's (y, z) plans), 2 = FP32 on the packed half spectrum.
 static int solve_variant(const Ctx* c, int P) {
   if (!c->xfft[P]) return 0;
-  return (P == 1 && c->yz32) ? 2 : 1;
+  return (P == 1 && c->packed32) ? 2 : 1;
 }
 
 static void get_variants(const Ctx* c, int32_t* v) {
@@ -2534,7 +2569,7 @@ static int set_variants(Ctx* c, const int32_t* v) {
       return FCM_ERR_INVALID;
     }
     if (P == 1 && c->p.precision != 1) continue;  // no FP32 grid
-    if ((sv >= 1 && !c->xfft_cap[P]) || (sv == 2 && !c->yz32_cap)) {
+    if ((sv >= 1 && !c->xfft_cap[P]) || (sv == 2 && !c->packed_cap)) {
       set_error("this grid does not allow solve variant " + std::to_string(sv));
       return FCM_ERR_INVALID;
     }
@@ -2543,7 +2578,7 @@ static int set_variants(Ctx* c, const int32_t* v) {
     if (P == 1 && c->p.precision != 1) continue;
     c->spread_variant[P] = v[2 * P];
     c->xfft[P] = v[2 * P + 1] >= 1;
-    if (P == 1) c->yz32 = v[3] == 2;
+    if (P == 1) c->packed32 = v[3] == 2;
     c->interp_variant[P] = v[4 + P];
   }
   c->graph_stale = true;
@@ -2599,16 +2634,16 @@ static int tune_precision(Ctx* c, int reps, double* t) {
   }
   FCM_CUDA(cudaMemsetAsync(gb.r, 0, sizeof(T) * 3 * (size_t)c->g.G, c->stream));
   for (int v = 0; v < 3; ++v) {
-    if ((v >= 1 && !c->xfft_cap[P]) || (v == 2 && (P == 0 || !c->yz32_cap))) continue;
+    if ((v >= 1 && !c->xfft_cap[P]) || (v == 2 && (P == 0 || !c->packed_cap))) continue;
     c->xfft[P] = v >= 1;
-    if (P == 1) c->yz32 = v == 2;
+    if (P == 1) c->packed32 = v == 2;
     FCM_TRY(time_calls(c, reps, [&] { return stokes_t<T>(c); }, &t[6 + v]));
   }
   int best = 0;
   for (int v = 1; v < 3; ++v)
     if (t[6 + v] >= 0.0 && t[6 + v] < t[6 + best]) best = v;
   c->xfft[P] = best >= 1;
-  if (P == 1) c->yz32 = best == 2;
+  if (P == 1) c->packed32 = best == 2;
   if (bt.tiled) {  // interpolation of the (zeroed) grid into scratch
     for (int v = 0; v < NIP; ++v) {
       c->interp_variant[P] = v;
@@ -2665,7 +2700,7 @@ int fcm_debug_bounds(int32_t* checked, int64_t* count, int32_t* site, int64_t* i
     const int on = 0;
 #endif
     int (*readers[])(BoundsRecord*, int) = {bounds_read_grid, bounds_read_cells, bounds_read_kspace,
-                                            bounds_read_blas};
+                                            bounds_read_packed, bounds_read_blas};
     unsigned long long total = 0;
     BoundsRecord first{};
     for (auto rd : readers) {

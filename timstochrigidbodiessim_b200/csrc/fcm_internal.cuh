@@ -123,6 +123,7 @@ static __device__ __forceinline__ bool fcm_inb(long long i, long long n, int sit
 int bounds_read_grid(BoundsRecord* out, int reset);
 int bounds_read_cells(BoundsRecord* out, int reset);
 int bounds_read_kspace(BoundsRecord* out, int reset);
+int bounds_read_packed(BoundsRecord* out, int reset);
 int bounds_read_blas(BoundsRecord* out, int reset);
 
 template <typename T>
@@ -325,14 +326,14 @@ struct Ctx {
   // on when nx is a supported length and nz is even (FP64 up to 256 points, beyond
   // which the 3D transforms are faster); twiddles exp(-2 pi i j / nx), j < nx
   bool xfft[2] = {false, false};
-  // FP32 (y, z) transforms by this library's kernels instead of cuFFT's 2D plans
-  // (fused FP32 grids whose ny and nz are supported lengths, nz even, nz <= 256);
-  // twiddles exp(-2 pi i j / n) for n = ny, nz
-  bool yz32 = false;
+  // the packed half-spectrum solve (fcm_packed.cu): all three lengths supported; FP32
+  // solve variant 2 (packed32) and the FP64 fused variant take it, see use_packed;
+  // twiddles exp(-2 pi i j / n) for n = ny, nz in both precisions
+  bool packed_cap = false;
+  bool packed32 = false;
   // what the grids allow (fcm_autotune chooses within it): the fused x-transform per
-  // precision (its (y, z) plans exist), the library's (y, z) kernels up to 512 points
+  // precision (its (y, z) plans exist)
   bool xfft_cap[2] = {false, false};
-  bool yz32_cap = false;
   // spread kernel per precision: 0 the persistent software-pipelined one (FP64
   // default), 1 / 2 / 3 one CTA per tile staging 16 / 8 / 32 blobs per round, 4
   // one warp per tile (FP32 default); all sum every point's blobs in the same order
@@ -344,6 +345,8 @@ struct Ctx {
   int interp_variant[2] = {1, 1};
   void* d_ytw32 = nullptr;
   void* d_ztw32 = nullptr;
+  void* d_ytw64 = nullptr;
+  void* d_ztw64 = nullptr;
   void* d_xtw64 = nullptr;
   void* d_xtw32 = nullptr;
   double* d_ushear = nullptr;
@@ -368,6 +371,15 @@ struct Ctx {
   bool det_ready = false;   // deterministic velocity grid holds u
   int urand_prec = 0;       // precision of the random field last produced
 };
+
+// Whether the Stokes solve of precision P runs on the packed half spectrum: FP32 by
+// variant 2; FP64 where the lengths allow it by variant 1, and beyond 256 points along x
+// by variant 0 too, whose cuFFT 3D transforms took 9.42 ms at 512^3 against 6.49 ms (6.01
+// against 2.65 ms at 384^3).
+inline bool use_packed(const Ctx& c, int P) {
+  if (!c.packed_cap) return false;
+  return P == 1 ? c.xfft[1] && c.packed32 : c.xfft[0] || c.g.nx > 256;
+}
 
 // ------------------------------------------------------------------ batches
 // One member suspension of a batch as the batched kernels see it (a device
@@ -399,7 +411,7 @@ struct BMember {
   TileGeom tg[2];  // tile geometry of each precision's tables (their stencil widths differ)
   KParams kp;
   double dx3;
-  int xfft[2];  // the member's grids of each precision use the fused x-transform
+  int xfft[2];  // the member's grids of each precision project in their x-transform kernel
 };
 
 // Which members a batched kernel works on.
@@ -531,9 +543,19 @@ template <typename T>
 int xfft_prepare(const Ctx& c);
 template <typename T>
 int launch_xfft_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s);
-// the FP32 (y, z) transforms of `members` consecutive grids of c's shape (fcm_kspace.cu)
-int launch_yz_forward(const Ctx& c, const float* r, cufftComplex* spec, int members, cudaStream_t s);
-int launch_yz_inverse(const Ctx& c, cufftComplex* spec, float* r, int members, cudaStream_t s);
+// the packed half-spectrum solve (fcm_packed.cu) of `members` consecutive grids of c's
+// shape: (y, z) transforms, x transforms with the projection, inverse (y, z) transforms
+int packed_tables_init();
+template <typename T>
+long long packed_spectrum_size(const Ctx& c);  // complex values of one grid's spectrum
+template <typename T>
+int launch_packed_forward(const Ctx& c, const T* r, typename cplx_t<T>::type* spec, int members, cudaStream_t s);
+template <typename T>
+int launch_packed_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s);
+template <typename T>
+int launch_packed_inverse(const Ctx& c, typename cplx_t<T>::type* spec, T* r, int members, cudaStream_t s);
+template <typename T>
+int b_packed_project(const BatchGeom& b, const Ctx& c0, const int* gidx, int nm, int mask, cudaStream_t s);
 // the same for the members gidx[0..nm) of a batch group whose grids equal c0's
 template <typename T>
 int b_xfft_project(const BatchGeom& b, const Ctx& c0, const int* gidx, int nm, int mask, cudaStream_t s);

@@ -20,26 +20,12 @@
 #include <mutex>
 #include <type_traits>
 
+#include "fcm_dft.cuh"
 #include "fcm_internal.cuh"
 
 namespace fcm {
 
 namespace {
-
-template <typename T>
-struct V2 {
-  T x, y;
-};
-
-template <typename C>
-__device__ __forceinline__ V2<double> ld(const C& v) {
-  return V2<double>{(double)v.x, (double)v.y};
-}
-
-// Wavenumber of index i on an n-point grid (fcm_fluid_solver.cpp:77-91).
-__device__ __forceinline__ double wavenumber(int i, int n, double fac) {
-  return (i <= n / 2) ? (double)i * fac : (double)(i - n) * fac;
-}
 
 // Projection of one complex mode (re and im share the real factors).  The
 // reference divides every component by eta*G; here one reciprocal of the
@@ -339,7 +325,7 @@ __global__ void k_fluct(C* __restrict__ spec, const cufftDoubleComplex* __restri
 
 // ------------------------------------------------------------------ fused x-transform
 // The Stokes solve of a force grid as 2D transforms over (y, z) for every x-plane
-// (cuFFT, or the library's kernels further below) with the transform along x, the
+// (cuFFT) with the transform along x, the
 // projection and the inverse transform along x fused: interior CTAs take the
 // x-pencils of TK consecutive kz of one y row (all three components), transform
 // them along x, project every mode and transform back; plane CTAs do the same for
@@ -347,95 +333,6 @@ __global__ void k_fluct(C* __restrict__ spec, const cufftDoubleComplex* __restri
 // {k, -k}.  A 3D DFT is the x-DFT of the (y, z) DFTs, so this is the transform pair
 // of the 3D path with the projection between.  Pencils are transformed in two
 // register steps, N = N1 * N2 (both divisors of 96 up to 32).
-
-template <typename T, typename C>
-__device__ __forceinline__ V2<T> ldt(const C& v) {
-  return V2<T>{(T)v.x, (T)v.y};
-}
-
-__constant__ double2 c_w96d[96];  // exp(-2 pi i k / 96)
-__constant__ float2 c_w96f[96];
-
-template <typename T>
-__device__ __forceinline__ V2<T> w96(int k);
-template <>
-__device__ __forceinline__ V2<double> w96<double>(int k) {
-  const double2 w = c_w96d[k];
-  return V2<double>{w.x, w.y};
-}
-template <>
-__device__ __forceinline__ V2<float> w96<float>(int k) {
-  const float2 w = c_w96f[k];
-  return V2<float>{w.x, w.y};
-}
-
-template <typename T>
-__device__ __forceinline__ V2<T> cadd(V2<T> a, V2<T> b) { return V2<T>{a.x + b.x, a.y + b.y}; }
-template <typename T>
-__device__ __forceinline__ V2<T> csub(V2<T> a, V2<T> b) { return V2<T>{a.x - b.x, a.y - b.y}; }
-template <typename T>
-__device__ __forceinline__ V2<T> cmul(V2<T> a, V2<T> b) { return V2<T>{a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
-template <typename T>
-__device__ __forceinline__ V2<T> cmulc(V2<T> a, V2<T> b) { return V2<T>{a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y}; }
-// -i z (forward) or +i z (inverse)
-template <typename T, bool INV>
-__device__ __forceinline__ V2<T> rot(V2<T> z) { return INV ? V2<T>{-z.y, z.x} : V2<T>{z.y, -z.x}; }
-
-// In-register DFT of R points, R a divisor of 96: forward exp(-2 pi i n k / R),
-// inverse exp(+2 pi i n k / R), unnormalised.  Decimation in time, R = P * Q.
-template <typename T, int R, bool INV>
-__device__ __forceinline__ void dft(V2<T> (&a)[R]) {
-  if constexpr (R == 1) {
-    return;
-  } else if constexpr (R == 2) {
-    const V2<T> t = a[1];
-    a[1] = csub(a[0], t);
-    a[0] = cadd(a[0], t);
-  } else if constexpr (R == 3) {
-    // W_3 = -1/2 -+ i sqrt(3)/2
-    const T h = (T)0.86602540378443864676;
-    const V2<T> t1 = cadd(a[1], a[2]);
-    const V2<T> t2 = V2<T>{a[0].x - (T)0.5 * t1.x, a[0].y - (T)0.5 * t1.y};
-    const V2<T> d = rot<T, INV>(csub(a[1], a[2]));
-    a[0] = cadd(a[0], t1);
-    a[1] = V2<T>{t2.x + h * d.x, t2.y + h * d.y};
-    a[2] = V2<T>{t2.x - h * d.x, t2.y - h * d.y};
-  } else if constexpr (R == 4) {
-    const V2<T> s0 = cadd(a[0], a[2]), s1 = csub(a[0], a[2]);
-    const V2<T> s2 = cadd(a[1], a[3]), s3 = rot<T, INV>(csub(a[1], a[3]));
-    a[0] = cadd(s0, s2);
-    a[2] = csub(s0, s2);
-    a[1] = cadd(s1, s3);
-    a[3] = csub(s1, s3);
-  } else {
-    constexpr int P = (R % 4 == 0) ? 4 : ((R % 2 == 0) ? 2 : 3);
-    constexpr int Q = R / P;
-    static_assert(96 % R == 0, "register DFT sizes divide 96");
-    V2<T> b[P][Q];
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-#pragma unroll
-      for (int m = 0; m < Q; ++m) b[p][m] = a[P * m + p];
-#pragma unroll
-    for (int p = 0; p < P; ++p) dft<T, Q, INV>(b[p]);
-#pragma unroll
-    for (int p = 1; p < P; ++p)
-#pragma unroll
-      for (int m = 1; m < Q; ++m) {
-        const V2<T> w = w96<T>(((p * m) % R) * (96 / R));
-        b[p][m] = INV ? cmulc(b[p][m], w) : cmul(b[p][m], w);
-      }
-#pragma unroll
-    for (int m = 0; m < Q; ++m) {
-      V2<T> c[P];
-#pragma unroll
-      for (int p = 0; p < P; ++p) c[p] = b[p][m];
-      dft<T, P, INV>(c);
-#pragma unroll
-      for (int j = 0; j < P; ++j) a[m + Q * j] = c[j];
-    }
-  }
-}
 
 // Step over n1 (or k1) of every column: positions j*N2 + n2, j < N1.  Forward: DFT,
 // then the twiddle W_N^(n2 k1); inverse: DFT only (its twiddle came in step b).
@@ -768,440 +665,6 @@ __global__ void __launch_bounds__(xfft_block<T, N1, N2, TK, PLANES>(),
     xfft_interior_cta<T, C, N1, N2, TK>((C*)m.spec[P], m.kp, twN);
 }
 
-// ------------------------------------------------------------------ (y, z) transforms
-// The (y, z) transforms around k_xfft_project for FP32 grids up to 256 points
-// along z, replacing cuFFT's R2C / C2R of every x-plane.  z: the real lines are taken two at a time as the
-// real and imaginary parts of one complex pencil (the DFTs of the two real lines
-// are (Z(k) + conj Z(-k))/2 and (Z(k) - conj Z(-k))/2i), transformed in two
-// register steps with one shared-memory exchange, and written as nz/2 + 1 modes per
-// line; the inverse assembles Z(k) = A(k) + i B(k) from the two half spectra,
-// ignoring the imaginary parts of A, B at kz = 0 and nz/2 as a C2R transform does.
-// y: one CTA per (x-plane, TK kz), the step over n1 straight from global memory,
-// the step over n2 straight back to it, one barrier between.  Unnormalised, with
-// cuFFT's sign convention.
-
-// padded shared-memory index of pencil position pos (one gap after every Z2)
-template <int Z2>
-__device__ __forceinline__ int zpad(int pos) {
-  return pos + pos / Z2;
-}
-
-template <int Z1, int Z2>
-__device__ __forceinline__ int zpos(int k) {  // position of mode k after the two steps
-  return (k % Z1) * Z2 + k / Z1;
-}
-
-// Whether the z passes' middle step shares each row between two lanes where it
-// would otherwise leave half the CTA idle (Z2 = 2 Z1).
-#ifndef FCM_ZFFT_PAIR
-#define FCM_ZFFT_PAIR 1
-#endif
-
-// The Z2-point DFT of one shared-memory row (positions row[zpad(j)], j < Z2) by a
-// pair of lanes (lane and lane ^ 1): lane half h transforms the samples 2m + h
-// (Z2/2 points), the odd lane scales its result by W_Z2^k (conjugated for the
-// inverse), the pair swaps halves with shuffles and lane h writes outputs
-// k + h Z2/2 = E[k] +- W^k O[k].  Both lanes read their samples before either
-// writes (the shuffles order them).  With tw, output j > 0 is then scaled by the
-// outer twiddle tw[j k1] (conjugated for the inverse) before the store.
-template <typename T, int Z2, bool INV, typename C>
-__device__ __forceinline__ void pair_dft_row(V2<T>* row, int half, const C* __restrict__ tw, int k1) {
-  constexpr int H = Z2 / 2;
-  V2<T> a[H];
-#pragma unroll
-  for (int m = 0; m < H; ++m) a[m] = row[zpad<Z2>(2 * m + half)];
-  dft<T, H, INV>(a);
-  if (half) {
-#pragma unroll
-    for (int k = 1; k < H; ++k) {
-      const V2<T> w = w96<T>(k * (96 / Z2));
-      a[k] = INV ? cmulc(a[k], w) : cmul(a[k], w);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < H; ++k) {
-    const V2<T> o{__shfl_xor_sync(0xffffffffu, a[k].x, 1), __shfl_xor_sync(0xffffffffu, a[k].y, 1)};
-    V2<T> x = half ? csub(o, a[k]) : cadd(a[k], o);
-    const int j = k + half * H;
-    if (tw && j > 0) {
-      const V2<T> w = ldt<T>(__ldg(&tw[j * k1]));
-      x = INV ? cmulc(x, w) : cmul(x, w);
-    }
-    row[zpad<Z2>(j)] = x;
-  }
-}
-
-template <typename T, typename C, int Z1, int Z2>
-__global__ void __launch_bounds__(256) k_zfft_r2c(const T* __restrict__ in, C* __restrict__ out, long long nlines,
-                                                  const C* __restrict__ twZ) {
-  constexpr int N = Z1 * Z2;
-  constexpr int Q = 256 / Z2;        // complex pencils (two lines each) per CTA
-  constexpr int PS = Z1 * (Z2 + 1);  // padded pencil
-  extern __shared__ __align__(16) unsigned char zfft_smem[];
-  V2<T>* s = reinterpret_cast<V2<T>*>(zfft_smem);
-  const long long l0 = (long long)blockIdx.x * 2 * Q;
-  for (int i = threadIdx.x; i < Q * Z2; i += blockDim.x) {
-    const int p = i / Z2, n2 = i % Z2;
-    const long long la = l0 + 2 * p, lb = la + 1;
-    V2<T> a[Z1];
-#pragma unroll
-    for (int j = 0; j < Z1; ++j) {
-      const int z = j * Z2 + n2;
-      a[j].x = la < nlines ? in[la * N + z] : (T)0;
-      a[j].y = lb < nlines ? in[lb * N + z] : (T)0;
-    }
-    dft<T, Z1, false>(a);
-#pragma unroll
-    for (int j = 1; j < Z1; ++j) a[j] = cmul(a[j], ldt<T>(__ldg(&twZ[n2 * j])));
-#pragma unroll
-    for (int j = 0; j < Z1; ++j) s[p * PS + zpad<Z2>(j * Z2 + n2)] = a[j];
-  }
-  __syncthreads();
-  if constexpr (FCM_ZFFT_PAIR && 2 * Q * Z1 == 256 && Z2 % 2 == 0 && 96 % Z2 == 0) {
-    // half the threads would have an item: each row is shared by a lane pair
-    const int i = threadIdx.x >> 1, p = i / Z1, k1 = i % Z1;
-    pair_dft_row<T, Z2, false, C>(s + p * PS + zpad<Z2>(k1 * Z2), threadIdx.x & 1, nullptr, 0);
-  } else {
-    for (int i = threadIdx.x; i < Q * Z1; i += blockDim.x) {
-      const int p = i / Z1, k1 = i % Z1;
-      V2<T> b[Z2];
-#pragma unroll
-      for (int j = 0; j < Z2; ++j) b[j] = s[p * PS + zpad<Z2>(k1 * Z2 + j)];
-      dft<T, Z2, false>(b);
-#pragma unroll
-      for (int j = 0; j < Z2; ++j) s[p * PS + zpad<Z2>(k1 * Z2 + j)] = b[j];
-    }
-  }
-  __syncthreads();
-  constexpr int NZH = N / 2 + 1;  // the spectrum's row length (nzh); a constant divisor below
-  for (int i = threadIdx.x; i < Q * NZH; i += blockDim.x) {
-    const int p = i / NZH, k = i % NZH;
-    const long long la = l0 + 2 * p, lb = la + 1;
-    const V2<T> zk = s[p * PS + zpad<Z2>(zpos<Z1, Z2>(k))];
-    const V2<T> zm = s[p * PS + zpad<Z2>(zpos<Z1, Z2>((N - k) % N))];
-    if (la < nlines) {
-      C o;
-      o.x = (T)0.5 * (zk.x + zm.x);
-      o.y = (T)0.5 * (zk.y - zm.y);
-      out[la * NZH + k] = o;
-    }
-    if (lb < nlines) {
-      C o;
-      o.x = (T)0.5 * (zk.y + zm.y);
-      o.y = (T)0.5 * (zm.x - zk.x);
-      out[lb * NZH + k] = o;
-    }
-  }
-}
-
-template <typename T, typename C, int Z1, int Z2>
-__global__ void __launch_bounds__(256) k_zfft_c2r(const C* __restrict__ in, T* __restrict__ out, long long nlines,
-                                                  const C* __restrict__ twZ) {
-  constexpr int N = Z1 * Z2;
-  constexpr int Q = 256 / Z2;
-  constexpr int PS = Z1 * (Z2 + 1);
-  extern __shared__ __align__(16) unsigned char zfft_smem[];
-  V2<T>* s = reinterpret_cast<V2<T>*>(zfft_smem);
-  const long long l0 = (long long)blockIdx.x * 2 * Q;
-  // all of a thread's half-spectrum values are loaded before any is stored
-  constexpr int NZH = N / 2 + 1, ITEMS = (Q * NZH + 255) / 256;
-  V2<T> A[ITEMS], B[ITEMS];
-#pragma unroll
-  for (int u = 0; u < ITEMS; ++u) {
-    const int i = threadIdx.x + 256 * u;
-    const int p = i / NZH, k = i % NZH;
-    const long long la = l0 + 2 * p, lb = la + 1;
-    const bool live = i < Q * NZH;
-    A[u] = live && la < nlines ? ldt<T>(in[la * NZH + k]) : V2<T>{(T)0, (T)0};
-    B[u] = live && lb < nlines ? ldt<T>(in[lb * NZH + k]) : V2<T>{(T)0, (T)0};
-  }
-#pragma unroll
-  for (int u = 0; u < ITEMS; ++u) {
-    const int i = threadIdx.x + 256 * u;
-    if (i >= Q * NZH) break;
-    const int p = i / NZH, k = i % NZH;
-    V2<T> a = A[u], bb = B[u];
-    if (k == 0 || 2 * k == N) {
-      a.y = (T)0;
-      bb.y = (T)0;
-    }
-    s[p * PS + zpad<Z2>(zpos<Z1, Z2>(k))] = V2<T>{a.x - bb.y, a.y + bb.x};
-    if (k > 0 && 2 * k < N) s[p * PS + zpad<Z2>(zpos<Z1, Z2>(N - k))] = V2<T>{a.x + bb.y, bb.x - a.y};
-  }
-  __syncthreads();
-  if constexpr (FCM_ZFFT_PAIR && 2 * Q * Z1 == 256 && Z2 % 2 == 0 && 96 % Z2 == 0) {
-    // half the threads would have an item: each row is shared by a lane pair
-    const int i = threadIdx.x >> 1, p = i / Z1, k1 = i % Z1;
-    pair_dft_row<T, Z2, true, C>(s + p * PS + zpad<Z2>(k1 * Z2), threadIdx.x & 1, twZ, k1);
-  } else {
-    for (int i = threadIdx.x; i < Q * Z1; i += blockDim.x) {
-      const int p = i / Z1, k1 = i % Z1;
-      V2<T> b[Z2];
-#pragma unroll
-      for (int j = 0; j < Z2; ++j) b[j] = s[p * PS + zpad<Z2>(k1 * Z2 + j)];
-      dft<T, Z2, true>(b);
-#pragma unroll
-      for (int j = 1; j < Z2; ++j) b[j] = cmulc(b[j], ldt<T>(__ldg(&twZ[j * k1])));
-#pragma unroll
-      for (int j = 0; j < Z2; ++j) s[p * PS + zpad<Z2>(k1 * Z2 + j)] = b[j];
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < Q * Z2; i += blockDim.x) {
-    const int p = i / Z2, n2 = i % Z2;
-    const long long la = l0 + 2 * p, lb = la + 1;
-    V2<T> a[Z1];
-#pragma unroll
-    for (int j = 0; j < Z1; ++j) a[j] = s[p * PS + zpad<Z2>(j * Z2 + n2)];
-    dft<T, Z1, true>(a);
-#pragma unroll
-    for (int j = 0; j < Z1; ++j) {
-      const int z = j * Z2 + n2;
-      if (la < nlines) out[la * N + z] = a[j].x;
-      if (lb < nlines) out[lb * N + z] = a[j].y;
-    }
-  }
-}
-
-// Whether the y pass's first step loads two items per thread before transforming
-// either (where the items divide evenly among the threads); off: at 512 points it
-// measured 1% slower.
-#ifndef FCM_YFFT_BATCH
-#define FCM_YFFT_BATCH 0
-#endif
-
-// C2C along y, in place: blockIdx.y = x-plane (3 nx per grid), TK kz per CTA.
-// Both directions split NY = Y1 Y2 the same way (input n = j Y2 + n2, output
-// k = k1 + Y1 k2): Y1-point DFTs over j, the twiddles W_NY^(n2 k1) (conjugated for
-// the inverse), Y2-point DFTs over n2.  The first step reads its pencils straight
-// into registers and writes them to shared memory (an asynchronous-copy prologue
-// measured slower here), the second writes the result to the spectrum.
-template <typename T, typename C, int Y1, int Y2, int TK, bool INV>
-__global__ void __launch_bounds__(256) k_yfft(C* __restrict__ spec, int nzh, const C* __restrict__ twY) {
-  constexpr int NY = Y1 * Y2;
-  extern __shared__ __align__(16) unsigned char yfft_smem[];
-  V2<T>* s = reinterpret_cast<V2<T>*>(yfft_smem);  // [NY][TK]
-  const int k0 = (int)blockIdx.x * TK;
-  C* base = spec + (long long)blockIdx.y * NY * nzh + k0;
-  // first step: IPT items per thread when they divide evenly (every item's loads
-  // issued before any transform), else one item at a time
-  constexpr int IPT = (FCM_YFFT_BATCH && (Y2 * TK) % 256 == 0 && Y2 * TK / 256 <= 2) ? Y2 * TK / 256 : 1;
-  for (int i0 = threadIdx.x; i0 < Y2 * TK; i0 += IPT * blockDim.x) {
-    V2<T> a[IPT][Y1];
-#pragma unroll
-    for (int u = 0; u < IPT; ++u) {
-      const int i = i0 + u * blockDim.x, kzl = i % TK, n2 = i / TK;
-      const bool live = i < Y2 * TK && k0 + kzl < nzh;
-#pragma unroll
-      for (int j = 0; j < Y1; ++j)
-        a[u][j] = live ? ldt<T>(base[(long long)(j * Y2 + n2) * nzh + kzl]) : V2<T>{(T)0, (T)0};
-    }
-#pragma unroll
-    for (int u = 0; u < IPT; ++u) {
-      const int i = i0 + u * blockDim.x, kzl = i % TK, n2 = i / TK;
-      if (i >= Y2 * TK) break;
-      dft<T, Y1, INV>(a[u]);
-#pragma unroll
-      for (int j = 1; j < Y1; ++j) {
-        const V2<T> w = ldt<T>(__ldg(&twY[n2 * j]));
-        a[u][j] = INV ? cmulc(a[u][j], w) : cmul(a[u][j], w);
-      }
-#pragma unroll
-      for (int j = 0; j < Y1; ++j) s[(j * Y2 + n2) * TK + kzl] = a[u][j];
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < Y1 * TK; i += blockDim.x) {
-    const int kzl = i % TK, k1 = i / TK;
-    if (k0 + kzl >= nzh) continue;
-    V2<T> b[Y2];
-#pragma unroll
-    for (int j = 0; j < Y2; ++j) b[j] = s[(k1 * Y2 + j) * TK + kzl];
-    dft<T, Y2, INV>(b);
-#pragma unroll
-    for (int j = 0; j < Y2; ++j) {
-      C o;
-      o.x = b[j].x;
-      o.y = b[j].y;
-      base[(long long)(k1 + Y1 * j) * nzh + kzl] = o;
-    }
-  }
-}
-
-// ------------------------------------------------------------------ (y, z) transforms, a CTA per plane
-// Grids with ny == nz = N up to 96 points: one (component, x-plane) per CTA, so the
-// z and y transforms of a plane take one pass over HBM each way instead of two.
-// The CTA's shared memory holds the plane's half spectrum [N][N/2 + 1].  Forward:
-// the rows are transformed two at a time (as k_zfft_r2c does) and every mode of a
-// pencil (y, y + 1) is stored into the plane buffer: Z(k) at row y, column k for
-// k <= N/2, at row y + 1, column N - k above; then the two lines' spectra are
-// separated in place, the columns transformed along y and written.  The inverse
-// runs the same steps backwards.  The arithmetic is that of k_zfft_* and k_yfft
-// step for step.  (Planes of 256 points split over a cluster of 4 CTAs, the modes
-// exchanged through distributed shared memory, took 280 us against 174 us for the
-// separate passes: two 102 KB CTAs per SM left the phases between barriers latency
-// bound at 15% of DRAM throughput.)
-template <typename T, typename C, int N1, int N2>
-__global__ void __launch_bounds__(256) k_yz_r2c(const T* __restrict__ in, C* __restrict__ out,
-                                                const C* __restrict__ twY, const C* __restrict__ twZ) {
-  constexpr int N = N1 * N2, KS = N / 2 + 1, PEN = N / 2;
-  constexpr int Q = 256 / N2, PS = N1 * (N2 + 1);
-  extern __shared__ __align__(16) unsigned char yz_smem[];
-  V2<T>* buf = reinterpret_cast<V2<T>*>(yz_smem);  // [N][KS]
-  V2<T>* s = buf + N * KS;                         // [Q][PS]
-  const long long plane = (long long)blockIdx.x;
-  const T* src = in + plane * N * N;
-  for (int p0 = 0; p0 < PEN; p0 += Q) {
-    for (int i = threadIdx.x; i < Q * N2; i += blockDim.x) {
-      const int p = i / N2, n2 = i % N2;
-      if (p0 + p >= PEN) continue;
-      const T* la = src + (long long)(2 * (p0 + p)) * N;
-      V2<T> a[N1];
-#pragma unroll
-      for (int j = 0; j < N1; ++j) a[j] = V2<T>{la[j * N2 + n2], la[N + j * N2 + n2]};
-      dft<T, N1, false>(a);
-#pragma unroll
-      for (int j = 1; j < N1; ++j) a[j] = cmul(a[j], ldt<T>(__ldg(&twZ[n2 * j])));
-#pragma unroll
-      for (int j = 0; j < N1; ++j) s[p * PS + zpad<N2>(j * N2 + n2)] = a[j];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < Q * N1; i += blockDim.x) {
-      const int p = i / N1, k1 = i % N1;
-      if (p0 + p >= PEN) continue;
-      V2<T> b[N2];
-#pragma unroll
-      for (int j = 0; j < N2; ++j) b[j] = s[p * PS + zpad<N2>(k1 * N2 + j)];
-      dft<T, N2, false>(b);
-      const int y = 2 * (p0 + p);
-#pragma unroll
-      for (int j = 0; j < N2; ++j) {
-        const int k = k1 + N1 * j;
-        buf[2 * k <= N ? y * KS + k : (y + 1) * KS + (N - k)] = b[j];
-      }
-    }
-    __syncthreads();
-  }
-  for (int i = threadIdx.x; i < (N / 2) * KS; i += blockDim.x) {
-    const int q = i / KS, k = i % KS;
-    V2<T>* ra = buf + 2 * q * KS + k;
-    const V2<T> zk = ra[0];
-    const V2<T> zm = (k == 0 || 2 * k == N) ? zk : ra[KS];
-    ra[0] = V2<T>{(T)0.5 * (zk.x + zm.x), (T)0.5 * (zk.y - zm.y)};
-    ra[KS] = V2<T>{(T)0.5 * (zk.y + zm.y), (T)0.5 * (zm.x - zk.x)};
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < N2 * KS; i += blockDim.x) {
-    const int k = i % KS, n2 = i / KS;
-    V2<T> a[N1];
-#pragma unroll
-    for (int j = 0; j < N1; ++j) a[j] = buf[(j * N2 + n2) * KS + k];
-    dft<T, N1, false>(a);
-#pragma unroll
-    for (int j = 1; j < N1; ++j) a[j] = cmul(a[j], ldt<T>(__ldg(&twY[n2 * j])));
-#pragma unroll
-    for (int j = 0; j < N1; ++j) buf[(j * N2 + n2) * KS + k] = a[j];
-  }
-  __syncthreads();
-  C* dst = out + plane * N * KS;
-  for (int i = threadIdx.x; i < N1 * KS; i += blockDim.x) {
-    const int k = i % KS, k1 = i / KS;
-    V2<T> b[N2];
-#pragma unroll
-    for (int j = 0; j < N2; ++j) b[j] = buf[(k1 * N2 + j) * KS + k];
-    dft<T, N2, false>(b);
-#pragma unroll
-    for (int j = 0; j < N2; ++j) {
-      C o;
-      o.x = b[j].x;
-      o.y = b[j].y;
-      dst[(k1 + N1 * j) * KS + k] = o;
-    }
-  }
-}
-
-template <typename T, typename C, int N1, int N2>
-__global__ void __launch_bounds__(256) k_yz_c2r(const C* __restrict__ in, T* __restrict__ out,
-                                                const C* __restrict__ twY, const C* __restrict__ twZ) {
-  constexpr int N = N1 * N2, KS = N / 2 + 1, PEN = N / 2;
-  constexpr int Q = 256 / N2, PS = N1 * (N2 + 1);
-  extern __shared__ __align__(16) unsigned char yz_smem[];
-  V2<T>* buf = reinterpret_cast<V2<T>*>(yz_smem);
-  V2<T>* s = buf + N * KS;
-  const long long plane = (long long)blockIdx.x;
-  const C* src = in + plane * N * KS;
-  for (int i = threadIdx.x; i < N1 * KS; i += blockDim.x) {
-    const int k = i % KS, k1 = i / KS;
-    V2<T> b[N2];
-#pragma unroll
-    for (int j = 0; j < N2; ++j) b[j] = ldt<T>(src[(k1 + N1 * j) * KS + k]);
-    dft<T, N2, true>(b);
-#pragma unroll
-    for (int j = 1; j < N2; ++j) b[j] = cmulc(b[j], ldt<T>(__ldg(&twY[j * k1])));
-#pragma unroll
-    for (int j = 0; j < N2; ++j) buf[(k1 * N2 + j) * KS + k] = b[j];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < N2 * KS; i += blockDim.x) {
-    const int k = i % KS, n2 = i / KS;
-    V2<T> a[N1];
-#pragma unroll
-    for (int j = 0; j < N1; ++j) a[j] = buf[(j * N2 + n2) * KS + k];
-    dft<T, N1, true>(a);
-#pragma unroll
-    for (int j = 0; j < N1; ++j) buf[(j * N2 + n2) * KS + k] = a[j];
-  }
-  __syncthreads();
-  // row 2q <- Z(k) = A(k) + i B(k), row 2q + 1 <- Z(N - k), Im A, Im B ignored at kz = 0, N/2
-  for (int i = threadIdx.x; i < (N / 2) * KS; i += blockDim.x) {
-    const int q = i / KS, k = i % KS;
-    V2<T>* ra = buf + 2 * q * KS + k;
-    V2<T> a = ra[0], bb = ra[KS];
-    if (k == 0 || 2 * k == N) {
-      a.y = (T)0;
-      bb.y = (T)0;
-    }
-    ra[0] = V2<T>{a.x - bb.y, a.y + bb.x};
-    ra[KS] = V2<T>{a.x + bb.y, bb.x - a.y};
-  }
-  __syncthreads();
-  T* dsts = out + plane * N * N;
-  for (int p0 = 0; p0 < PEN; p0 += Q) {
-    for (int i = threadIdx.x; i < Q * N1; i += blockDim.x) {
-      const int p = i / N1, k1 = i % N1;
-      if (p0 + p >= PEN) continue;
-      const int y = 2 * (p0 + p);
-      V2<T> b[N2];
-#pragma unroll
-      for (int j = 0; j < N2; ++j) {
-        const int k = k1 + N1 * j;
-        b[j] = buf[2 * k <= N ? y * KS + k : (y + 1) * KS + (N - k)];
-      }
-      dft<T, N2, true>(b);
-#pragma unroll
-      for (int j = 1; j < N2; ++j) b[j] = cmulc(b[j], ldt<T>(__ldg(&twZ[j * k1])));
-#pragma unroll
-      for (int j = 0; j < N2; ++j) s[p * PS + zpad<N2>(k1 * N2 + j)] = b[j];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < Q * N2; i += blockDim.x) {
-      const int p = i / N2, n2 = i % N2;
-      if (p0 + p >= PEN) continue;
-      V2<T> a[N1];
-#pragma unroll
-      for (int j = 0; j < N1; ++j) a[j] = s[p * PS + zpad<N2>(j * N2 + n2)];
-      dft<T, N1, true>(a);
-      T* la = dsts + (long long)(2 * (p0 + p)) * N;
-#pragma unroll
-      for (int j = 0; j < N1; ++j) {
-        la[j * N2 + n2] = a[j].x;
-        la[N + j * N2 + n2] = a[j].y;
-      }
-    }
-    __syncthreads();
-  }
-}
-
 }  // namespace
 
 KParams make_kparams(const Ctx& c) {
@@ -1331,203 +794,7 @@ int xfft_dispatch(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s, 
 
 }  // namespace
 
-// exp(-2 pi i k / 96) into the constant tables of the current device (once per device).
-int xfft_tables_init() {
-  static std::mutex mu;
-  static std::vector<bool> done;
-  int dev = 0;
-  FCM_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lock(mu);
-  if ((int)done.size() <= dev) done.resize(dev + 1, false);
-  if (done[dev]) return FCM_OK;
-  const double PI = 3.14159265358979323846264338327950288;
-  double2 wd[96];
-  float2 wf[96];
-  for (int j = 0; j < 96; ++j) {
-    wd[j] = make_double2(std::cos(2.0 * PI * j / 96.0), -std::sin(2.0 * PI * j / 96.0));
-    wf[j] = make_float2((float)wd[j].x, (float)wd[j].y);
-  }
-  FCM_CUDA(cudaMemcpyToSymbol(c_w96d, wd, sizeof(wd)));
-  FCM_CUDA(cudaMemcpyToSymbol(c_w96f, wf, sizeof(wf)));
-  done[dev] = true;
-  return FCM_OK;
-}
-
-namespace {
-
-// Calls f(integral_constant<N1>, integral_constant<N2>) for a supported length n.
-template <typename F>
-int with_factors(int n, F&& f) {
-  using std::integral_constant;
-  switch (n) {
-    case 8: return f(integral_constant<int, 2>{}, integral_constant<int, 4>{});
-    case 12: return f(integral_constant<int, 3>{}, integral_constant<int, 4>{});
-    case 16: return f(integral_constant<int, 4>{}, integral_constant<int, 4>{});
-    case 24: return f(integral_constant<int, 4>{}, integral_constant<int, 6>{});
-    case 32: return f(integral_constant<int, 4>{}, integral_constant<int, 8>{});
-    case 48: return f(integral_constant<int, 6>{}, integral_constant<int, 8>{});
-    case 64: return f(integral_constant<int, 8>{}, integral_constant<int, 8>{});
-    case 96: return f(integral_constant<int, 8>{}, integral_constant<int, 12>{});
-    case 128: return f(integral_constant<int, 8>{}, integral_constant<int, 16>{});
-    case 192: return f(integral_constant<int, 12>{}, integral_constant<int, 16>{});
-    case 256: return f(integral_constant<int, 16>{}, integral_constant<int, 16>{});
-    case 384: return f(integral_constant<int, 16>{}, integral_constant<int, 24>{});
-    case 512: return f(integral_constant<int, 16>{}, integral_constant<int, 32>{});
-    default: break;
-  }
-  set_error("(y, z) transforms: unsupported length " + std::to_string(n));
-  return FCM_ERR_INVALID;
-}
-
-// Dynamic shared memory above the default 48 KB for `kernel`, set once per kernel
-// and device (kernels of one signature share the template instance, so the cache
-// is keyed by the kernel's address).
-template <typename K>
-int smem_attr_once(K kernel, size_t smem) {
-  if (smem <= 48 * 1024) return FCM_OK;
-  static std::mutex mu;
-  static std::vector<std::pair<int, const void*>> done;
-  int dev = 0;
-  FCM_CUDA(cudaGetDevice(&dev));
-  const std::pair<int, const void*> key(dev, reinterpret_cast<const void*>(kernel));
-  std::lock_guard<std::mutex> lock(mu);
-  if (std::find(done.begin(), done.end(), key) == done.end()) {
-    FCM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    done.push_back(key);
-  }
-  return FCM_OK;
-}
-
-// z passes of Z1 x Z2 points, Q = 256 / Z2 complex pencils (two real lines each)
-// per CTA.
-template <typename T, int Z1, int Z2>
-int zfft_run(const T* r, typename cplx_t<T>::type* spec, T* r_out, long long nlines, bool inverse,
-             const typename cplx_t<T>::type* tw, cudaStream_t s) {
-  using C = typename cplx_t<T>::type;
-  constexpr int Q = 256 / Z2;
-  const size_t smem = (size_t)Q * Z1 * (Z2 + 1) * sizeof(C);
-  const unsigned grid = (unsigned)((nlines + 2 * Q - 1) / (2 * Q));
-  if (inverse) {
-    FCM_TRY(smem_attr_once(k_zfft_c2r<T, C, Z1, Z2>, smem));
-    k_zfft_c2r<T, C, Z1, Z2><<<grid, 256, smem, s>>>(spec, r_out, nlines, tw);
-  } else {
-    FCM_TRY(smem_attr_once(k_zfft_r2c<T, C, Z1, Z2>, smem));
-    k_zfft_r2c<T, C, Z1, Z2><<<grid, 256, smem, s>>>(r, spec, nlines, tw);
-  }
-  FCM_LAUNCH_CHECK();
-  return (int)FCM_OK;
-}
-
-// At 512 points the split is 32 x 16 (the middle step then has Q Z1 = 512 items, two
-// per thread; 16 x 32 left half the CTA idle there), elsewhere the table's.
-#ifndef FCM_ZFFT512_Z1
-#define FCM_ZFFT512_Z1 16
-#endif
-
-template <typename T>
-int zfft(const Ctx& c, const T* r, typename cplx_t<T>::type* spec, T* r_out, long long nlines, bool inverse,
-         cudaStream_t s) {
-  using C = typename cplx_t<T>::type;
-  const C* tw = (const C*)c.d_ztw32;
-  return with_factors(c.g.nz, [&](auto a, auto b) -> int {
-    constexpr int Z1 = decltype(a)::value, Z2 = decltype(b)::value;
-    if constexpr (Z1 * Z2 == 512)
-      return zfft_run<T, FCM_ZFFT512_Z1, 512 / FCM_ZFFT512_Z1>(r, spec, r_out, nlines, inverse, tw, s);
-    else
-      return zfft_run<T, Z1, Z2>(r, spec, r_out, nlines, inverse, tw, s);
-  });
-}
-
-// y pass: 16 kz per CTA (rows of 128 bytes in FP32; the second step has Y1 * 16 =
-// 256 items, one per thread, for Y1 = 16); 64 KB of shared memory at 512 points.
-template <typename T>
-int yfft(const Ctx& c, typename cplx_t<T>::type* spec, int nplanes, bool inverse, cudaStream_t s) {
-  using C = typename cplx_t<T>::type;
-  const C* tw = (const C*)c.d_ytw32;
-  const int nzh = c.g.nzh;
-  return with_factors(c.g.ny, [&](auto a, auto b) -> int {
-    constexpr int Y1 = decltype(a)::value, Y2 = decltype(b)::value;
-    constexpr int TK = 16;
-    const size_t smem = (size_t)Y1 * Y2 * TK * sizeof(C);
-    const dim3 grid((unsigned)((nzh + TK - 1) / TK), (unsigned)nplanes);
-    if (inverse) {
-      FCM_TRY(smem_attr_once(k_yfft<T, C, Y1, Y2, TK, true>, smem));
-      k_yfft<T, C, Y1, Y2, TK, true><<<grid, 256, smem, s>>>(spec, nzh, tw);
-    } else {
-      FCM_TRY(smem_attr_once(k_yfft<T, C, Y1, Y2, TK, false>, smem));
-      k_yfft<T, C, Y1, Y2, TK, false><<<grid, 256, smem, s>>>(spec, nzh, tw);
-    }
-    FCM_LAUNCH_CHECK();
-    return (int)FCM_OK;
-  });
-}
-
-// One launch of the per-plane kernels over `planes` (component, x-plane) planes of
-// grids with ny == nz = N1 N2, or (prepare) their shared-memory attribute.
-template <int N1, int N2>
-int yz_plane_go(const Ctx& c, const float* r, cufftComplex* spec, float* r_out, long long planes, bool inverse,
-                cudaStream_t s, bool prepare) {
-  using C = cufftComplex;
-  constexpr int N = N1 * N2;
-  const size_t smem = ((size_t)N * (N / 2 + 1) + (size_t)(256 / N2) * N1 * (N2 + 1)) * sizeof(C);
-  auto kf = k_yz_r2c<float, C, N1, N2>;
-  auto ki = k_yz_c2r<float, C, N1, N2>;
-  if (prepare) {
-    FCM_TRY(xfft_smem_attr(kf, smem));
-    return xfft_smem_attr(ki, smem);
-  }
-  const C* twY = (const C*)c.d_ytw32;
-  const C* twZ = (const C*)c.d_ztw32;
-  if (inverse)
-    ki<<<(unsigned)planes, 256, smem, s>>>(spec, r_out, twY, twZ);
-  else
-    kf<<<(unsigned)planes, 256, smem, s>>>(r, spec, twY, twZ);
-  FCM_LAUNCH_CHECK();
-  return FCM_OK;
-}
-
-// Square (y, z) planes of these sizes take the per-plane kernels (55 KB of shared
-// memory at 96 points, four CTAs per SM).
-bool yz_plane_ok(const Ctx& c) {
-  switch (c.g.nz) {
-    case 16: case 32: case 48: case 64: case 96: return c.g.ny == c.g.nz;
-    default: return false;
-  }
-}
-
-int yz_plane(const Ctx& c, const float* r, cufftComplex* spec, float* r_out, long long planes, bool inverse,
-             cudaStream_t s, bool prepare) {
-  switch (c.g.nz) {
-    case 16: return yz_plane_go<4, 4>(c, r, spec, r_out, planes, inverse, s, prepare);
-    case 32: return yz_plane_go<4, 8>(c, r, spec, r_out, planes, inverse, s, prepare);
-    case 48: return yz_plane_go<6, 8>(c, r, spec, r_out, planes, inverse, s, prepare);
-    case 64: return yz_plane_go<8, 8>(c, r, spec, r_out, planes, inverse, s, prepare);
-    case 96: return yz_plane_go<8, 12>(c, r, spec, r_out, planes, inverse, s, prepare);
-    default: break;
-  }
-  set_error("(y, z) plane transforms: unsupported length " + std::to_string(c.g.nz));
-  return FCM_ERR_INVALID;
-}
-
-}  // namespace
-
-// The (y, z) transforms of `members` consecutive FP32 grids of c's shape: forward
-// from the real grid r into the spectrum, inverse from the spectrum (overwritten)
-// into r.  Square (y, z) planes up to 96 points take the per-plane kernels, other
-// shapes the z and y passes one after the other.
-int launch_yz_forward(const Ctx& c, const float* r, cufftComplex* spec, int members, cudaStream_t s) {
-  if (yz_plane_ok(c)) return yz_plane(c, r, spec, nullptr, 3LL * c.g.nx * members, false, s, false);
-  const long long nlines = 3LL * c.g.nx * c.g.ny * members;
-  FCM_TRY(zfft<float>(c, r, spec, nullptr, nlines, false, s));
-  return yfft<float>(c, spec, 3 * c.g.nx * members, false, s);
-}
-
-int launch_yz_inverse(const Ctx& c, cufftComplex* spec, float* r, int members, cudaStream_t s) {
-  if (yz_plane_ok(c)) return yz_plane(c, nullptr, spec, r, 3LL * c.g.nx * members, true, s, false);
-  const long long nlines = 3LL * c.g.nx * c.g.ny * members;
-  FCM_TRY(yfft<float>(c, spec, 3 * c.g.nx * members, true, s));
-  return zfft<float>(c, nullptr, spec, r, nlines, true, s);
-}
+int xfft_tables_init() { return w96_upload(); }
 
 template <typename T>
 int launch_xfft_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s) {
@@ -1536,8 +803,6 @@ int launch_xfft_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream
 
 template <typename T>
 int xfft_prepare(const Ctx& c) {
-  if constexpr (sizeof(T) == 4)
-    if (c.yz32_cap && yz_plane_ok(c)) FCM_TRY(yz_plane(c, nullptr, nullptr, nullptr, 0, false, 0, true));
   return xfft_dispatch<T>(c, nullptr, 0, true);
 }
 
