@@ -599,22 +599,43 @@ int noise_dev(Ctx* c, uint64_t seed, uint64_t counter, const uint64_t* d_args = 
   return FCM_OK;
 }
 
-// gmres_solver.cpp:72-83 on device vectors (system size).
-int saddle_matvec(Ctx* c, int prec, const double* in, double* out) {
-  FCM_TRY(mobility_dev(c, prec, in, out));
-  FCM_TRY(launch_multiply_K(*c, c->d_qm, in + 3 * (size_t)c->Nb, out, 1.0, c->stream));
-  FCM_TRY(launch_multiply_KT(*c, c->d_qm, in, out + 3 * (size_t)c->Nb, -1.0, nullptr, 0.0, c->stream));
+__global__ void k_gm_loop_cond(cudaGraphConditionalHandle h, const GmState* __restrict__ gm, StepRecord* sd,
+                               int enter, int limit) {
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  if (enter) sd->guard = 0;
+  else ++sd->guard;
+  cudaGraphSetConditional(h, (!gm->done && sd->guard < limit) ? 1u : 0u);
+}
+
+int loop_condition(Ctx* c, cudaGraphConditionalHandle h, StepRecord* sd, int enter, int limit) {
+  k_gm_loop_cond<<<1, 32, 0, c->stream>>>(h, c->gm, sd, enter, limit);
+  FCM_LAUNCH_CHECK();
   return FCM_OK;
 }
 
+// gmres_solver.cpp:72-83 on device vectors (system size).
+template <typename T>
+int saddle_t(Ctx* c, const BlobTable<T>& t, const double* in, double* out) {
+  FCM_TRY(spread_t<T>(c, t, in));
+  FCM_TRY(stokes_t<T>(c));
+  NvtxRange r(sizeof(T) == 8 ? "fcm interp fp64" : "fcm interp fp32");
+  return launch_saddle_end<T>(*c, t, grid_of<T>(c).r, c->d_qm, in, out, c->stream);
+}
+int saddle_matvec(Ctx* c, int prec, const double* in, double* out) {
+  return prec == 0 ? saddle_t<double>(c, c->g64.blobs, in, out) : saddle_t<float>(c, c->g32.blobs, in, out);
+}
+
 // One Arnoldi iteration of the device-side GMRES on c->stream:
-//   z_in = Q[k]; z = P^-1 z_in; w = A z; orthogonalise, normalise, Givens.
-int enqueue_gm_iteration(Ctx* c, int prec) {
-  FCM_TRY(gm_fetch(*c, c->d_sys_b, c->stream));
-  FCM_TRY(launch_pinv(*c, c->d_qm, c->d_sys_b, c->d_sys_a, c->stream));
+//   z = P^-1 Q[k]; w = A z; orthogonalise, normalise, Givens
+// and, in a device loop (sd given), the loop's condition.
+int enqueue_gm_iteration(Ctx* c, int prec, cudaGraphConditionalHandle handle = {}, StepRecord* sd = nullptr,
+                         int limit = 0) {
+  FCM_TRY(launch_pinv_column(*c, c->d_qm, c->d_sys_a, c->stream));
   FCM_TRY(saddle_matvec(c, prec, c->d_sys_a, c->d_sys_b));
+  if (gm_one_launch(*c)) return gm_arnoldi(*c, c->d_sys_b, c->stream, handle, sd, limit);
   FCM_TRY(gm_orthogonalize(*c, c->d_sys_b, c->stream));
-  return FCM_OK;
+  if (!sd) return FCM_OK;
+  return loop_condition(c, handle, sd, 0, limit);
 }
 
 // The Arnoldi iteration captured once per precision in a CUDA graph on the
@@ -850,14 +871,6 @@ int divU_dev(Ctx* c, double* out) {
 
 // Condition of a GMRES while-loop: go on while the solve is not done, for at
 // most `limit` iterations of this loop.
-__global__ void k_gm_loop_cond(cudaGraphConditionalHandle h, const GmState* __restrict__ gm, StepRecord* sd,
-                               int enter, int limit) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (enter) sd->guard = 0;
-  else ++sd->guard;
-  cudaGraphSetConditional(h, (!gm->done && sd->guard < limit) ? 1u : 0u);
-}
-
 __global__ void k_step_begin(StepRecord* sd) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   sd->iters = 0;
@@ -1016,16 +1029,12 @@ int enqueue_gmres_loop(Ctx* c, int prec, const double* d_b, double* d_x, double 
   FCM_TRY(gm_init(*c, d_b, tol, max_iter, c->stream, d_tol));
   cudaGraphConditionalHandle h;
   FCM_TRY(new_handle(c->stream, &h));
-  k_gm_loop_cond<<<1, 32, 0, c->stream>>>(h, c->gm, c->d_step, 1, max_iter);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(loop_condition(c, h, c->d_step, 1, max_iter));
   cudaGraph_t body = nullptr;
   FCM_TRY(add_while_node(c->stream, h, &body));
   const long long l0 = launch_count();
   FCM_TRY(capture_body(c, body, bs, [&] {
-    FCM_TRY(enqueue_gm_iteration(c, prec));
-    k_gm_loop_cond<<<1, 32, 0, c->stream>>>(h, c->gm, c->d_step, 0, max_iter);
-    FCM_LAUNCH_CHECK();
-    return (int)FCM_OK;
+    return enqueue_gm_iteration(c, prec, h, c->d_step, max_iter);
   }));
   *iter_kernels = launch_count() - l0;
   FCM_TRY(gm_finish(*c, c->d_sys_b, c->stream));

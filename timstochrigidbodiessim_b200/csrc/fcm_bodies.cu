@@ -5,53 +5,11 @@
 // recomputed from q on every use, as the reference does
 // (collection_of_rigid_bodies.cpp:707-757, gmres_solver.cpp:97-134).
 #include "fcm_internal.cuh"
+#include "fcm_rigid.cuh"
 
 namespace fcm {
 
 namespace {
-
-// quaternion.cpp:61-103 with round-to-nearest intrinsics, so the product order
-// (and therefore every bit) matches a non-contracting CPU build.
-__device__ __forceinline__ void quat_matrix(const double* q, double R[3][3]) {
-  const double s = q[0], v0 = q[1], v1 = q[2], v2 = q[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) R[i][j] = (i == j) ? 1.0 : 0.0;
-  double t = __dmul_rn(__dmul_rn(2.0, v0), v0);
-  R[1][1] = __dsub_rn(R[1][1], t); R[2][2] = __dsub_rn(R[2][2], t);
-  t = __dmul_rn(__dmul_rn(2.0, v1), v1);
-  R[0][0] = __dsub_rn(R[0][0], t); R[2][2] = __dsub_rn(R[2][2], t);
-  t = __dmul_rn(__dmul_rn(2.0, v2), v2);
-  R[0][0] = __dsub_rn(R[0][0], t); R[1][1] = __dsub_rn(R[1][1], t);
-  t = __dmul_rn(__dmul_rn(2.0, v0), v1);
-  R[1][0] = __dadd_rn(R[1][0], t); R[0][1] = __dadd_rn(R[0][1], t);
-  t = __dmul_rn(__dmul_rn(2.0, v0), v2);
-  R[2][0] = __dadd_rn(R[2][0], t); R[0][2] = __dadd_rn(R[0][2], t);
-  t = __dmul_rn(__dmul_rn(2.0, v1), v2);
-  R[1][2] = __dadd_rn(R[1][2], t); R[2][1] = __dadd_rn(R[2][1], t);
-  t = __dmul_rn(__dmul_rn(2.0, s), v2);
-  R[1][0] = __dadd_rn(R[1][0], t); R[0][1] = __dsub_rn(R[0][1], t);
-  t = __dmul_rn(__dmul_rn(2.0, s), v1);
-  R[2][0] = __dsub_rn(R[2][0], t); R[0][2] = __dadd_rn(R[0][2], t);
-  t = __dmul_rn(__dmul_rn(2.0, s), v0);
-  R[2][1] = __dadd_rn(R[2][1], t); R[1][2] = __dsub_rn(R[1][2], t);
-}
-
-__device__ __forceinline__ void rot(const double R[3][3], const double* v, double* o) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-    o[i] = __dadd_rn(__dadd_rn(__dmul_rn(R[i][0], v[0]), __dmul_rn(R[i][1], v[1])), __dmul_rn(R[i][2], v[2]));
-}
-__device__ __forceinline__ void rotT(const double R[3][3], const double* v, double* o) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) o[i] = R[0][i] * v[0] + R[1][i] * v[1] + R[2][i] * v[2];
-}
-__device__ __forceinline__ void cross3(const double* a, const double* b, double* c) {
-  c[0] = a[1] * b[2] - a[2] * b[1];
-  c[1] = a[2] * b[0] - a[0] * b[2];
-  c[2] = a[0] * b[1] - a[1] * b[0];
-}
 
 // collection_of_rigid_bodies.cpp:155-193: Y = x + R r_m, wrapped p - L floor(p/L).
 // Body n's shape starts at ref + n*rs (rs = 0: one shape shared by all bodies).
@@ -73,53 +31,11 @@ __global__ void k_fill_blob_pos(const double* __restrict__ x, const double* __re
   }
 }
 
-// collection_of_rigid_bodies.cpp:707-731: out_m (+)= U + Omega x (R r_m).
-__device__ __forceinline__ void multiply_K_one(const double* __restrict__ q, const double* __restrict__ ref, int rs,
-                                               const double* __restrict__ in, double* __restrict__ out, int i,
-                                               int nb, int subtract) {
-  const int n = i / nb, m = i - n * nb;
-  double R[3][3];
-  quat_matrix(q + 4 * n, R);
-  double r[3], c[3];
-  rot(R, ref + (size_t)n * rs + 3 * m, r);
-  cross3(in + 6 * n + 3, r, c);
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double v = in[6 * n + d] + c[d];
-    out[3 * i + d] = subtract ? out[3 * i + d] - v : v;
-  }
-}
-
 __global__ void k_multiply_K(const double* __restrict__ q, const double* __restrict__ ref, int rs,
                              const double* __restrict__ in, double* __restrict__ out, int Nb, int nb, int subtract) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Nb) return;
   multiply_K_one(q, ref, rs, in, out, i, nb, subtract);
-}
-
-// collection_of_rigid_bodies.cpp:733-757: F = sum lambda_m, T = sum (R r_m) x lambda_m;
-// out = scale * K^T in + add_scale * add.
-__device__ __forceinline__ void multiply_KT_one(const double* __restrict__ q, const double* __restrict__ ref, int rs,
-                                                const double* __restrict__ in, double* __restrict__ out, int n,
-                                                int nb, double scale, const double* __restrict__ add,
-                                                double add_scale) {
-  double R[3][3];
-  quat_matrix(q + 4 * n, R);
-  ref += (size_t)n * rs;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int m = 0; m < nb; ++m) {
-    const double* l = in + 3 * (n * nb + m);
-    double r[3], c[3];
-    rot(R, ref + 3 * m, r);
-    cross3(r, l, c);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      acc[d] += l[d];
-      acc[3 + d] += c[d];
-    }
-  }
-#pragma unroll
-  for (int d = 0; d < 6; ++d) out[6 * n + d] = scale * acc[d] + (add ? add_scale * add[6 * n + d] : 0.0);
 }
 
 __global__ void k_multiply_KT(const double* __restrict__ q, const double* __restrict__ ref, int rs,
@@ -221,6 +137,17 @@ __global__ void k_pinv(const double* __restrict__ q, const double* __restrict__ 
                        const double* __restrict__ in, double* __restrict__ out, int M, int nb, int Nb) {
   extern __shared__ double sm[];
   pinv_block(q, ref, rs, Minv, ms, Nm, ns, in, out, M, nb, Nb, sm);
+}
+
+// The preconditioner on the newest Krylov column, in = Q[:, k] (k from the state): one
+// launch less per iteration than a copy of the column first.
+__global__ void k_pinv_column(const GmState* __restrict__ st, const double* __restrict__ Q, long long n,
+                              const double* __restrict__ q, const double* __restrict__ ref, int rs,
+                              const double* __restrict__ Minv, long long ms, const double* __restrict__ Nm, int ns,
+                              double* __restrict__ out, int M, int nb, int Nb) {
+  extern __shared__ double sm[];
+  if (st->done) return;
+  pinv_block(q, ref, rs, Minv, ms, Nm, ns, Q + (size_t)st->k * n, out, M, nb, Nb, sm);
 }
 
 // Rigid projection of blob velocities with ref_KTKinv
@@ -372,6 +299,17 @@ int launch_pinv(const Ctx& c, const double* qm, const double* in, double* out, c
   const size_t shm = sizeof(double) * warps * (size_t)(6 * c.nb + 12);
   k_pinv<<<(c.M + warps - 1) / warps, 32 * warps, shm, s>>>(qm, c.d_ref, c.ref_stride, c.d_Minv, c.minv_stride, c.d_N,
                                                                  c.n_stride, in, out, c.M, c.nb, c.Nb);
+  FCM_LAUNCH_CHECK();
+  return FCM_OK;
+}
+
+int launch_pinv_column(const Ctx& c, const double* qm, double* out, cudaStream_t s) {
+  if (c.M == 0) return FCM_OK;
+  const int warps = 4;
+  const size_t shm = sizeof(double) * warps * (size_t)(6 * c.nb + 12);
+  k_pinv_column<<<(c.M + warps - 1) / warps, 32 * warps, shm, s>>>(c.gm, c.d_Qm, c.nsys, qm, c.d_ref, c.ref_stride,
+                                                                   c.d_Minv, c.minv_stride, c.d_N, c.n_stride, out,
+                                                                   c.M, c.nb, c.Nb);
   FCM_LAUNCH_CHECK();
   return FCM_OK;
 }

@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "fcm_internal.cuh"
+#include "fcm_rigid.cuh"
 
 namespace fcm {
 
@@ -1825,10 +1826,10 @@ __global__ void k_interp_reduce(const int* __restrict__ base, const T* __restric
 // the eight lanes combine in a fixed butterfly.  Deterministic; 16 blobs per
 // 128-thread CTA.
 template <typename T>
-__global__ void __launch_bounds__(128) k_interp_reduce8(const int* __restrict__ base, const T* __restrict__ partial,
-                                                        int n, TileGeom g, double dx3, double* __restrict__ V) {
-  const int b = blockIdx.x * 16 + (threadIdx.x >> 3), k = threadIdx.x & 7;
-  double s0 = 0, s1 = 0, s2 = 0;
+__device__ __forceinline__ void interp_reduce8(const int* __restrict__ base, const T* __restrict__ partial, int n,
+                                               const TileGeom& g, int block, double& s0, double& s1, double& s2) {
+  const int b = block * 16 + (threadIdx.x >> 3), k = threadIdx.x & 7;
+  s0 = s1 = s2 = 0;
   if (b < n) {
     int f[3], cnt[3];
     blob_tiles(base, b, g, f, cnt);
@@ -1847,11 +1848,46 @@ __global__ void __launch_bounds__(128) k_interp_reduce8(const int* __restrict__ 
     s1 += __shfl_xor_sync(0xffffffffu, s1, off);
     s2 += __shfl_xor_sync(0xffffffffu, s2, off);
   }
-  if (b < n && k == 0) {
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128) k_interp_reduce8(const int* __restrict__ base, const T* __restrict__ partial,
+                                                        int n, TileGeom g, double dx3, double* __restrict__ V) {
+  const int b = blockIdx.x * 16 + (threadIdx.x >> 3);
+  double s0, s1, s2;
+  interp_reduce8<T>(base, partial, n, g, blockIdx.x, s0, s1, s2);
+  if (b < n && (threadIdx.x & 7) == 0) {
     V[3 * b] = s0 * dx3;
     V[3 * b + 1] = s1 * dx3;
     V[3 * b + 2] = s2 * dx3;
   }
+}
+
+// The end of the saddle-point product in one launch (three before, 4-8 us each whatever
+// the size): out[lambda] = M lambda - K U from the partials (blocks [0, rblocks), the sums
+// of k_interp_reduce8 with the rigid velocity of the blob subtracted), out[U] = -K^T lambda
+// (the blocks after them, one body per thread).
+template <typename T>
+__global__ void __launch_bounds__(128) k_saddle_end(const int* __restrict__ base, const T* __restrict__ partial, int n,
+                                                    TileGeom g, double dx3, int rblocks, const double* __restrict__ q,
+                                                    const double* __restrict__ ref, int rs,
+                                                    const double* __restrict__ in, double* __restrict__ out, int M,
+                                                    int nb) {
+  if ((int)blockIdx.x < rblocks) {
+    const int b = blockIdx.x * 16 + (threadIdx.x >> 3);
+    double s0, s1, s2;
+    interp_reduce8<T>(base, partial, n, g, blockIdx.x, s0, s1, s2);
+    if (b < n && (threadIdx.x & 7) == 0) {
+      double v[3];
+      blob_K_velocity(q, ref, rs, in + 3 * (size_t)n, b, nb, v);
+      out[3 * b] = __dsub_rn(__dmul_rn(s0, dx3), v[0]);  // rounded as the separate kernels do
+      out[3 * b + 1] = __dsub_rn(__dmul_rn(s1, dx3), v[1]);
+      out[3 * b + 2] = __dsub_rn(__dmul_rn(s2, dx3), v[2]);
+    }
+    return;
+  }
+  const int body = (blockIdx.x - rblocks) * 128 + threadIdx.x;
+  if (body < M) multiply_KT_one(q, ref, rs, in, out + 3 * (size_t)n, body, nb, -1.0, nullptr, 0.0);
 }
 
 // Spreading of grids that cannot be tiled: one CTA per blob, each thread owns
@@ -2071,50 +2107,75 @@ int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid
   return FCM_OK;
 }
 
+// The per-(blob, tile) partials of a tiled grid's interpolation; g receives the geometry.
+template <typename T>
+static int launch_interp_tiles(const Ctx& c, const BlobTable<T>& t, const T* grid, TileGeom& g, cudaStream_t s) {
+  g = tile_geom(c.g, t);
+  g.ycut = c.p.slip_channel ? c.g.ny / 2 : c.g.ny;  // fcm_fluid_solver.cpp:387-389
+  const int v = c.interp_variant[sizeof(T) == 8 ? 0 : 1];
+  // the tensor-core kernels copy 16-byte parts of the grid's rows (every caller's grid is
+  // an allocation of its own, so aligned; otherwise the 64-thread kernel)
+  const bool aligned = (reinterpret_cast<uintptr_t>(grid) & 15u) == 0;
+  if (v == 2) {
+    k_interp_rows<T, 2><<<t.ntiles, 32, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
+    FCM_LAUNCH_CHECK();
+    return FCM_OK;
+  }
+  if constexpr (sizeof(T) == 8) {
+    if (v == 1 && aligned) {
+      k_interp_mma64<<<std::min(t.ntiles, persistent_ctas(k_interp_mma64, 32, c.device)), 32, 0, s>>>(
+          t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles);
+      FCM_LAUNCH_CHECK();
+      return FCM_OK;
+    }
+  } else {
+    if (v == 3 && aligned) {
+      k_interp_mma<<<std::min(t.ntiles, persistent_ctas(k_interp_mma, 32, c.device)), 32, 0, s>>>(
+          t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles);
+      FCM_LAUNCH_CHECK();
+      return FCM_OK;
+    }
+    if (v == 1) {
+      k_interp_warp<T><<<t.ntiles, 32, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
+      FCM_LAUNCH_CHECK();
+      return FCM_OK;
+    }
+  }
+  k_interp_tiled<T><<<t.ntiles, 64, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
+  FCM_LAUNCH_CHECK();
+  return FCM_OK;
+}
+
 template <typename T>
 int launch_interp(const Ctx& c, const BlobTable<T>& t, const T* grid, double* dV, cudaStream_t s) {
   if (t.n == 0) return FCM_OK;
   const double dx3 = c.g.dx * c.g.dx * c.g.dx;
-  const int ycut = c.p.slip_channel ? c.g.ny / 2 : c.g.ny;  // fcm_fluid_solver.cpp:387-389
   if (t.tiled) {
-    TileGeom g = tile_geom(c.g, t);
-    g.ycut = ycut;
-    const int v = c.interp_variant[sizeof(T) == 8 ? 0 : 1];
-    if constexpr (sizeof(T) == 8) {
-      // FP64 variant 1; the kernel copies 16-byte parts of the grid's rows (every caller's
-      // grid is an allocation of its own, so aligned; otherwise the 64-thread kernel)
-      if (v == 1 && (reinterpret_cast<uintptr_t>(grid) & 15u) == 0) {
-        k_interp_mma64<<<std::min(t.ntiles, persistent_ctas(k_interp_mma64, 32, c.device)), 32, 0, s>>>(
-            t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles);
-        FCM_LAUNCH_CHECK();
-        k_interp_reduce8<T><<<(t.n + 15) / 16, 128, 0, s>>>(t.base, t.partial, t.n, g, dx3, dV);
-        FCM_LAUNCH_CHECK();
-        return FCM_OK;
-      }
-    }
-    if constexpr (sizeof(T) == 4) {
-      // the tensor-core kernel copies 16-byte rows of the grid asynchronously
-      if (v == 3 && (reinterpret_cast<uintptr_t>(grid) & 15u) == 0) {
-        k_interp_mma<<<std::min(t.ntiles, persistent_ctas(k_interp_mma, 32, c.device)), 32, 0, s>>>(
-            t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles);
-        FCM_LAUNCH_CHECK();
-        k_interp_reduce8<T><<<(t.n + 15) / 16, 128, 0, s>>>(t.base, t.partial, t.n, g, dx3, dV);
-        FCM_LAUNCH_CHECK();
-        return FCM_OK;
-      }
-    }
-    if (v == 2)
-      k_interp_rows<T, 2><<<t.ntiles, 32, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
-    else if (sizeof(T) == 4 && v == 1)
-      k_interp_warp<T><<<t.ntiles, 32, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
-    else
-      k_interp_tiled<T><<<t.ntiles, 64, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
-    FCM_LAUNCH_CHECK();
+    TileGeom g;
+    FCM_TRY(launch_interp_tiles<T>(c, t, grid, g, s));
     k_interp_reduce8<T><<<(t.n + 15) / 16, 128, 0, s>>>(t.base, t.partial, t.n, g, dx3, dV);
     FCM_LAUNCH_CHECK();
     return FCM_OK;
   }
+  const int ycut = c.p.slip_channel ? c.g.ny / 2 : c.g.ny;  // fcm_fluid_solver.cpp:387-389
   k_interp_block<T, 256><<<t.n, 256, 0, s>>>(t.base, t.w, grid, t.W, c.g.nx, c.g.ny, c.g.nz, c.g.G, dx3, dV, ycut);
+  FCM_LAUNCH_CHECK();
+  return FCM_OK;
+}
+
+template <typename T>
+int launch_saddle_end(const Ctx& c, const BlobTable<T>& t, const T* grid, const double* qm, const double* in,
+                      double* out, cudaStream_t s) {
+  if (t.n == 0 || !t.tiled) {
+    FCM_TRY(launch_interp<T>(c, t, grid, out, s));
+    FCM_TRY(launch_multiply_K(c, qm, in + 3 * (size_t)c.Nb, out, 1.0, s));
+    return launch_multiply_KT(c, qm, in, out + 3 * (size_t)c.Nb, -1.0, nullptr, 0.0, s);
+  }
+  TileGeom g;
+  FCM_TRY(launch_interp_tiles<T>(c, t, grid, g, s));
+  const int rblocks = (t.n + 15) / 16;
+  k_saddle_end<T><<<rblocks + (c.M + 127) / 128, 128, 0, s>>>(t.base, t.partial, t.n, g, c.g.dx * c.g.dx * c.g.dx,
+                                                              rblocks, qm, c.d_ref, c.ref_stride, in, out, c.M, c.nb);
   FCM_LAUNCH_CHECK();
   return FCM_OK;
 }
@@ -2159,6 +2220,10 @@ template int launch_set_up_gaussians<double>(const Ctx&, BlobTable<double>&, con
 template int launch_set_up_gaussians<float>(const Ctx&, BlobTable<float>&, const double*, cudaStream_t);
 template int launch_spread<double>(const Ctx&, const BlobTable<double>&, const double*, double*, cudaStream_t);
 template int launch_spread<float>(const Ctx&, const BlobTable<float>&, const double*, float*, cudaStream_t);
+template int launch_saddle_end<double>(const Ctx&, const BlobTable<double>&, const double*, const double*,
+                                       const double*, double*, cudaStream_t);
+template int launch_saddle_end<float>(const Ctx&, const BlobTable<float>&, const float*, const double*,
+                                      const double*, double*, cudaStream_t);
 template int launch_interp<double>(const Ctx&, const BlobTable<double>&, const double*, double*, cudaStream_t);
 template int launch_interp<float>(const Ctx&, const BlobTable<float>&, const float*, double*, cudaStream_t);
 

@@ -521,6 +521,11 @@ template <typename T>
 int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid, cudaStream_t s);
 template <typename T>
 int launch_interp(const Ctx& c, const BlobTable<T>& t, const T* grid, double* dV, cudaStream_t s);
+// out = [J u - K U; -K^T lambda] for in = [lambda; U] and the velocity grid u = L^-1 J^T
+// lambda: the interpolation and the rigid-body part of the saddle-point product
+template <typename T>
+int launch_saddle_end(const Ctx& c, const BlobTable<T>& t, const T* grid, const double* qm, const double* in,
+                      double* out, cudaStream_t s);
 // force dipoles (fcm_grid.cu): D (9 per blob) added to the force grid; moments
 // of the velocity grid into Omega (3 per blob) and E (9 per blob)
 // slip channel: the image of the lower half over the upper half of a force grid
@@ -574,6 +579,7 @@ int launch_fill_blob_pos(const Ctx& c, const double* x, const double* q, double*
 int launch_multiply_K(const Ctx& c, const double* qm, const double* in6, double* out3, double scale_acc, cudaStream_t s);
 int launch_multiply_KT(const Ctx& c, const double* qm, const double* in3, double* out6, double scale, const double* add6, double add_scale, cudaStream_t s);
 int launch_pinv(const Ctx& c, const double* qm, const double* in, double* out, cudaStream_t s);
+int launch_pinv_column(const Ctx& c, const double* qm, double* out, cudaStream_t s);  // of the newest Krylov column
 int launch_rigid_projection(const Ctx& c, const double* q, const double* V, double* U6, cudaStream_t s);
 // U scaled by `scale`, times *d_nu when d_nu is given.
 int launch_body_update(const Ctx& c, double* x, double* q, const double* U6, double scale, cudaStream_t s,
@@ -608,8 +614,13 @@ int blas_sum_accumulate(const Ctx& c, const double* a, long long n, double* d_ou
 // device-side GMRES pieces (fcm_blas.cu)
 // tol is read from *d_tol instead when d_tol is given.
 int gm_init(const Ctx& c, const double* b, double tol, int maxit, cudaStream_t s, const double* d_tol = nullptr);
-int gm_fetch(const Ctx& c, double* dst, cudaStream_t s);
 int gm_orthogonalize(const Ctx& c, double* w, cudaStream_t s);
+// Whether a context's orthogonalisation is one launch (gm_arnoldi, small systems), which
+// also sets a loop condition when sd is given: go on while not done and fewer than limit
+// iterations (sd->guard) have run.
+bool gm_one_launch(const Ctx& c);
+int gm_arnoldi(const Ctx& c, const double* w, cudaStream_t s, cudaGraphConditionalHandle handle, StepRecord* sd,
+               int limit);
 int gm_finish(const Ctx& c, double* soln_pre, cudaStream_t s);
 
 // symmetric inverse: inv() when well conditioned, otherwise the pseudo-inverse
