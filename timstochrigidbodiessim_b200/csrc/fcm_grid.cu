@@ -1646,24 +1646,28 @@ __global__ void __launch_bounds__(32) k_spread_mma64(const double* __restrict__ 
 // of four (y, z) with the tile's velocities as B fragments in registers (48 doubles per
 // lane), for two groups of eight blobs; then partial_kc = sum over x of P_c[k, x] wx_k[x].
 // Persistent and pipelined as the spread; the next tile's grid is copied to shared
-// memory while this tile's rounds run.  48 MMAs and 16 products per eight blobs; the 252
-// registers (the grid in fragments) leave eight warps per SM, and half the cycles have no
-// MMA in flight (350 us at 256^3 with 57.7 blobs per tile, 138 us with 2048 rods; the
-// shuffle-reduced warp kernel took 499 and 178 us).  A warp per component (a third of the
+// memory while this tile's rounds run.  48 MMAs and 16 products per eight blobs: 346 us at
+// 256^3 with 57.7 blobs per tile, 124 us with 2048 rods (the shuffle-reduced warp kernel
+// took 499 and 178 us).  Without the MMAs the rest takes 142 us there and the two add up,
+// whether eight or eleven warps per SM are resident. A warp per component (a third of the
 // registers, but the operand products and the round's overhead three times) took 403 us,
-// register caps for ten or eleven warps per SM 385 us and more (spills).
+// contiguous ranges of tiles with equal shares of the list entries 360 us.
 constexpr int SGX64 = TE * TE + 4;  // padded x-plane: the fragment reads fall in different banks
 
 __device__ __forceinline__ void grid_tile_async64(const double* __restrict__ grid, const TileGeom& g, long long G,
                                                   int tile, double* sg) {
   const int tz = tile % g.ntz, ty = (tile / g.ntz) % g.nty, tx = tile / (g.ntz * g.nty);
+  const int y = threadIdx.x >> 2, part = threadIdx.x & 3;  // row y of every (component, x), a quarter of its 64 bytes
+  const long long i0 = ((long long)(tx * TE) * g.ny + ty * TE + y) * g.nz + tz * TE + 2 * part;
+  const long long xs = (long long)g.ny * g.nz;
+  double* d0 = sg + y * TE + 2 * part;
 #pragma unroll
-  for (int q = 0; q < 24; ++q) {  // 3 x 8 x 8 rows of four 16-byte parts
-    const int i = threadIdx.x + 32 * q, row = i >> 2, part = i & 3;
-    const int c = row >> 6, x = (row >> 3) & 7, y = row & 7;
-    const long long idx = ((long long)(tx * TE + x) * g.ny + ty * TE + y) * g.nz + tz * TE + 2 * part;
-    cp_async16_or_zero(sg + (c * TE + x) * SGX64 + y * TE + 2 * part, grid + c * G + idx, FCM_INB(idx + 1, G, BS_GRID));
-  }
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int x = 0; x < TE; ++x) {
+      const long long idx = i0 + x * xs;
+      cp_async16_or_zero(d0 + (c * TE + x) * SGX64, grid + c * G + idx, FCM_INB(idx + 1, G, BS_GRID));
+    }
 }
 
 __global__ void __launch_bounds__(32) k_interp_mma64(const double* __restrict__ wc, const double* __restrict__ grid,
@@ -1707,13 +1711,13 @@ __global__ void __launch_bounds__(32) k_interp_mma64(const double* __restrict__ 
     if (first) {
       const int ty = (cur.tile / g.ntz) % g.nty;
 #pragma unroll
-      for (int j = 0; j < 2 * TE; ++j) {
-        const bool live = ty * TE + (j >> 1) < g.ycut;  // rows at or above the slip channel's upper wall read as 0
+      for (int j = 0; j < 2 * TE; ++j)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const double v = sg[(c * TE + gq) * SGX64 + 4 * j + tq];
-          u[j][c] = live ? v : 0.0;
-        }
+        for (int c = 0; c < 3; ++c) u[j][c] = sg[(c * TE + gq) * SGX64 + 4 * j + tq];
+      if (ty * TE + TE > g.ycut) {  // rows at or above the slip channel's upper wall read as 0
+#pragma unroll
+        for (int j = 0; j < 2 * TE; ++j)
+          if (ty * TE + (j >> 1) >= g.ycut) u[j][0] = u[j][1] = u[j][2] = 0.0;
       }
       __syncwarp();  // every lane has its fragments: the buffer takes the next tile
       const int nt = cur.tile + (int)gridDim.x;
