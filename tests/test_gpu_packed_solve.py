@@ -47,3 +47,20 @@ def test_velocity_field(gpu, n):
     g.stokes_solve(1)
     assert rel_err(g.interp(1), Vo) < 1e-6
 
+
+
+@pytest.mark.parametrize("slip", [0, 1])
+@pytest.mark.parametrize("n", [(8, 8, 8), (16, 24, 12), (24, 16, 16), (64, 48, 32), (256, 8, 16), (384, 12, 8)])
+def test_fluctuating_field(gpu, n, slip):
+    """The FP64 fluctuating field, drawn inside the x pass of the packed spectrum, against
+    the same draws in the whole half spectrum with cuFFT's 3D transform, which the FP32
+    field of a mixed-precision context takes: norm-wise 2e-6 (FP32 amplitudes and
+    transform), with the slip channel's image-symmetric stress and without."""
+    nb = 2
+    fields = []
+    for prec in (0, 1):
+        g = Suspension(_params(n, nb, slip_channel=slip).copy(precision=prec), [0, 0, 0])
+        g.produce_random_velocity_field(11, 7)
+        fields.append([np.asarray(u).reshape(n[0], n[1], -1)[:, :, :n[2]] for u in g.get_velocity_field(1)])
+    for a, b in zip(*fields):
+        assert np.any(a) and rel_err(b, a) < 2e-6

@@ -485,6 +485,7 @@ struct BatchGeom {
 };
 
 KParams make_kparams(const Ctx& c);
+void stress_amplitudes(const Ctx& c, double& diag, double& off);  // standard deviations of a stress mode's parts
 // Tile geometry of a grid for tables of nblobs blobs with a tile list of
 // list_cap entries.
 TileGeom tile_geom(const GridDims& g, int W, int nblobs, long long list_cap);
@@ -559,6 +560,8 @@ template <typename T>
 int launch_packed_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s);
 template <typename T>
 int launch_packed_inverse(const Ctx& c, typename cplx_t<T>::type* spec, T* r, int members, cudaStream_t s);
+int launch_packed_noise(const Ctx& c, cufftDoubleComplex* spec, double* r, uint64_t seed, uint64_t counter,
+                        const uint64_t* d_args, cudaStream_t s);
 template <typename T>
 int b_packed_project(const BatchGeom& b, const Ctx& c0, const int* gidx, int nm, int mask, cudaStream_t s);
 // the same for the members gidx[0..nm) of a batch group whose grids equal c0's

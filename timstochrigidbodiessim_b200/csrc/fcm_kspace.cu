@@ -21,31 +21,12 @@
 #include <type_traits>
 
 #include "fcm_dft.cuh"
+#include "fcm_fluct.cuh"
 #include "fcm_internal.cuh"
 
 namespace fcm {
 
 namespace {
-
-// Projection of one complex mode (re and im share the real factors).  The
-// reference divides every component by eta*G; here one reciprocal of the
-// mode's |q|^2 and a precomputed 1/(eta*G) are used instead (a last-bit change).
-template <typename T>
-__device__ __forceinline__ void project_mode(double q1, double q2, double q3, const V2<T> f[3], V2<T> u[3],
-                                             T inv_etaG) {
-  const T t1 = (T)q1, t2 = (T)q2, t3 = (T)q3;
-  const T qq = (T)(q2 * q2) + (T)(q1 * q1) + (T)1e-16;
-  const T norm = (T)1 / (qq + (T)(q3 * q3));
-  const T kr = (t1 * f[0].x + t2 * f[1].x + t3 * f[2].x) * norm;
-  const T ki = (t1 * f[0].y + t2 * f[1].y + t3 * f[2].y) * norm;
-  const T sc = norm * inv_etaG;
-  const T qv[3] = {t1, t2, t3};
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    u[c].x = sc * (f[c].x - qv[c] * kr);
-    u[c].y = sc * (f[c].y - qv[c] * ki);
-  }
-}
 
 __device__ __forceinline__ void mode_coords(long long t, const KParams& k, int& x, int& y, int& kz) {
   kz = (int)(t % k.nzh);
@@ -141,51 +122,6 @@ __global__ void __launch_bounds__(256, 4) k_b_project(const BMember* __restrict_
   const BMember& m = mem[mb.x];
   if (bskip(m, mask) || m.xfft[P]) return;  // that precision's fused x-transform projects it
   project_one<T, C>((C*)m.spec[P], m.kp, (long long)mb.y * 256 + threadIdx.x);
-}
-
-// f = i (q~ . sigma) for one mode; sigma order xx, yy, zz, xy, xz, yz.
-template <typename T>
-__device__ __forceinline__ void stress_divergence(double q1, double q2, double q3, const V2<T> s[6], V2<T> f[3]) {
-  const T a = (T)q1, b = (T)q2, c = (T)q3;
-  // (q.sigma)_x = q1 sxx + q2 sxy + q3 sxz, etc.; i*(r + i m) = -m + i r
-  const T rx = a * s[0].x + b * s[3].x + c * s[4].x, mx = a * s[0].y + b * s[3].y + c * s[4].y;
-  const T ry = a * s[3].x + b * s[1].x + c * s[5].x, my = a * s[3].y + b * s[1].y + c * s[5].y;
-  const T rz = a * s[4].x + b * s[5].x + c * s[2].x, mz = a * s[4].y + b * s[5].y + c * s[2].y;
-  f[0].x = -mx; f[0].y = rx;
-  f[1].x = -my; f[1].y = ry;
-  f[2].x = -mz; f[2].y = rz;
-}
-
-// Nyquist-zeroed wavenumbers of the stress divergence (fcm_fluid_solver.cpp:245-278).
-__device__ __forceinline__ void divergence_q(int x, int y, int kz, const KParams& k, double& q1, double& q2,
-                                             double& q3) {
-  q1 = (x == k.nx / 2) ? 0.0 : wavenumber(x, k.nx, k.fx);
-  q2 = (y == k.ny / 2) ? 0.0 : wavenumber(y, k.ny, k.fy);
-  q3 = (kz == k.nzh - 1) ? 0.0 : (double)kz * k.fz;
-}
-
-// Two standard normals from two 32-bit words (Box-Muller, single precision).
-__device__ __forceinline__ void box_muller(unsigned int a, unsigned int b, float& n1, float& n2) {
-  const float u1 = ((float)a + 0.5f) * 2.3283064365386963e-10f;
-  const float u2 = ((float)b + 0.5f) * 2.3283064365386963e-10f;
-  const float r = sqrtf(-2.0f * logf(u1));
-  float sn, cs;
-  sincospif(2.0f * u2, &sn, &cs);
-  n1 = r * cs;
-  n2 = r * sn;
-}
-
-// Twelve normals for mode index m: three Philox blocks with counter
-// (m, block, counter_lo, counter_hi), key (seed_lo, seed_hi).
-__device__ __forceinline__ void mode_normals(unsigned long long m, uint64_t seed, uint64_t counter, float nrm[12]) {
-  const uint2 key = make_uint2((unsigned int)seed, (unsigned int)(seed >> 32));
-#pragma unroll
-  for (int blk = 0; blk < 3; ++blk) {
-    const uint4 r = philox4x32_10(make_uint4((unsigned int)m, (unsigned int)blk, (unsigned int)counter,
-                                             (unsigned int)(counter >> 32)), key);
-    box_muller(r.x, r.y, nrm[4 * blk], nrm[4 * blk + 1]);
-    box_muller(r.z, r.w, nrm[4 * blk + 2], nrm[4 * blk + 3]);
-  }
 }
 
 // Fluctuating velocity spectrum.  Source 0: six stress spectra (R2C of the
@@ -829,7 +765,7 @@ int launch_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s)
 
 // Standard deviations of the stress (fcm_fluid_solver.cpp:169-170):
 // var1 = sqrt(2 kT eta / (DX^3 dt)) off-diagonal, var2 = sqrt(2) var1 diagonal.
-static void stress_amplitudes(const Ctx& c, double& diag, double& off) {
+void stress_amplitudes(const Ctx& c, double& diag, double& off) {
   const double dx = c.g.dx;
   const double var1 = sqrt(2.0 * c.p.kT * c.p.viscosity / (dx * dx * dx * c.p.dt));
   const double var2 = sqrt(2.0) * var1;

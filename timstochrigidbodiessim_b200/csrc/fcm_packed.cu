@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "fcm_dft.cuh"
+#include "fcm_fluct.cuh"
 #include "fcm_internal.cuh"
 
 namespace fcm {
@@ -411,6 +412,19 @@ struct XShape {
   __device__ static __forceinline__ int at(int k1, int k2) { return k1 * ROW + k2 * C3; }
 };
 
+// The packed modes a at kx and b (conjugated) at -kx of the pair u, v (the inverse of the
+// separation below, doubled as the real transform of 2 H points wants).
+template <typename T>
+__device__ __forceinline__ void fold_pair(V2<T> (&a)[3], V2<T> (&b)[3], const V2<T> (&u)[3], const V2<T> (&v)[3],
+                                          V2<T> p) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const V2<T> e = cadd(u[c], v[c]), d = cmulc(csub(u[c], v[c]), p);
+    a[c] = cadd(e, d);
+    b[c] = csub(e, d);
+  }
+}
+
 // The projection of one pair: a, b the packed modes (b conjugated) of A at kx and B at
 // -kx; p = -i W_nz^kz.  f = X(kx, yA, kz), g = conj X(-kx, yB, H - kz), both doubled (ie
 // carries the 1/2 of the separation).
@@ -438,20 +452,22 @@ __device__ __forceinline__ void project_pair(V2<T> (&a)[3], V2<T> (&b)[3], V2<T>
       if (zero) u[c] = V2<T>{(T)0, (T)0};
     }
   }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const V2<T> e = cadd(u[c], v[c]), d = cmulc(csub(u[c], v[c]), p);
-    a[c] = cadd(e, d);
-    b[c] = csub(e, d);
-  }
+  fold_pair<T>(a, b, u, v, p);
 }
 
 // The x transforms of TK column pairs of one slot, the projection between.  Five steps:
 // N1-point DFTs from global memory, N2-point DFTs in place, the pairs, inverse N2-point
 // DFTs in place, inverse N1-point DFTs to global memory.
-template <typename T, typename C, int N1, int N2, int TK, int NT>
+// NOISE: the pairs are the velocities of the fluctuating stress instead (drawn here, so the
+// spectrum is written once), and only the inverse steps run.
+struct NoiseArgs {
+  uint64_t seed, counter;
+  const uint64_t* dargs;  // (seed, counter) in device memory, if given
+  double amp_diag, amp_off;
+};
+template <typename T, typename C, int N1, int N2, int TK, int NT, bool NOISE>
 __device__ __forceinline__ void packed_x_cta(C* __restrict__ spec, const KParams& k, const C* __restrict__ twx,
-                                             const C* __restrict__ twz) {
+                                             const C* __restrict__ twz, const NoiseArgs& na) {
   using S = XShape<C, N1, N2, TK>;
   constexpr int N = S::N, C3 = S::C3;
   extern __shared__ __align__(16) unsigned char packed_smem[];
@@ -476,37 +492,41 @@ __device__ __forceinline__ void packed_x_cta(C* __restrict__ spec, const KParams
     const int x = q * N2 + n2;
     return (x / XB) * xs + (x % XB) * t.TKB;
   };
-  // items (pair j, n2, component, side): consecutive lanes the columns of a tile, then x
-  for (int i = threadIdx.x; i < 2 * N2 * C3; i += NT) {
-    const int j = i % TK, n2 = (i / TK) % N2, c = (i / (TK * N2)) % 3, side = i / (TK * N2 * 3);
-    if (j0 + j >= PC) continue;
-    const long long e = pencil(side, c, j);
-    V2<T> a[N1];
+  if constexpr (!NOISE) {
+    // items (pair j, n2, component, side): consecutive lanes the columns of a tile, then x
+    for (int i = threadIdx.x; i < 2 * N2 * C3; i += NT) {
+      const int j = i % TK, n2 = (i / TK) % N2, c = (i / (TK * N2)) % 3, side = i / (TK * N2 * 3);
+      if (j0 + j >= PC) continue;
+      const long long e = pencil(side, c, j);
+      V2<T> a[N1];
 #pragma unroll
-    for (int q = 0; q < N1; ++q) {
-      const long long at = e + x_at(q, n2);
-      a[q] = FCM_INB(at, t.size(), BS_SPECTRUM) ? ldt<T>(spec[at]) : V2<T>{(T)0, (T)0};
+      for (int q = 0; q < N1; ++q) {
+        const long long at = e + x_at(q, n2);
+        a[q] = FCM_INB(at, t.size(), BS_SPECTRUM) ? ldt<T>(spec[at]) : V2<T>{(T)0, (T)0};
+      }
+      dft<T, N1, false>(a);
+#pragma unroll
+      for (int q = 1; q < N1; ++q) a[q] = cmul(a[q], ldt<T>(__ldg(&twx[n2 * q])));
+#pragma unroll
+      for (int q = 0; q < N1; ++q) s[side * S::SIDE + S::at(q, n2) + 3 * j + c] = a[q];
     }
-    dft<T, N1, false>(a);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * N1 * C3; i += NT) {
+      const int col = i % C3, k1 = (i / C3) % N1, side = i / (C3 * N1);
+      if (j0 + col / 3 >= PC) continue;
+      V2<T>* row = s + side * S::SIDE + S::at(k1, 0) + col;
+      V2<T> b[N2];
 #pragma unroll
-    for (int q = 1; q < N1; ++q) a[q] = cmul(a[q], ldt<T>(__ldg(&twx[n2 * q])));
+      for (int j = 0; j < N2; ++j) b[j] = row[j * C3];
+      dft<T, N2, false>(b);
 #pragma unroll
-    for (int q = 0; q < N1; ++q) s[side * S::SIDE + S::at(q, n2) + 3 * j + c] = a[q];
+      for (int j = 0; j < N2; ++j) row[j * C3] = b[j];
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 2 * N1 * C3; i += NT) {
-    const int col = i % C3, k1 = (i / C3) % N1, side = i / (C3 * N1);
-    if (j0 + col / 3 >= PC) continue;
-    V2<T>* row = s + side * S::SIDE + S::at(k1, 0) + col;
-    V2<T> b[N2];
-#pragma unroll
-    for (int j = 0; j < N2; ++j) b[j] = row[j * C3];
-    dft<T, N2, false>(b);
-#pragma unroll
-    for (int j = 0; j < N2; ++j) row[j * C3] = b[j];
-  }
-  __syncthreads();
   static_assert(NT % TK == 0, "a thread keeps its column pair");
+  const uint64_t seed = NOISE && na.dargs ? na.dargs[0] : na.seed;
+  const uint64_t counter = NOISE && na.dargs ? na.dargs[1] : na.counter;
   const T ie = (T)(0.5 * k.inv_etaG);
   const int pj = threadIdx.x % TK;
   const PairSlot p = pair_slot(y0, j0 + pj, k.ny, H);
@@ -526,12 +546,21 @@ __device__ __forceinline__ void packed_x_cta(C* __restrict__ spec, const KParams
       V2<T>* sa = s + r * S::SIDE + S::at(k1, k2) + 3 * pj;
       V2<T>* sb = s + (p.self ? r : 1) * S::SIDE + S::at(m1, m2) + 3 * pj;
       V2<T> a[3], b[3];
+      if constexpr (NOISE) {
+        V2<T> u[3], v[3];
+        fluct_velocity<T>(kx, yA, p.kz, k, seed, counter, na.amp_diag, na.amp_off, u);
+        fluct_velocity<T>(kxp, p.self ? yA : p.yB, H - p.kz, k, seed, counter, na.amp_diag, na.amp_off, v);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        a[c] = sa[c];
-        b[c] = V2<T>{sb[c].x, -sb[c].y};
+        for (int c = 0; c < 3; ++c) v[c].y = -v[c].y;
+        fold_pair<T>(a, b, u, v, pw);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          a[c] = sa[c];
+          b[c] = V2<T>{sb[c].x, -sb[c].y};
+        }
+        project_pair<T>(a, b, pw, wx[kx], wx[kxp], y, yp, z, zp, p.plane, kx == 0 && yA == 0, ie);
       }
-      project_pair<T>(a, b, pw, wx[kx], wx[kxp], y, yp, z, zp, p.plane, kx == 0 && yA == 0, ie);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         sa[c] = a[c];
@@ -576,7 +605,14 @@ __device__ __forceinline__ void packed_x_cta(C* __restrict__ spec, const KParams
 template <typename T, typename C, int N1, int N2, int TK, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_packed_x(C* __restrict__ spec, KParams k, const C* __restrict__ twx,
                                                        const C* __restrict__ twz) {
-  packed_x_cta<T, C, N1, N2, TK, NT>(spec, k, twx, twz);
+  packed_x_cta<T, C, N1, N2, TK, NT, false>(spec, k, twx, twz, NoiseArgs{});
+}
+
+// The spectrum of a fluctuating velocity field, transformed along x.
+template <typename T, typename C, int N1, int N2, int TK, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_packed_noise(C* __restrict__ spec, KParams k, const C* __restrict__ twx,
+                                                           const C* __restrict__ twz, NoiseArgs na) {
+  packed_x_cta<T, C, N1, N2, TK, NT, true>(spec, k, twx, twz, na);
 }
 
 // Batched: blockIdx.z = member gidx[blockIdx.z] of a group of equal grids.
@@ -586,7 +622,7 @@ __global__ void __launch_bounds__(NT, MINB) k_b_packed_x(const BMember* __restri
                                                          const C* __restrict__ twz) {
   const BMember& m = mem[gidx[blockIdx.z]];
   if (bskip(m, mask)) return;
-  packed_x_cta<T, C, N1, N2, TK, NT>((C*)m.spec[P], m.kp, twx, twz);
+  packed_x_cta<T, C, N1, N2, TK, NT, false>((C*)m.spec[P], m.kp, twx, twz, NoiseArgs{});
 }
 
 // ------------------------------------------------------------------ launches
@@ -805,6 +841,27 @@ long long packed_spectrum_size(const Ctx& c) {
 template <typename T>
 int launch_packed_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s) {
   return packed_x<T>(c, spec, s, nullptr, nullptr, 0, 0);
+}
+
+// The fluctuating velocity field of (seed, counter), or d_args[0..1] where given, into r.
+int launch_packed_noise(const Ctx& c, cufftDoubleComplex* spec, double* r, uint64_t seed, uint64_t counter,
+                        const uint64_t* d_args, cudaStream_t s) {
+  using T = double;
+  using C = cufftDoubleComplex;
+  NoiseArgs na{seed, counter, d_args, 0.0, 0.0};
+  stress_amplitudes(c, na.amp_diag, na.amp_off);
+  FCM_TRY(with_factors(c.g.nx, [&](auto a, auto d) -> int {
+    constexpr int N1 = decltype(a)::value, N2 = decltype(d)::value, N = N1 * N2;
+    constexpr int TK = px_tk<T, N>(), NT = px_threads<T, N>(), MB = px_min<T, N>();
+    constexpr size_t smem = XShape<C, N1, N2, TK>::SMEM;
+    const dim3 grid((unsigned)((c.g.nz / 4 + TK - 1) / TK), (unsigned)c.g.ny);
+    auto kern = k_packed_noise<T, C, N1, N2, TK, NT, MB>;
+    FCM_TRY(smem_attr_once(kern, smem));
+    kern<<<grid, NT, smem, s>>>(spec, make_kparams(c), xtw<T>(c), ztw<T>(c), na);
+    FCM_LAUNCH_CHECK();
+    return FCM_OK;
+  }));
+  return launch_packed_inverse<T>(c, spec, r, 1, s);
 }
 
 template <typename T>
