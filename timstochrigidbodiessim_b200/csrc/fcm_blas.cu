@@ -59,6 +59,7 @@ __device__ __forceinline__ void finish(double my_partial, double* partials, unsi
 // *out (op)= sum a[i]*b[i]  (b == nullptr: sum a[i])
 __global__ void __launch_bounds__(RT) k_dot(const double* __restrict__ a, const double* __restrict__ b, long long n,
                                             double* partials, unsigned int* counter, double* out, int mode) {
+  chain_begin();
   __shared__ double sh[RT / 32];
   double s = 0.0;
   for (long long i = blockIdx.x * (long long)RT + threadIdx.x; i < n; i += (long long)gridDim.x * RT)
@@ -72,6 +73,7 @@ __global__ void __launch_bounds__(RT) k_dot(const double* __restrict__ a, const 
 __global__ void __launch_bounds__(RT) k_mgs(double* __restrict__ w, const double* __restrict__ q_prev,
                                             const double* __restrict__ h_prev, const double* __restrict__ q_i,
                                             long long n, double* partials, unsigned int* counter, double* hout) {
+  chain_begin();
   __shared__ double sh[RT / 32];
   const double h = q_prev ? *h_prev : 0.0;
   double s = 0.0;
@@ -100,6 +102,7 @@ __global__ void k_scale(double* __restrict__ v, const double* __restrict__ num, 
 
 __global__ void k_copy_scaled(double* __restrict__ dst, const double* __restrict__ src, const double* __restrict__ num,
                               int invert, long long n) {
+  chain_begin();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double s = *num;
@@ -107,6 +110,7 @@ __global__ void k_copy_scaled(double* __restrict__ dst, const double* __restrict
 }
 
 __global__ void k_axpby(double* __restrict__ y, const double* __restrict__ x, double a, double b, long long n) {
+  chain_begin();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   y[i] = a * x[i] + b * y[i];
@@ -132,29 +136,27 @@ inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 }  // namespace
 
 int blas_dot(const Ctx& c, const double* a, const double* b, long long n, double* d_out, cudaStream_t s) {
-  k_dot<<<c.red_blocks, RT, 0, s>>>(a, b, n, c.d_partials, c.d_counter, d_out, 0);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_dot, dim3(c.red_blocks), dim3(RT), 0, s, a, b, n, c.d_partials, c.d_counter, d_out, 0));
   return FCM_OK;
 }
 
 // sum of a[] accumulated into *d_out (b == nullptr, mode 1)
 int blas_sum_accumulate(const Ctx& c, const double* a, long long n, double* d_out, cudaStream_t s) {
-  k_dot<<<c.red_blocks, RT, 0, s>>>(a, nullptr, n, c.d_partials, c.d_counter, d_out, 1);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_dot, dim3(c.red_blocks), dim3(RT), 0, s, a, nullptr, n, c.d_partials, c.d_counter, d_out,
+                         1));
   return FCM_OK;
 }
 
 int blas_norm_sq_partial(const Ctx& c, const double* a, long long n, double* d_out, cudaStream_t s) {
-  k_mgs<<<c.red_blocks, RT, 0, s>>>(const_cast<double*>(a), nullptr, nullptr, nullptr, n, c.d_partials, c.d_counter,
-                                    d_out);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_mgs, dim3(c.red_blocks), dim3(RT), 0, s, const_cast<double*>(a), nullptr, nullptr, nullptr,
+                         n, c.d_partials, c.d_counter, d_out));
   return FCM_OK;
 }
 
 int blas_mgs_step(const Ctx& c, double* w, const double* q_prev, const double* h_prev, const double* q_i, long long n,
                   double* d_hout, cudaStream_t s) {
-  k_mgs<<<c.red_blocks, RT, 0, s>>>(w, q_prev, h_prev, q_i, n, c.d_partials, c.d_counter, d_hout);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_mgs, dim3(c.red_blocks), dim3(RT), 0, s, w, q_prev, h_prev, q_i, n, c.d_partials,
+                         c.d_counter, d_hout));
   return FCM_OK;
 }
 
@@ -165,14 +167,12 @@ int blas_scale(double* v, const double* d_num, int invert, long long n, cudaStre
 }
 
 int blas_copy_scaled(double* dst, const double* src, const double* d_num, int invert, long long n, cudaStream_t s) {
-  k_copy_scaled<<<nblk(n, 256), 256, 0, s>>>(dst, src, d_num, invert, n);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_copy_scaled, dim3(nblk(n, 256)), dim3(256), 0, s, dst, src, d_num, invert, n));
   return FCM_OK;
 }
 
 int blas_axpby(double* y, const double* x, double a, double b, long long n, cudaStream_t s) {
-  k_axpby<<<nblk(n, 256), 256, 0, s>>>(y, x, a, b, n);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_axpby, dim3(nblk(n, 256)), dim3(256), 0, s, y, x, a, b, n));
   return FCM_OK;
 }
 
@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(MDT) k_multidot(const GmState* __restrict__ st
                                                   const double* __restrict__ w, long long n,
                                                   double* __restrict__ partials, unsigned int* __restrict__ counters,
                                                   double* __restrict__ h) {
+  chain_begin();
   __shared__ double sh[MDT / 32];
   __shared__ bool last;
   const int col = blockIdx.y;
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(MDT) k_multidot(const GmState* __restrict__ st
 // w -= sum_{i<=k} h[i] Q[:, i]
 __global__ void k_gs_update(const GmState* __restrict__ st, const double* __restrict__ Q,
                             const double* __restrict__ h, long long n, double* __restrict__ w) {
+  chain_begin();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n || st->done) return;
   const int k = st->k;
@@ -254,6 +256,7 @@ __global__ void k_gs_update(const GmState* __restrict__ st, const double* __rest
 // Q[k+1] = w / |w| (|w| = 0: a happy breakdown, the column is left as w)
 __global__ void k_gm_normalize(const GmState* __restrict__ st, const double* __restrict__ w,
                                const double* __restrict__ hnorm, long long n, double* __restrict__ Q, int hn) {
+  chain_begin();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n || st->done) return;
   if (!FCM_INB(st->k + 1, hn, BS_KRYLOV)) return;
@@ -329,6 +332,7 @@ __device__ __forceinline__ void givens_step(GmState* st, double* __restrict__ H,
 __global__ void k_gm_givens(GmState* st, double* __restrict__ H, int hn, double* __restrict__ beta,
                             double* __restrict__ CS, double* __restrict__ SN, const double* __restrict__ hA,
                             const double* __restrict__ hB, const double* __restrict__ hnorm) {
+  chain_begin();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   givens_step(st, H, hn, beta, CS, SN, hA, hB, hnorm);
 }
@@ -354,6 +358,7 @@ __global__ void __cluster_dims__(AC, 1, 1) __launch_bounds__(AT)
     k_gm_arnoldi(GmState* st, double* __restrict__ Q, long long n, const double* __restrict__ w_in,
                  double* __restrict__ H, int hn, double* __restrict__ beta, double* __restrict__ CS,
                  double* __restrict__ SN, cudaGraphConditionalHandle handle, StepRecord* sd, int limit) {
+  chain_begin();
   namespace cg = cooperative_groups;
   extern __shared__ double gsm[];
   double* wsum = gsm;                     // [AW][hn]
@@ -478,6 +483,7 @@ __global__ void __cluster_dims__(AC, 1, 1) __launch_bounds__(AT)
 // beta[0] = |b|, k = 0 (one thread); |b| == 0 or non-finite ends the solve.
 __global__ void k_gm_init(GmState* st, const double* __restrict__ normb, double* __restrict__ beta, double tol,
                           const double* __restrict__ d_tol, int maxit) {
+  chain_begin();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const double nb = *normb;
   if (d_tol) tol = *d_tol;
@@ -512,6 +518,7 @@ __device__ __forceinline__ void backsub_step(const GmState* __restrict__ st, con
 
 __global__ void k_gm_backsub(const GmState* __restrict__ st, const double* __restrict__ H, int hn,
                              const double* __restrict__ beta, double* __restrict__ y) {
+  chain_begin();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   backsub_step(st, H, hn, beta, y);
 }
@@ -519,6 +526,7 @@ __global__ void k_gm_backsub(const GmState* __restrict__ st, const double* __res
 // soln = sum_{i<k} y_i Q[:, i] (gmres_solver.cpp:320-326), k from the state.
 __global__ void k_gm_combine(const GmState* __restrict__ st, const double* __restrict__ Q,
                              const double* __restrict__ y, long long n, double* __restrict__ out) {
+  chain_begin();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int k = st->k;
@@ -539,9 +547,8 @@ int gm_arnoldi(const Ctx& c, const double* w, cudaStream_t s, cudaGraphCondition
   const size_t smem = gm_cluster_smem(hn);
   if (smem > 40 * 1024)  // not a stream operation: allowed while capturing
     FCM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<AC, AT, smem, s>>>(c.gm, c.d_Qm, n, w, c.d_Hd, hn, c.d_beta, c.d_CS, c.d_SN, handle, sd, limit);
-  FCM_LAUNCH_CHECK();
-  return FCM_OK;
+  return launch_chained(kern, dim3(AC), dim3(AT), smem, s, c.gm, c.d_Qm, n, w, c.d_Hd, hn, c.d_beta, c.d_CS, c.d_SN,
+                        handle, sd, limit);
 }
 
 int gm_orthogonalize(const Ctx& c, double* w, cudaStream_t s) {
@@ -549,35 +556,30 @@ int gm_orthogonalize(const Ctx& c, double* w, cudaStream_t s) {
   const dim3 grid(c.md_blocks, c.maxit_alloc + 1);
   double* hab[2] = {c.d_hA, c.d_hB};
   for (int pass = 0; pass < 2; ++pass) {
-    k_multidot<<<grid, MDT, 0, s>>>(c.gm, c.d_Qm, w, n, c.d_mdpart, c.d_mdcount, hab[pass]);
-    FCM_LAUNCH_CHECK();
-    k_gs_update<<<nblk(n, 256), 256, 0, s>>>(c.gm, c.d_Qm, hab[pass], n, w);
-    FCM_LAUNCH_CHECK();
+    FCM_TRY(launch_chained(k_multidot, dim3(grid), dim3(MDT), 0, s, c.gm, c.d_Qm, w, n, c.d_mdpart, c.d_mdcount,
+                           hab[pass]));
+    FCM_TRY(launch_chained(k_gs_update, dim3(nblk(n, 256)), dim3(256), 0, s, c.gm, c.d_Qm, hab[pass], n, w));
   }
   FCM_TRY(blas_norm_sq_partial(c, w, n, c.d_hnorm, s));
-  k_gm_normalize<<<nblk(n, 256), 256, 0, s>>>(c.gm, w, c.d_hnorm, n, c.d_Qm, c.maxit_alloc + 1);
-  FCM_LAUNCH_CHECK();
-  k_gm_givens<<<1, 32, 0, s>>>(c.gm, c.d_Hd, c.maxit_alloc + 1, c.d_beta, c.d_CS, c.d_SN, c.d_hA, c.d_hB,
-                               c.d_hnorm);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_gm_normalize, dim3(nblk(n, 256)), dim3(256), 0, s, c.gm, w, c.d_hnorm, n, c.d_Qm,
+                         c.maxit_alloc + 1));
+  FCM_TRY(launch_chained(k_gm_givens, dim3(1), dim3(32), 0, s, c.gm, c.d_Hd, c.maxit_alloc + 1, c.d_beta, c.d_CS,
+                         c.d_SN, c.d_hA, c.d_hB, c.d_hnorm));
   return FCM_OK;
 }
 
 int gm_init(const Ctx& c, const double* b, double tol, int maxit, cudaStream_t s, const double* d_tol) {
   const long long n = c.nsys;
   FCM_TRY(blas_norm_sq_partial(c, b, n, c.d_hnorm, s));
-  k_gm_init<<<1, 32, 0, s>>>(c.gm, c.d_hnorm, c.d_beta, tol, d_tol, maxit);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_gm_init, dim3(1), dim3(32), 0, s, c.gm, c.d_hnorm, c.d_beta, tol, d_tol, maxit));
   FCM_TRY(blas_copy_scaled(c.d_Qm, b, c.d_hnorm, 1, n, s));
   return FCM_OK;
 }
 
 int gm_finish(const Ctx& c, double* soln_pre, cudaStream_t s) {
   const long long n = c.nsys;
-  k_gm_backsub<<<1, 32, 0, s>>>(c.gm, c.d_Hd, c.maxit_alloc + 1, c.d_beta, c.d_y);
-  FCM_LAUNCH_CHECK();
-  k_gm_combine<<<nblk(n, 256), 256, 0, s>>>(c.gm, c.d_Qm, c.d_y, n, soln_pre);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_gm_backsub, dim3(1), dim3(32), 0, s, c.gm, c.d_Hd, c.maxit_alloc + 1, c.d_beta, c.d_y));
+  FCM_TRY(launch_chained(k_gm_combine, dim3(nblk(n, 256)), dim3(256), 0, s, c.gm, c.d_Qm, c.d_y, n, soln_pre));
   return FCM_OK;
 }
 

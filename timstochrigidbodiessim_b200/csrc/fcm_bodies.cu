@@ -16,6 +16,7 @@ namespace {
 __global__ void k_fill_blob_pos(const double* __restrict__ x, const double* __restrict__ q,
                                 const double* __restrict__ ref, int rs, int Nb, int nb, double Lx, double Ly,
                                 double Lz, double* __restrict__ Y) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Nb) return;
   const int n = i / nb, m = i - n * nb;
@@ -33,6 +34,7 @@ __global__ void k_fill_blob_pos(const double* __restrict__ x, const double* __re
 
 __global__ void k_multiply_K(const double* __restrict__ q, const double* __restrict__ ref, int rs,
                              const double* __restrict__ in, double* __restrict__ out, int Nb, int nb, int subtract) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Nb) return;
   multiply_K_one(q, ref, rs, in, out, i, nb, subtract);
@@ -41,6 +43,7 @@ __global__ void k_multiply_K(const double* __restrict__ q, const double* __restr
 __global__ void k_multiply_KT(const double* __restrict__ q, const double* __restrict__ ref, int rs,
                               const double* __restrict__ in, double* __restrict__ out, int M, int nb, double scale,
                               const double* __restrict__ add, double add_scale) {
+  chain_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= M) return;
   multiply_KT_one(q, ref, rs, in, out, n, nb, scale, add, add_scale);
@@ -135,6 +138,7 @@ __device__ __forceinline__ void pinv_block(const double* __restrict__ q, const d
 __global__ void k_pinv(const double* __restrict__ q, const double* __restrict__ ref, int rs,
                        const double* __restrict__ Minv, long long ms, const double* __restrict__ Nm, int ns,
                        const double* __restrict__ in, double* __restrict__ out, int M, int nb, int Nb) {
+  chain_begin();
   extern __shared__ double sm[];
   pinv_block(q, ref, rs, Minv, ms, Nm, ns, in, out, M, nb, Nb, sm);
 }
@@ -145,6 +149,7 @@ __global__ void k_pinv_column(const GmState* __restrict__ st, const double* __re
                               const double* __restrict__ q, const double* __restrict__ ref, int rs,
                               const double* __restrict__ Minv, long long ms, const double* __restrict__ Nm, int ns,
                               double* __restrict__ out, int M, int nb, int Nb) {
+  chain_begin();
   extern __shared__ double sm[];
   if (st->done) return;
   pinv_block(q, ref, rs, Minv, ms, Nm, ns, Q + (size_t)st->k * n, out, M, nb, Nb, sm);
@@ -156,6 +161,7 @@ __global__ void k_pinv_column(const GmState* __restrict__ st, const double* __re
 __global__ void k_rigid_projection(const double* __restrict__ q, const double* __restrict__ ref, int rs,
                                    const double* __restrict__ KTKinv, int ks, const double* __restrict__ V,
                                    double* __restrict__ U, int M, int nb) {
+  chain_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= M) return;
   ref += (size_t)n * rs;
@@ -214,6 +220,7 @@ __device__ void body_update_one(double* x, double* q, const double u[6], double 
 
 __global__ void k_body_update(double* __restrict__ x, double* __restrict__ q, const double* __restrict__ U, int M,
                               double scale, const double* __restrict__ d_nu, double Lx, double Ly, double Lz) {
+  chain_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= M) return;
   if (d_nu) scale = __dmul_rn(*d_nu, scale);  // nu * dt with nu from device memory
@@ -224,6 +231,7 @@ __global__ void k_body_update(double* __restrict__ x, double* __restrict__ q, co
 
 __global__ void k_body_update_uniform(double* __restrict__ x, double* __restrict__ q, int M, double e0, double e1,
                                       double e2, double e3, double e4, double e5, double Lx, double Ly, double Lz) {
+  chain_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= M) return;
   const double u[6] = {e0, e1, e2, e3, e4, e5};
@@ -263,6 +271,7 @@ __global__ void k_mcmc_restore(double* __restrict__ x, double* __restrict__ q, c
 // (collection_of_rigid_bodies.cpp:941-948).
 __global__ void k_divU_terms(const double* __restrict__ U, const double* __restrict__ U0, int M, int comp,
                              double delta, double* __restrict__ out) {
+  chain_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= M) return;
   out[n] = (U[6 * n + comp] - U0[6 * n + comp]) / delta;
@@ -272,24 +281,24 @@ __global__ void k_divU_terms(const double* __restrict__ U, const double* __restr
 
 int launch_fill_blob_pos(const Ctx& c, const double* x, const double* q, double* Y, cudaStream_t s) {
   if (c.Nb == 0) return FCM_OK;
-  k_fill_blob_pos<<<(c.Nb + 127) / 128, 128, 0, s>>>(x, q, c.d_ref, c.ref_stride, c.Nb, c.nb, c.g.Lx, c.g.Ly, c.g.Lz, Y);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_fill_blob_pos, dim3((c.Nb + 127) / 128), dim3(128), 0, s, x, q, c.d_ref, c.ref_stride, c.Nb,
+                         c.nb, c.g.Lx, c.g.Ly, c.g.Lz, Y));
   return FCM_OK;
 }
 
 int launch_multiply_K(const Ctx& c, const double* qm, const double* in6, double* out3, double subtract,
                       cudaStream_t s) {
   if (c.Nb == 0) return FCM_OK;
-  k_multiply_K<<<(c.Nb + 127) / 128, 128, 0, s>>>(qm, c.d_ref, c.ref_stride, in6, out3, c.Nb, c.nb, subtract != 0.0 ? 1 : 0);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_multiply_K, dim3((c.Nb + 127) / 128), dim3(128), 0, s, qm, c.d_ref, c.ref_stride, in6, out3,
+                         c.Nb, c.nb, subtract != 0.0 ? 1 : 0));
   return FCM_OK;
 }
 
 int launch_multiply_KT(const Ctx& c, const double* qm, const double* in3, double* out6, double scale,
                        const double* add6, double add_scale, cudaStream_t s) {
   if (c.M == 0) return FCM_OK;
-  k_multiply_KT<<<(c.M + 127) / 128, 128, 0, s>>>(qm, c.d_ref, c.ref_stride, in3, out6, c.M, c.nb, scale, add6, add_scale);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_multiply_KT, dim3((c.M + 127) / 128), dim3(128), 0, s, qm, c.d_ref, c.ref_stride, in3, out6,
+                         c.M, c.nb, scale, add6, add_scale));
   return FCM_OK;
 }
 
@@ -297,9 +306,8 @@ int launch_pinv(const Ctx& c, const double* qm, const double* in, double* out, c
   if (c.M == 0) return FCM_OK;
   const int warps = 4;
   const size_t shm = sizeof(double) * warps * (size_t)(6 * c.nb + 12);
-  k_pinv<<<(c.M + warps - 1) / warps, 32 * warps, shm, s>>>(qm, c.d_ref, c.ref_stride, c.d_Minv, c.minv_stride, c.d_N,
-                                                                 c.n_stride, in, out, c.M, c.nb, c.Nb);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_pinv, dim3((c.M + warps - 1) / warps), dim3(32 * warps), shm, s, qm, c.d_ref, c.ref_stride,
+                         c.d_Minv, c.minv_stride, c.d_N, c.n_stride, in, out, c.M, c.nb, c.Nb));
   return FCM_OK;
 }
 
@@ -307,26 +315,24 @@ int launch_pinv_column(const Ctx& c, const double* qm, double* out, cudaStream_t
   if (c.M == 0) return FCM_OK;
   const int warps = 4;
   const size_t shm = sizeof(double) * warps * (size_t)(6 * c.nb + 12);
-  k_pinv_column<<<(c.M + warps - 1) / warps, 32 * warps, shm, s>>>(c.gm, c.d_Qm, c.nsys, qm, c.d_ref, c.ref_stride,
-                                                                   c.d_Minv, c.minv_stride, c.d_N, c.n_stride, out,
-                                                                   c.M, c.nb, c.Nb);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_pinv_column, dim3((c.M + warps - 1) / warps), dim3(32 * warps), shm, s, c.gm, c.d_Qm,
+                         c.nsys, qm, c.d_ref, c.ref_stride, c.d_Minv, c.minv_stride, c.d_N, c.n_stride, out, c.M, c.nb,
+                         c.Nb));
   return FCM_OK;
 }
 
 int launch_rigid_projection(const Ctx& c, const double* q, const double* V, double* U6, cudaStream_t s) {
   if (c.M == 0) return FCM_OK;
-  k_rigid_projection<<<(c.M + 127) / 128, 128, 0, s>>>(q, c.d_ref, c.ref_stride, c.d_KTKinv, c.n_stride, V, U6,
-                                                       c.M, c.nb);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_rigid_projection, dim3((c.M + 127) / 128), dim3(128), 0, s, q, c.d_ref, c.ref_stride,
+                         c.d_KTKinv, c.n_stride, V, U6, c.M, c.nb));
   return FCM_OK;
 }
 
 int launch_body_update(const Ctx& c, double* x, double* q, const double* U6, double scale, cudaStream_t s,
                        const double* d_nu) {
   if (c.M == 0) return FCM_OK;
-  k_body_update<<<(c.M + 127) / 128, 128, 0, s>>>(x, q, U6, c.M, scale, d_nu, c.g.Lx, c.g.Ly, c.g.Lz);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_body_update, dim3((c.M + 127) / 128), dim3(128), 0, s, x, q, U6, c.M, scale, d_nu, c.g.Lx,
+                         c.g.Ly, c.g.Lz));
   return FCM_OK;
 }
 
@@ -346,17 +352,15 @@ int launch_mcmc_restore(const Ctx& c, const McmcDev* st, cudaStream_t s) {
 
 int launch_body_update_uniform(const Ctx& c, double* x, double* q, const double* e6, cudaStream_t s) {
   if (c.M == 0) return FCM_OK;
-  k_body_update_uniform<<<(c.M + 127) / 128, 128, 0, s>>>(x, q, c.M, e6[0], e6[1], e6[2], e6[3], e6[4], e6[5],
-                                                          c.g.Lx, c.g.Ly, c.g.Lz);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_body_update_uniform, dim3((c.M + 127) / 128), dim3(128), 0, s, x, q, c.M, e6[0], e6[1],
+                         e6[2], e6[3], e6[4], e6[5], c.g.Lx, c.g.Ly, c.g.Lz));
   return FCM_OK;
 }
 
 int launch_divU_accumulate(const Ctx& c, const double* U6, const double* U0, int component, double delta,
                            double* acc, cudaStream_t s) {
   if (c.M == 0) return FCM_OK;
-  k_divU_terms<<<(c.M + 127) / 128, 128, 0, s>>>(U6, U0, c.M, component, delta, acc);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_divU_terms, dim3((c.M + 127) / 128), dim3(128), 0, s, U6, U0, c.M, component, delta, acc));
   return FCM_OK;
 }
 

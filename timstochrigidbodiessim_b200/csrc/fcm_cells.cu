@@ -31,6 +31,7 @@ __device__ __forceinline__ int cell_coord(double y, double L, int N) {
 
 __global__ void k_cell_ids(const double* __restrict__ Y, int Nb, CellGeom g, int* __restrict__ cell,
                            int* __restrict__ count) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Nb) return;
   const int cx = cell_coord(Y[3 * i], g.Lx, g.N);
@@ -47,6 +48,7 @@ __global__ void k_cell_ids(const double* __restrict__ Y, int Nb, CellGeom g, int
 // consecutive ones, the thread totals scanned by warp shuffles and a second
 // warp level.
 __global__ void k_exclusive_scan(const int* __restrict__ in, int* __restrict__ out, int n) {
+  chain_begin();
   constexpr int IPT = 8;
   __shared__ int warp_sums[32];
   __shared__ int carry;
@@ -179,6 +181,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_chunks(const int* __restrict__ 
 // (most of it launches of one to four CTAs).
 constexpr int SCAN_DIRECT = 8 * SCAN_CH;
 __global__ void __launch_bounds__(SCAN_T) k_scan_direct(const int* __restrict__ in, int* __restrict__ out, int n) {
+  chain_begin();
   __shared__ int warp_sums[32];
   const int c0 = blockIdx.x * SCAN_CH;
   int before = 0;
@@ -204,6 +207,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_direct(const int* __restrict__ 
 
 __global__ void k_cell_scatter(const int* __restrict__ cell, int Nb, int ncell, const int* __restrict__ start,
                                int* __restrict__ cursor, int* __restrict__ sorted) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Nb) return;
   const int c = cell[i];
@@ -214,6 +218,7 @@ __global__ void k_cell_scatter(const int* __restrict__ cell, int Nb, int ncell, 
 
 // Ascending blob order within each cell, so every traversal is deterministic.
 __global__ void k_cell_sort(const int* __restrict__ start, int ncell, int* __restrict__ sorted) {
+  chain_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncell) return;
   const int b = start[c], e = start[c + 1];
@@ -381,6 +386,7 @@ __device__ __forceinline__ double wall_energy(const Walls& w, double y) {
 
 __global__ void k_steric(PairArgs a, int type, double rad, double kT, double fs, double rc, double* __restrict__ F,
                          int accumulate, Walls w) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.Nb) return;
   double f0 = 0, f1 = 0, f2 = 0;
@@ -428,6 +434,7 @@ __global__ void k_wall_overlap(const double* __restrict__ Y, int Nb, double half
 }
 
 __global__ void k_overlap(PairArgs a, double lim, int* __restrict__ flag) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.Nb) return;
   bool hit = false;
@@ -471,14 +478,12 @@ PairArgs pair_args(const Ctx& c) {
 
 int launch_exclusive_scan(const int* in, int* out, int n, cudaStream_t s) {
   if (n <= 2 * SCAN_CH) {  // one or two chunks: one CTA
-    k_exclusive_scan<<<1, SCAN_T, 0, s>>>(in, out, n);
-    FCM_LAUNCH_CHECK();
+    FCM_TRY(launch_chained(k_exclusive_scan, dim3(1), dim3(SCAN_T), 0, s, in, out, n));
     return FCM_OK;
   }
   const int nchunks = (n + SCAN_CH - 1) / SCAN_CH;
   if (n <= SCAN_DIRECT) {
-    k_scan_direct<<<nchunks, SCAN_T, 0, s>>>(in, out, n);
-    FCM_LAUNCH_CHECK();
+    FCM_TRY(launch_chained(k_scan_direct, dim3(nchunks), dim3(SCAN_T), 0, s, in, out, n));
     return FCM_OK;
   }
   k_scan_chunk_sums<<<nchunks, SCAN_T, 0, s>>>(in, out, n);
@@ -500,15 +505,12 @@ int cells_build(Ctx& c, cudaStream_t s) {
     return FCM_OK;
   }
   CellGeom g{c.p.ncells, c.g.Lx, c.g.Ly, c.g.Lz};
-  k_cell_ids<<<(c.Nb + 255) / 256, 256, 0, s>>>(c.d_Y, c.Nb, g, c.d_cell, c.d_cell_count);
-  FCM_LAUNCH_CHECK();
-  k_exclusive_scan<<<1, 1024, 0, s>>>(c.d_cell_count, c.d_cell_start, nc);
-  FCM_LAUNCH_CHECK();
-  k_cell_scatter<<<(c.Nb + 255) / 256, 256, 0, s>>>(c.d_cell, c.Nb, nc, c.d_cell_start, c.d_cell_cursor,
-                                                    c.d_cell_sorted);
-  FCM_LAUNCH_CHECK();
-  k_cell_sort<<<(nc + 255) / 256, 256, 0, s>>>(c.d_cell_start, nc, c.d_cell_sorted);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_cell_ids, dim3((c.Nb + 255) / 256), dim3(256), 0, s, c.d_Y, c.Nb, g, c.d_cell,
+                         c.d_cell_count));
+  FCM_TRY(launch_chained(k_exclusive_scan, dim3(1), dim3(1024), 0, s, c.d_cell_count, c.d_cell_start, nc));
+  FCM_TRY(launch_chained(k_cell_scatter, dim3((c.Nb + 255) / 256), dim3(256), 0, s, c.d_cell, c.Nb, nc, c.d_cell_start,
+                         c.d_cell_cursor, c.d_cell_sorted));
+  FCM_TRY(launch_chained(k_cell_sort, dim3((nc + 255) / 256), dim3(256), 0, s, c.d_cell_start, nc, c.d_cell_sorted));
   return FCM_OK;
 }
 
@@ -520,9 +522,9 @@ Walls walls(const Ctx& c, bool on) {
 
 int cells_steric_forces(const Ctx& c, double* F, bool accumulate, cudaStream_t s, bool with_walls) {
   if (c.Nb == 0) return FCM_OK;
-  k_steric<<<(c.Nb + 127) / 128, 128, 0, s>>>(pair_args(c), c.p.potential, c.p.blob_radius, c.p.kT, c.p.steric_fs,
-                                              c.p.steric_rc, F, accumulate ? 1 : 0, walls(c, with_walls));
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_steric, dim3((c.Nb + 127) / 128), dim3(128), 0, s, pair_args(c), c.p.potential,
+                         c.p.blob_radius, c.p.kT, c.p.steric_fs, c.p.steric_rc, F, accumulate ? 1 : 0, walls(c,
+                         with_walls)));
   return FCM_OK;
 }
 
@@ -545,8 +547,7 @@ int cells_overlap(const Ctx& c, int* d_flag, cudaStream_t s) {
   FCM_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(int), s));
   if (c.Nb == 0) return FCM_OK;
   const double lim = 4.0 * c.p.blob_radius * c.p.blob_radius;
-  k_overlap<<<(c.Nb + 127) / 128, 128, 0, s>>>(pair_args(c), lim, d_flag);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_overlap, dim3((c.Nb + 127) / 128), dim3(128), 0, s, pair_args(c), lim, d_flag));
   return FCM_OK;
 }
 

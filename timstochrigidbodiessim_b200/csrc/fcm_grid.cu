@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(128) k_set_up_gaussians_warp(const double* __r
                                                                double anorm, double anorm2, int* __restrict__ base,
                                                                T* __restrict__ w, T* __restrict__ wc,
                                                                double* __restrict__ ypos) {
+  chain_begin();
   const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= 3LL * n) return;  // uniform over the warp
@@ -148,6 +149,7 @@ __device__ __forceinline__ int overlap_tile(const TileGeom& g, const int f[3], i
 // takes 3-5 us each.
 __global__ void __launch_bounds__(128) k_tile_count(const int* __restrict__ base, int n, TileGeom g,
                                                     int* __restrict__ count) {
+  chain_begin();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int b = (int)(t >> 6), s = (int)(t & 63);
   if (b >= n) return;
@@ -165,6 +167,7 @@ __global__ void __launch_bounds__(128) k_tile_count(const int* __restrict__ base
 __global__ void __launch_bounds__(128) k_tile_fill(const int* __restrict__ base, int n, TileGeom g,
                                                    const int* __restrict__ offset, int* __restrict__ count,
                                                    unsigned long long* __restrict__ list) {
+  chain_begin();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int b = (int)(t >> 6), s = (int)(t & 63);
   if (b >= n) return;
@@ -210,6 +213,7 @@ __global__ void k_tile_sort(const int* __restrict__ offset, int ntiles, unsigned
 constexpr int TSORT = 256;
 __global__ void __launch_bounds__(128) k_tile_sort_warp(const int* __restrict__ offset, int ntiles,
                                                         unsigned long long* __restrict__ list, long long cap) {
+  chain_begin();
   __shared__ unsigned long long buf[4][TSORT];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + w;
@@ -492,6 +496,7 @@ __global__ void __launch_bounds__(32) k_spread_warp(const T* __restrict__ wc, co
                                                     TileGeom g, const int* __restrict__ offset,
                                                     const unsigned long long* __restrict__ list, long long G,
                                                     T* __restrict__ grid) {
+  chain_begin();
   __shared__ __align__(16) T sw[SCB][3][TE];
   __shared__ __align__(16) T sF[SCB][4];
   __shared__ unsigned sflag[SCB];
@@ -1089,6 +1094,7 @@ __global__ void __launch_bounds__(32) k_interp_warp(const T* __restrict__ wc, co
                                                     TileGeom g, const int* __restrict__ offset,
                                                     const unsigned long long* __restrict__ list, long long G,
                                                     T* __restrict__ partial) {
+  chain_begin();
   __shared__ __align__(16) T sw[SCB][3][TE];
   __shared__ unsigned sflag[SCB], sblob[SCB];
   const int tile = blockIdx.x;
@@ -1273,6 +1279,7 @@ __global__ void __launch_bounds__(32) k_spread_mma(const float* __restrict__ wc,
                                                    TileGeom g, const int* __restrict__ offset,
                                                    const unsigned long long* __restrict__ list, long long G,
                                                    float* __restrict__ grid) {
+  chain_begin();
   __shared__ __align__(16) float sw[2][8][3][TE];
   __shared__ __align__(16) float sF[2][8][4];
   const int tile = blockIdx.x;
@@ -1385,6 +1392,7 @@ __global__ void __launch_bounds__(32) k_interp_mma(const float* __restrict__ wc,
                                                    TileGeom g, const int* __restrict__ offset,
                                                    const unsigned long long* __restrict__ list, long long G,
                                                    float* __restrict__ partial, int ntiles) {
+  chain_begin();
   __shared__ __align__(16) float sw[2][SCB][3][TE];
   __shared__ unsigned sflag[2][SCB], sblob[2][SCB];
   __shared__ __align__(16) float sg[2][3 * TE * SGX];
@@ -1571,6 +1579,7 @@ __global__ void __launch_bounds__(32) k_spread_mma64(const double* __restrict__ 
                                                      TileGeom g, const int* __restrict__ offset,
                                                      const unsigned long long* __restrict__ list, long long G,
                                                      double* __restrict__ grid, int ntiles) {
+  chain_begin();
   constexpr int RB = 8;
   __shared__ __align__(16) double sw[2][RB * SBL];
   __shared__ __align__(16) double sF[2][RB][3];
@@ -1674,6 +1683,7 @@ __global__ void __launch_bounds__(32) k_interp_mma64(const double* __restrict__ 
                                                      TileGeom g, const int* __restrict__ offset,
                                                      const unsigned long long* __restrict__ list, long long G,
                                                      double* __restrict__ partial, int ntiles) {
+  chain_begin();
   constexpr int RB = 16;
   __shared__ __align__(16) double sw[2][RB * SBL];
   __shared__ unsigned long long sent[2][RB];
@@ -1857,6 +1867,7 @@ __device__ __forceinline__ void interp_reduce8(const int* __restrict__ base, con
 template <typename T>
 __global__ void __launch_bounds__(128) k_interp_reduce8(const int* __restrict__ base, const T* __restrict__ partial,
                                                         int n, TileGeom g, double dx3, double* __restrict__ V) {
+  chain_begin();
   const int b = blockIdx.x * 16 + (threadIdx.x >> 3);
   double s0, s1, s2;
   interp_reduce8<T>(base, partial, n, g, blockIdx.x, s0, s1, s2);
@@ -1877,6 +1888,7 @@ __global__ void __launch_bounds__(128) k_saddle_end(const int* __restrict__ base
                                                     const double* __restrict__ ref, int rs,
                                                     const double* __restrict__ in, double* __restrict__ out, int M,
                                                     int nb) {
+  chain_begin();
   if ((int)blockIdx.x < rblocks) {
     const int b = blockIdx.x * 16 + (threadIdx.x >> 3);
     double s0, s1, s2;
@@ -1899,6 +1911,7 @@ __global__ void __launch_bounds__(128) k_saddle_end(const int* __restrict__ base
 template <typename T>
 __global__ void k_spread_atomic(const int* __restrict__ base, const T* __restrict__ w, const double* __restrict__ F,
                                 int W, int nx, int ny, int nz, long long G, T* __restrict__ grid) {
+  chain_begin();
   const int np = blockIdx.x;
   const int bx = base[3 * np], by = base[3 * np + 1], bz = base[3 * np + 2];
   const T* gx = w + (size_t)(3 * np) * W;
@@ -1926,6 +1939,7 @@ template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_interp_block(const int* __restrict__ base, const T* __restrict__ w,
                                                      const T* __restrict__ grid, int W, int nx, int ny, int nz,
                                                      long long G, double dx3, double* __restrict__ V, int ycut) {
+  chain_begin();
   const int np = blockIdx.x;
   const int bx = base[3 * np], by = base[3 * np + 1], bz = base[3 * np + 2];
   const T* gx = w + (size_t)(3 * np) * W;
@@ -2055,20 +2069,17 @@ int launch_set_up_gaussians(const Ctx& c, BlobTable<T>& t, const double* dY, cud
   const double anorm = 1.0 / (sqrt(2.0) * a);
   const double anorm2 = 2.0 * a * a / PI;
   const int nt = 3 * t.n;
-  k_set_up_gaussians_warp<T><<<(unsigned)((32LL * nt + 127) / 128), 128, 0, s>>>(dY, t.n, t.W, c.g.dx, anorm, anorm2,
-                                                                               t.base, t.w,
-                                                          t.tiled ? t.wc : nullptr, t.ypos);
-  FCM_LAUNCH_CHECK();
+  if (t.tiled) FCM_CUDA(cudaMemsetAsync(t.tile_count, 0, sizeof(int) * (size_t)t.ntiles, s));
+  FCM_TRY(launch_chained(k_set_up_gaussians_warp<T>, dim3((unsigned)((32LL * nt + 127) / 128)), dim3(128), 0, s, dY,
+                         t.n, t.W, c.g.dx, anorm, anorm2, t.base, t.w, t.tiled ? t.wc : nullptr, t.ypos));
   if (t.tiled) {
     const TileGeom g = tile_geom(c.g, t);
-    FCM_CUDA(cudaMemsetAsync(t.tile_count, 0, sizeof(int) * (size_t)t.ntiles, s));
-    k_tile_count<<<tile_bin_ctas(t.n), 128, 0, s>>>(t.base, t.n, g, t.tile_count);
-    FCM_LAUNCH_CHECK();
+    FCM_TRY(launch_chained(k_tile_count, dim3(tile_bin_ctas(t.n)), dim3(128), 0, s, t.base, t.n, g, t.tile_count));
     FCM_TRY(launch_exclusive_scan(t.tile_count, t.tile_offset, t.ntiles, s));
-    k_tile_fill<<<tile_bin_ctas(t.n), 128, 0, s>>>(t.base, t.n, g, t.tile_offset, t.tile_count, t.tile_list);
-    FCM_LAUNCH_CHECK();
-    k_tile_sort_warp<<<(t.ntiles + 3) / 4, 128, 0, s>>>(t.tile_offset, t.ntiles, t.tile_list, t.tile_cap);
-    FCM_LAUNCH_CHECK();
+    FCM_TRY(launch_chained(k_tile_fill, dim3(tile_bin_ctas(t.n)), dim3(128), 0, s, t.base, t.n, g, t.tile_offset,
+                           t.tile_count, t.tile_list));
+    FCM_TRY(launch_chained(k_tile_sort_warp, dim3((t.ntiles + 3) / 4), dim3(128), 0, s, t.tile_offset, t.ntiles,
+                           t.tile_list, t.tile_cap));
   }
   return FCM_OK;
 }
@@ -2084,7 +2095,9 @@ int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid
     if (v == 0) {
       if constexpr (sizeof(T) == 8) {
         const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_mma64, 32, c.device));
-        k_spread_mma64<<<ctas, 32, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid, t.ntiles);
+        return launch_chained(k_spread_mma64, dim3(ctas), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
+                              c.g.G,
+                              grid, t.ntiles);
       } else {
         const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_pipe<T>, 64, c.device));
         k_spread_pipe<T><<<ctas, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid, t.ntiles);
@@ -2094,10 +2107,12 @@ int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid
     } else if (v == 3) {
       k_spread_tiled<T, 32><<<t.ntiles, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid);
     } else if (v == 4) {
-      k_spread_warp<T><<<t.ntiles, 32, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid);
+      return launch_chained(k_spread_warp<T>, dim3(t.ntiles), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
+                            c.g.G, grid);
     } else if (v == 5 && sizeof(T) == 4) {
       if constexpr (sizeof(T) == 4)
-        k_spread_mma<<<t.ntiles, 32, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid);
+        return launch_chained(k_spread_mma, dim3(t.ntiles), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
+                              c.g.G, grid);
     } else {
       k_spread_tiled<T, 16><<<t.ntiles, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid);
     }
@@ -2106,8 +2121,8 @@ int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid
   }
   FCM_CUDA(cudaMemsetAsync(grid, 0, sizeof(T) * 3 * (size_t)c.g.G, s));
   if (t.n == 0) return FCM_OK;
-  k_spread_atomic<T><<<t.n, 128, 0, s>>>(t.base, t.w, dF, t.W, c.g.nx, c.g.ny, c.g.nz, c.g.G, grid);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_spread_atomic<T>, dim3(t.n), dim3(128), 0, s, t.base, t.w, dF, t.W, c.g.nx, c.g.ny, c.g.nz,
+                         c.g.G, grid));
   return FCM_OK;
 }
 
@@ -2127,21 +2142,19 @@ static int launch_interp_tiles(const Ctx& c, const BlobTable<T>& t, const T* gri
   }
   if constexpr (sizeof(T) == 8) {
     if (v == 1 && aligned) {
-      k_interp_mma64<<<std::min(t.ntiles, persistent_ctas(k_interp_mma64, 32, c.device)), 32, 0, s>>>(
-          t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles);
-      FCM_LAUNCH_CHECK();
+      FCM_TRY(launch_chained(k_interp_mma64, dim3(std::min(t.ntiles, persistent_ctas(k_interp_mma64, 32, c.device))),
+                             dim3(32), 0, s, t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles));
       return FCM_OK;
     }
   } else {
     if (v == 3 && aligned) {
-      k_interp_mma<<<std::min(t.ntiles, persistent_ctas(k_interp_mma, 32, c.device)), 32, 0, s>>>(
-          t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles);
-      FCM_LAUNCH_CHECK();
+      FCM_TRY(launch_chained(k_interp_mma, dim3(std::min(t.ntiles, persistent_ctas(k_interp_mma, 32, c.device))),
+                             dim3(32), 0, s, t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles));
       return FCM_OK;
     }
     if (v == 1) {
-      k_interp_warp<T><<<t.ntiles, 32, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
-      FCM_LAUNCH_CHECK();
+      FCM_TRY(launch_chained(k_interp_warp<T>, dim3(t.ntiles), dim3(32), 0, s, t.wc, grid, g, t.tile_offset,
+                             t.tile_list, c.g.G, t.partial));
       return FCM_OK;
     }
   }
@@ -2157,13 +2170,13 @@ int launch_interp(const Ctx& c, const BlobTable<T>& t, const T* grid, double* dV
   if (t.tiled) {
     TileGeom g;
     FCM_TRY(launch_interp_tiles<T>(c, t, grid, g, s));
-    k_interp_reduce8<T><<<(t.n + 15) / 16, 128, 0, s>>>(t.base, t.partial, t.n, g, dx3, dV);
-    FCM_LAUNCH_CHECK();
+    FCM_TRY(launch_chained(k_interp_reduce8<T>, dim3((t.n + 15) / 16), dim3(128), 0, s, t.base, t.partial, t.n, g, dx3,
+                           dV));
     return FCM_OK;
   }
   const int ycut = c.p.slip_channel ? c.g.ny / 2 : c.g.ny;  // fcm_fluid_solver.cpp:387-389
-  k_interp_block<T, 256><<<t.n, 256, 0, s>>>(t.base, t.w, grid, t.W, c.g.nx, c.g.ny, c.g.nz, c.g.G, dx3, dV, ycut);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_interp_block<T, 256>, dim3(t.n), dim3(256), 0, s, t.base, t.w, grid, t.W, c.g.nx, c.g.ny,
+                         c.g.nz, c.g.G, dx3, dV, ycut));
   return FCM_OK;
 }
 
@@ -2178,9 +2191,8 @@ int launch_saddle_end(const Ctx& c, const BlobTable<T>& t, const T* grid, const 
   TileGeom g;
   FCM_TRY(launch_interp_tiles<T>(c, t, grid, g, s));
   const int rblocks = (t.n + 15) / 16;
-  k_saddle_end<T><<<rblocks + (c.M + 127) / 128, 128, 0, s>>>(t.base, t.partial, t.n, g, c.g.dx * c.g.dx * c.g.dx,
-                                                              rblocks, qm, c.d_ref, c.ref_stride, in, out, c.M, c.nb);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_saddle_end<T>, dim3(rblocks + (c.M + 127) / 128), dim3(128), 0, s, t.base, t.partial, t.n,
+                         g, c.g.dx * c.g.dx * c.g.dx, rblocks, qm, c.d_ref, c.ref_stride, in, out, c.M, c.nb));
   return FCM_OK;
 }
 
@@ -2189,6 +2201,7 @@ int launch_saddle_end(const Ctx& c, const BlobTable<T>& t, const T* grid, const 
 // negated).  Rows above ny/2 read rows below it, which this kernel does not write.
 template <typename T>
 __global__ void k_slip_image(T* __restrict__ grid, int ny, int nz, long long G) {
+  chain_begin();
   const int h = ny / 2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < G; t += (long long)gridDim.x * blockDim.x) {
     const int k = (int)(t % nz);
@@ -2209,8 +2222,7 @@ template <typename T>
 int launch_slip_image(const Ctx& c, T* grid, cudaStream_t s) {
   const long long G = c.g.G;
   const long long nb = std::min<long long>((G + 255) / 256, 148LL * 16);
-  k_slip_image<T><<<(unsigned)nb, 256, 0, s>>>(grid, c.g.ny, c.g.nz, G);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_slip_image<T>, dim3((unsigned)nb), dim3(256), 0, s, grid, c.g.ny, c.g.nz, G));
   return FCM_OK;
 }
 template int launch_slip_image<double>(const Ctx&, double*, cudaStream_t);
@@ -2744,11 +2756,10 @@ extern "C" int fcm_interp_noalloc(int32_t nx, int32_t ny, int32_t nz, double dx,
   k_set_up_gaussians<double><<<(3 * n + 127) / 128, 128, 0, s>>>(Y, n, W, dx, anorm, anorm2, s_base, s_w, s_wc,
                                                                  nullptr);
   FCM_LAUNCH_CHECK();
-  k_tile_count<<<tile_bin_ctas(n), 128, 0, s>>>(s_base, n, g, s_count);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_tile_count, dim3(tile_bin_ctas(n)), dim3(128), 0, s, s_base, n, g, s_count));
   FCM_TRY(launch_exclusive_scan(s_count, s_offset, (int)ntiles, s));
-  k_tile_fill<<<tile_bin_ctas(n), 128, 0, s>>>(s_base, n, g, s_offset, s_count, s_list);
-  FCM_LAUNCH_CHECK();
+  FCM_TRY(launch_chained(k_tile_fill, dim3(tile_bin_ctas(n)), dim3(128), 0, s, s_base, n, g, s_offset, s_count,
+                         s_list));
   k_tile_sort<<<(unsigned)((ntiles + 127) / 128), 128, 0, s>>>(s_offset, (int)ntiles, s_list, (long long)cap);
   FCM_LAUNCH_CHECK();
   k_interp_tiled<double><<<(unsigned)ntiles, 64, 0, s>>>(s_wc, grid, g, s_offset, s_list, G, s_partial);

@@ -125,6 +125,7 @@ __device__ __forceinline__ void tile_item(int i, int& p, int& n) {
 template <typename T, typename C, int XB, int Z1, int Z2, int NT, bool INV>
 __global__ void __launch_bounds__(NT) k_packed_z(C* __restrict__ real, C* __restrict__ spec, Tiles<C, XB> t,
                                                  const C* __restrict__ tw) {
+  chain_begin();
   constexpr int H = Z1 * Z2;
   constexpr int ZM = Z1 > Z2 ? Z1 : Z2;
   constexpr int Q = NT / ZM, YQ = Q / XB;  // lines and rows per CTA
@@ -190,6 +191,7 @@ __global__ void __launch_bounds__(NT) k_packed_z(C* __restrict__ real, C* __rest
 // a contiguous run of 128 ny bytes, the two steps as above.
 template <typename T, typename C, int Y1, int Y2, int NT, bool INV>
 __global__ void __launch_bounds__(NT) k_packed_y(C* __restrict__ spec, const C* __restrict__ tw) {
+  chain_begin();
   constexpr int TK = 128 / (int)sizeof(C);  // values per tile
   extern __shared__ __align__(16) unsigned char packed_smem[];
   V2<T>* s = reinterpret_cast<V2<T>*>(packed_smem);  // [Y1 Y2][TK]
@@ -233,6 +235,7 @@ __global__ void __launch_bounds__(NT) k_packed_y(C* __restrict__ spec, const C* 
 template <typename T, typename C, int XB, int Z1, int Z2, int Y1, int Y2, int NT, bool INV>
 __global__ void __launch_bounds__(NT) k_packed_plane(C* __restrict__ real, C* __restrict__ spec, Tiles<C, XB> t,
                                                      const C* __restrict__ twy, const C* __restrict__ twz) {
+  chain_begin();
   constexpr int H = Z1 * Z2, N = Y1 * Y2, RS = H + 1;
   extern __shared__ __align__(16) unsigned char packed_smem[];
   V2<T>* s = reinterpret_cast<V2<T>*>(packed_smem);
@@ -605,6 +608,7 @@ __device__ __forceinline__ void packed_x_cta(C* __restrict__ spec, const KParams
 template <typename T, typename C, int N1, int N2, int TK, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_packed_x(C* __restrict__ spec, KParams k, const C* __restrict__ twx,
                                                        const C* __restrict__ twz) {
+  chain_begin();
   packed_x_cta<T, C, N1, N2, TK, NT, false>(spec, k, twx, twz, NoiseArgs{});
 }
 
@@ -612,6 +616,7 @@ __global__ void __launch_bounds__(NT, MINB) k_packed_x(C* __restrict__ spec, KPa
 template <typename T, typename C, int N1, int N2, int TK, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_packed_noise(C* __restrict__ spec, KParams k, const C* __restrict__ twx,
                                                            const C* __restrict__ twz, NoiseArgs na) {
+  chain_begin();
   packed_x_cta<T, C, N1, N2, TK, NT, true>(spec, k, twx, twz, na);
 }
 
@@ -620,6 +625,7 @@ template <typename T, typename C, int P, int N1, int N2, int TK, int NT, int MIN
 __global__ void __launch_bounds__(NT, MINB) k_b_packed_x(const BMember* __restrict__ mem, const int* __restrict__ gidx,
                                                          int mask, const C* __restrict__ twx,
                                                          const C* __restrict__ twz) {
+  chain_begin();
   const BMember& m = mem[gidx[blockIdx.z]];
   if (bskip(m, mask)) return;
   packed_x_cta<T, C, N1, N2, TK, NT, false>((C*)m.spec[P], m.kp, twx, twz, NoiseArgs{});
@@ -707,9 +713,7 @@ int packed_z(const Ctx& c, typename cplx_t<T>::type* real, typename cplx_t<T>::t
         FCM_TRY(smem_attr_once(kern, smem));
         const Tiles<C, XB> t(c.g.nx, c.g.ny, c.g.nz);
         const unsigned ctas = (unsigned)(3LL * members * t.nxb * ((t.ny + YQ - 1) / YQ));
-        kern<<<ctas, NT, smem, s>>>(real, spec, t, ztw<T>(c));
-        FCM_LAUNCH_CHECK();
-        return FCM_OK;
+        return launch_chained(kern, dim3(ctas), dim3(NT), smem, s, real, spec, t, ztw<T>(c));
       });
     }
   });
@@ -725,9 +729,7 @@ int packed_y(const Ctx& c, typename cplx_t<T>::type* spec, int members, cudaStre
     auto kern = k_packed_y<T, C, Y1, Y2, NT, INV>;
     FCM_TRY(smem_attr_once(kern, smem));
     const long long per = packed_spectrum_size<T>(c) / ((long long)Y1 * Y2 * (128 / (int)sizeof(C)));  // tile columns
-    kern<<<(unsigned)(per * members), NT, smem, s>>>(spec, ytw<T>(c));
-    FCM_LAUNCH_CHECK();
-    return FCM_OK;
+    return launch_chained(kern, dim3((unsigned)(per * members)), dim3(NT), smem, s, spec, ytw<T>(c));
   });
 }
 
@@ -756,10 +758,8 @@ int packed_plane(const Ctx& c, typename cplx_t<T>::type* real, typename cplx_t<T
           constexpr int XB = decltype(xb)::value;
           auto kern = k_packed_plane<T, C, XB, Z1, Z2, Y1, Y2, NT, INV>;
           FCM_TRY(smem_attr_once(kern, smem));
-          kern<<<(unsigned)(3LL * c.g.nx * members), NT, smem, s>>>(real, spec, Tiles<C, XB>(c.g.nx, c.g.ny, c.g.nz),
-                                                                    ytw<T>(c), ztw<T>(c));
-          FCM_LAUNCH_CHECK();
-          return FCM_OK;
+          return launch_chained(kern, dim3((unsigned)(3LL * c.g.nx * members)), dim3(NT), smem, s, real, spec,
+                                Tiles<C, XB>(c.g.nx, c.g.ny, c.g.nz), ytw<T>(c), ztw<T>(c));
         });
       }
     });
@@ -796,14 +796,12 @@ int packed_x(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s, const
     if (b) {
       auto kern = k_b_packed_x<T, C, P, N1, N2, TK, NT, MB>;
       FCM_TRY(smem_attr_once(kern, smem));
-      kern<<<grid, NT, smem, s>>>(b->mem, gidx, mask, xtw<T>(c), ztw<T>(c));
+      return launch_chained(kern, grid, dim3(NT), smem, s, b->mem, gidx, mask, xtw<T>(c), ztw<T>(c));
     } else {
       auto kern = k_packed_x<T, C, N1, N2, TK, NT, MB>;
       FCM_TRY(smem_attr_once(kern, smem));
-      kern<<<grid, NT, smem, s>>>(spec, make_kparams(c), xtw<T>(c), ztw<T>(c));
+      return launch_chained(kern, grid, dim3(NT), smem, s, spec, make_kparams(c), xtw<T>(c), ztw<T>(c));
     }
-    FCM_LAUNCH_CHECK();
-    return FCM_OK;
   });
 }
 
@@ -857,9 +855,7 @@ int launch_packed_noise(const Ctx& c, cufftDoubleComplex* spec, double* r, uint6
     const dim3 grid((unsigned)((c.g.nz / 4 + TK - 1) / TK), (unsigned)c.g.ny);
     auto kern = k_packed_noise<T, C, N1, N2, TK, NT, MB>;
     FCM_TRY(smem_attr_once(kern, smem));
-    kern<<<grid, NT, smem, s>>>(spec, make_kparams(c), xtw<T>(c), ztw<T>(c), na);
-    FCM_LAUNCH_CHECK();
-    return FCM_OK;
+    return launch_chained(kern, grid, dim3(NT), smem, s, spec, make_kparams(c), xtw<T>(c), ztw<T>(c), na);
   }));
   return launch_packed_inverse<T>(c, spec, r, 1, s);
 }
