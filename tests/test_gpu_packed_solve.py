@@ -22,11 +22,7 @@ def _params(n, nb, **kw):
                               precision=1, **kw)
 
 
-@pytest.mark.parametrize("n", [(8, 8, 8), (12, 8, 12), (8, 12, 16), (16, 8, 12), (24, 16, 8), (24, 24, 24),
-                               (48, 12, 16), (64, 32, 24), (96, 8, 48), (192, 16, 12), (256, 12, 8), (256, 16, 96),
-                               (8, 384, 16), (8, 16, 384), (12, 512, 512), (384, 8, 8), (384, 16, 24), (512, 8, 12),
-                               (512, 12, 16), (16, 48, 48), (8, 96, 96)])
-def test_velocity_field(gpu, n):
+def _against_oracle(n):
     nb = 30
     rng = np.random.default_rng(sum(n))
     Y = (rng.uniform(0, 1, (nb, 3)) * np.array(n)).ravel()
@@ -37,7 +33,6 @@ def test_velocity_field(gpu, n):
         s.set_up_gaussians(Y)
         s.set_up_force_distribution(F)
         s.produce_deterministic_velocity_field()
-    assert g.get_variants()[3] == 2
     ug = g.get_velocity_field(0)
     for c in range(3):
         a, b = (np.asarray(u).reshape(n[0], n[1], -1)[:, :, :n[2]] for u in (ug[c], o.get_grid(3 + c)))
@@ -46,11 +41,37 @@ def test_velocity_field(gpu, n):
     g.spread(F, 1)
     g.stokes_solve(1)
     assert rel_err(g.interp(1), Vo) < 1e-6
+    return g
 
+
+@pytest.mark.parametrize("n", [(8, 8, 8), (12, 8, 12), (8, 12, 16), (16, 8, 12), (24, 16, 8), (24, 24, 24),
+                               (48, 12, 16), (64, 32, 24), (96, 8, 48), (192, 16, 12), (256, 12, 8), (256, 16, 96),
+                               (8, 384, 16), (8, 16, 384), (12, 512, 512), (384, 8, 8), (384, 16, 24), (512, 8, 12),
+                               (512, 12, 16), (16, 48, 48), (8, 96, 96)])
+def test_velocity_field(gpu, n):
+    assert _against_oracle(n).get_variants()[3] == 2
+
+
+@pytest.mark.parametrize("n", [36, 40, 42, 50, 54, 56, 60, 70, 72, 80, 84, 90, 98, 100, 108, 112, 120, 126, 140, 144,
+                               150, 160, 162, 168, 180, 196, 200, 210, 216, 224, 240, 252, 270, 280, 288, 300, 320,
+                               400, 480])
+def test_velocity_field_lengths(gpu, n):
+    """The lengths with 5, 7 or 9 among their register sizes, along each direction and, up
+    to 96 points, as planes by one CTA; half of them odd along z (no column H/2), so are
+    those of the 126 by 90 box.  Tolerances as above."""
+    shapes = [(8, n, 8), (8, 8, n)]
+    if n % (8 if n >= 256 else 4) == 0:
+        shapes += [(n, 8, 12), (n, 12, 90)]
+    if n <= 96:
+        shapes.append((8, n, n))
+    if n in (90, 126):
+        shapes.append((256, 126, 90) if n == 90 else (100, 126, 90))
+    for shape in shapes:
+        _against_oracle(shape)
 
 
 @pytest.mark.parametrize("slip", [0, 1])
-@pytest.mark.parametrize("n", [(8, 8, 8), (16, 24, 12), (24, 16, 16), (64, 48, 32), (256, 8, 16), (384, 12, 8)])
+@pytest.mark.parametrize("n", [(8, 8, 8), (16, 24, 12), (40, 42, 90), (100, 16, 42), (24, 16, 16), (64, 48, 32), (256, 8, 16), (384, 12, 8)])
 def test_fluctuating_field(gpu, n, slip):
     """The FP64 fluctuating field, drawn inside the x pass of the packed spectrum, against
     the same draws in the whole half spectrum with cuFFT's 3D transform, which the FP32

@@ -386,6 +386,8 @@ int fp32_stencil(const Ctx* c) {
 // and nz is even -- for FP64 only up to 256 points, where it measured faster than
 // the 3D transforms (at 512^3 FP64 it was slower) -- and the twiddles
 // exp(-2 pi i j / nx) of both precisions.
+// The packed half-spectrum solve when its lengths include all three, with the twiddles
+// along y and z.
 int setup_xfft(Ctx* c) {
   int n1 = 0, n2 = 0;
   const bool ok = xfft_factor(c->g.nx, &n1, &n2) && c->g.nz % 2 == 0;
@@ -393,46 +395,31 @@ int setup_xfft(Ctx* c) {
   c->xfft[0] = ok && c->g.nx <= 256;  // FP64 beyond 256 points: the 3D transforms unless tuned
   c->xfft_cap[0] = ok;
   c->xfft_cap[1] = c->xfft[1];
-  if (!ok) return FCM_OK;
-  FCM_TRY(xfft_tables_init());
-  const int n = c->g.nx;
+  c->packed_cap = packed_lengths(c->g.nx, c->g.ny, c->g.nz);
+  c->packed_variant = c->packed_cap && ok && xfft_factor(c->g.ny, &n1, &n2) && xfft_factor(c->g.nz, &n1, &n2);
+  c->packed32 = c->packed_variant;
+  if (ok) FCM_TRY(xfft_tables_init());
+  if (c->packed_cap) FCM_TRY(packed_tables_init());
   const double PI = 3.14159265358979323846264338327950288;
-  std::vector<double2> wd(n);
-  std::vector<float2> wf(n);
-  for (int j = 0; j < n; ++j) {
-    wd[j] = make_double2(std::cos(2.0 * PI * j / n), -std::sin(2.0 * PI * j / n));
-    wf[j] = make_float2((float)wd[j].x, (float)wd[j].y);
-  }
-  double2* d64 = nullptr;
-  float2* d32 = nullptr;
-  FCM_TRY(dev_alloc(&d64, (size_t)n));
-  c->d_xtw64 = d64;
-  FCM_TRY(dev_alloc(&d32, (size_t)n));
-  c->d_xtw32 = d32;
-  FCM_CUDA(cudaMemcpy(d64, wd.data(), sizeof(double2) * n, cudaMemcpyHostToDevice));
-  FCM_CUDA(cudaMemcpy(d32, wf.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
-  // all three lengths supported: the packed half-spectrum solve and its twiddles along y, z
-  c->packed_cap = xfft_factor(c->g.ny, &n1, &n2) && xfft_factor(c->g.nz, &n1, &n2);
-  c->packed32 = c->packed_cap;
-  if (c->packed_cap) {
-    FCM_TRY(packed_tables_init());
-    for (int d = 0; d < 2; ++d) {
-      const int m = d == 0 ? c->g.ny : c->g.nz;
-      std::vector<double2> w64(m);
-      std::vector<float2> w32(m);
-      for (int j = 0; j < m; ++j) {
-        w64[j] = make_double2(std::cos(2.0 * PI * j / m), -std::sin(2.0 * PI * j / m));
-        w32[j] = make_float2((float)w64[j].x, (float)w64[j].y);
-      }
-      double2* t64 = nullptr;
-      float2* t32 = nullptr;
-      FCM_TRY(dev_alloc(&t64, (size_t)m));
-      (d == 0 ? c->d_ytw64 : c->d_ztw64) = t64;
-      FCM_TRY(dev_alloc(&t32, (size_t)m));
-      (d == 0 ? c->d_ytw32 : c->d_ztw32) = t32;
-      FCM_CUDA(cudaMemcpy(t64, w64.data(), sizeof(double2) * m, cudaMemcpyHostToDevice));
-      FCM_CUDA(cudaMemcpy(t32, w32.data(), sizeof(float2) * m, cudaMemcpyHostToDevice));
+  const int sides[3] = {c->g.nx, c->g.ny, c->g.nz};
+  void** const d64[3] = {&c->d_xtw64, &c->d_ytw64, &c->d_ztw64};
+  void** const d32[3] = {&c->d_xtw32, &c->d_ytw32, &c->d_ztw32};
+  for (int d = 0; d < (c->packed_cap ? 3 : ok ? 1 : 0); ++d) {
+    const int n = sides[d];
+    std::vector<double2> wd(n);
+    std::vector<float2> wf(n);
+    for (int j = 0; j < n; ++j) {
+      wd[j] = make_double2(std::cos(2.0 * PI * j / n), -std::sin(2.0 * PI * j / n));
+      wf[j] = make_float2((float)wd[j].x, (float)wd[j].y);
     }
+    double2* t64 = nullptr;
+    float2* t32 = nullptr;
+    FCM_TRY(dev_alloc(&t64, (size_t)n));
+    *d64[d] = t64;
+    FCM_TRY(dev_alloc(&t32, (size_t)n));
+    *d32[d] = t32;
+    FCM_CUDA(cudaMemcpy(t64, wd.data(), sizeof(double2) * n, cudaMemcpyHostToDevice));
+    FCM_CUDA(cudaMemcpy(t32, wf.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
   }
   return FCM_OK;
 }
@@ -459,8 +446,8 @@ int ensure_grid(Ctx* c) {
   FCM_CUFFT(cufftSetStream(gb.r2c, c->stream));
   FCM_CUFFT(cufftSetStream(gb.c2r, c->stream));
   // cuFFT's (y, z) transforms of the 3 nx planes, for the fused x-transform on grids
-  // without the packed solve and for FP32 variant 1
-  if (c->xfft_cap[sizeof(T) == 8 ? 0 : 1] && !(sizeof(T) == 8 && c->packed_cap)) {
+  // without the packed solve and for FP32 variant 1 beside it
+  if (c->xfft_cap[sizeof(T) == 8 ? 0 : 1] && (!c->packed_cap || (sizeof(T) == 4 && c->packed_variant))) {
     int n2[2] = {c->g.ny, c->g.nz};
     const int planes = 3 * c->g.nx;
     FCM_CUFFT(cufftPlanMany(&gb.r2c2d, 2, n2, nullptr, 1, c->g.ny * c->g.nz, nullptr, 1, c->g.ny * c->g.nzh,
@@ -2584,7 +2571,7 @@ static int set_variants(Ctx* c, const int32_t* v) {
       return FCM_ERR_INVALID;
     }
     if (P == 1 && c->p.precision != 1) continue;  // no FP32 grid
-    if ((sv >= 1 && !c->xfft_cap[P]) || (sv == 2 && !c->packed_cap)) {
+    if ((sv >= 1 && !c->xfft_cap[P]) || (sv == 2 && !c->packed_variant)) {
       set_error("this grid does not allow solve variant " + std::to_string(sv));
       return FCM_ERR_INVALID;
     }
@@ -2649,7 +2636,7 @@ static int tune_precision(Ctx* c, int reps, double* t) {
   }
   FCM_CUDA(cudaMemsetAsync(gb.r, 0, sizeof(T) * 3 * (size_t)c->g.G, c->stream));
   for (int v = 0; v < 3; ++v) {
-    if ((v >= 1 && !c->xfft_cap[P]) || (v == 2 && (P == 0 || !c->packed_cap))) continue;
+    if ((v >= 1 && !c->xfft_cap[P]) || (v == 2 && (P == 0 || !c->packed_variant))) continue;
     c->xfft[P] = v >= 1;
     if (P == 1) c->packed32 = v == 2;
     FCM_TRY(time_calls(c, reps, [&] { return stokes_t<T>(c); }, &t[6 + v]));
@@ -2715,7 +2702,7 @@ int fcm_debug_bounds(int32_t* checked, int64_t* count, int32_t* site, int64_t* i
     const int on = 0;
 #endif
     int (*readers[])(BoundsRecord*, int) = {bounds_read_grid, bounds_read_cells, bounds_read_kspace,
-                                            bounds_read_packed, bounds_read_blas};
+                                            bounds_read_packed, bounds_read_packed_x, bounds_read_blas};
     unsigned long long total = 0;
     BoundsRecord first{};
     for (auto rd : readers) {

@@ -162,6 +162,7 @@ int bounds_read_grid(BoundsRecord* out, int reset);
 int bounds_read_cells(BoundsRecord* out, int reset);
 int bounds_read_kspace(BoundsRecord* out, int reset);
 int bounds_read_packed(BoundsRecord* out, int reset);
+int bounds_read_packed_x(BoundsRecord* out, int reset);
 int bounds_read_blas(BoundsRecord* out, int reset);
 
 template <typename T>
@@ -364,10 +365,12 @@ struct Ctx {
   // on when nx is a supported length and nz is even (FP64 up to 256 points, beyond
   // which the 3D transforms are faster); twiddles exp(-2 pi i j / nx), j < nx
   bool xfft[2] = {false, false};
-  // the packed half-spectrum solve (fcm_packed.cu): all three lengths supported; FP32
-  // solve variant 2 (packed32) and the FP64 fused variant take it, see use_packed;
-  // twiddles exp(-2 pi i j / n) for n = ny, nz in both precisions
+  // the packed half-spectrum solve (fcm_packed.cuh): all three lengths among its own;
+  // packed_variant where they are among those of the fused x-transform too and solve
+  // variant 2 (packed32) selects it in FP32, see use_packed; twiddles exp(-2 pi i j / n)
+  // for n = nx, ny, nz in both precisions
   bool packed_cap = false;
+  bool packed_variant = false;
   bool packed32 = false;
   // what the grids allow (fcm_autotune chooses within it): the fused x-transform per
   // precision (its (y, z) plans exist)
@@ -410,13 +413,20 @@ struct Ctx {
   int urand_prec = 0;       // precision of the random field last produced
 };
 
-// Whether the Stokes solve of precision P runs on the packed half spectrum: FP32 by
-// variant 2; FP64 where the lengths allow it by variant 1, and beyond 256 points along x
-// by variant 0 too, whose cuFFT 3D transforms took 9.42 ms at 512^3 against 6.49 ms (6.01
-// against 2.65 ms at 384^3).
+// Whether the Stokes solve of precision P runs on the packed half spectrum.  Where the
+// lengths are those of the fused x-transform too: FP32 by variant 2, FP64 by variant 1, and
+// beyond 256 points along x by variant 0 as well, whose cuFFT 3D transforms took 9.42 ms at
+// 512^3 against 6.49 ms (6.01 against 2.65 ms at 384^3).  Where only the packed transforms
+// have the lengths (5, 7 or 9 among the factors), in place of cuFFT's transforms in the
+// variant the grid has, faster at every one measured (us, FP64 / FP32): 40^3 11 / 11 (35 /
+// 29), 72^3 28 / 19 (56 / 47), 100 x 126 x 90 61 / 42 (102 / 83), 144^3 150 / 75 (193 / 121),
+// 168^3 240 / 131 (572 / 360), 240^3 671 / 359 (1593 / 843), 320^3 1619 / 914 (3384 / 1995),
+// 400^3 3820 / 1880 (9610 / 5600).
 inline bool use_packed(const Ctx& c, int P) {
   if (!c.packed_cap) return false;
-  return P == 1 ? c.xfft[1] && c.packed32 : c.xfft[0] || c.g.nx > 256;
+  if (!c.xfft_cap[P]) return true;
+  if (P == 1) return c.xfft[1] && (c.packed32 || !c.packed_variant);
+  return c.xfft[0] || c.g.nx > 256;
 }
 
 // ------------------------------------------------------------------ batches
@@ -590,6 +600,8 @@ int launch_xfft_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream
 // the packed half-spectrum solve (fcm_packed.cu) of `members` consecutive grids of c's
 // shape: (y, z) transforms, x transforms with the projection, inverse (y, z) transforms
 int packed_tables_init();
+int packed_zy_tables_init();  // by packed_tables_init
+bool packed_lengths(int nx, int ny, int nz);  // whether the packed solve takes this grid
 template <typename T>
 long long packed_spectrum_size(const Ctx& c);  // complex values of one grid's spectrum
 template <typename T>

@@ -730,7 +730,7 @@ int xfft_dispatch(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s, 
 
 }  // namespace
 
-int xfft_tables_init() { return w96_upload(); }
+int xfft_tables_init() { return roots_upload(); }
 
 template <typename T>
 int launch_xfft_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s) {
