@@ -15,8 +15,18 @@
 // (no index arithmetic beyond the entry), accumulates its 512 points in registers
 // and writes every point of the tile exactly once (the zero-fill of
 // fcm_fluid_solver.cpp:556-562 is fused: tiles without blobs write zeros).  No
-// atomics touch the grid.  Grids that cannot be tiled (a dimension not a multiple
-// of 8, W + 8 > n, or W > 25) use the per-blob atomic scatter.
+// atomics touch the grid.
+//
+// Uneven tiles.  A dimension of n points that is not a multiple of 8 is cut into
+// ceil(n / 8) tiles, q = n - 7 ceil(n / 8) of 8 points, then tiles of 7 (n >= 7 ceil(n / 8):
+// every even n but 34 from 28 on).  Three tiles of 7 and a point hold the widest stencil
+// allowed there, W = 22.  The chunks follow the tiles: the eighth weight of a 7-point tile is
+// zero, so the kernels run as on whole tiles, leave that point out of the loads and stores
+// and take no vector accesses along z.  250 rods in a 100 x 126 x 90 box, FP64: spreading
+// 21 us and interpolation 26 us against 78 and 37 by the per-blob kernels below.
+//
+// Grids that cannot be tiled (W + 8 > n, W > 25, or uneven and W > 22) use the per-blob
+// atomic scatter.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -33,6 +43,7 @@ namespace {
 constexpr int TE = 8;    // tile edge
 constexpr int NCH = 4;   // 8-aligned chunks a stencil of at most 25 points meets per dimension
 constexpr int MAXW = 25;
+constexpr int MAXW_UNEVEN = 22;  // what four tiles hold when they may have 7 points
 constexpr int SCB = 16;  // blobs staged per round (four staging lanes per blob, 64 threads)
 
 // Entry layout (low word): bits 0-5 chunk index per dimension (2 bits each),
@@ -45,7 +56,52 @@ __device__ __forceinline__ int wrap_index(int i, int n) {
   return r < 0 ? r + n : r;
 }
 
+// The period of x: floor(x / n), without a division within a period of [0, n).
+__device__ __forceinline__ int period(int x, int n) {
+  if (x >= 0 && x < n) return 0;
+  if (x < 0 && x >= -n) return -1;
+  if (x >= n && x - n < n) return 1;
+  return x >= 0 ? x / n : -((-(x + 1)) / n + 1);
+}
+
 __device__ __forceinline__ int floordiv(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+
+// Tiles of a direction of n points in nt tiles, the first q of 8 points, the others of 7,
+// continued periodically: the tile of point x and the first point of tile t.
+__device__ __forceinline__ int tile_of(int x, int n, int nt, int q) {
+  if (q == nt) return floordiv(x, TE);
+  const int p = period(x, n), r = x - p * n;
+  return p * nt + (r < TE * q ? r / TE : q + (r - TE * q) / (TE - 1));
+}
+__device__ __forceinline__ int tile_start(int t, int n, int nt, int q) {
+  if (q == nt) return t * TE;
+  const int p = period(t, nt), r = t - p * nt;
+  return p * n + TE * r - max(0, r - q);
+}
+
+// First point and points per direction of a tile.
+template <bool UNEVEN>
+struct TileBox {
+  int ox, oy, oz, ex, ey, ez;
+  __device__ __forceinline__ TileBox(const TileGeom& g, int tile) {
+    const int tz = tile % g.ntz, ty = (tile / g.ntz) % g.nty, tx = tile / (g.ntz * g.nty);
+    ox = tx * TE;
+    oy = ty * TE;
+    oz = tz * TE;
+    ex = ey = ez = TE;
+    if constexpr (UNEVEN) {
+      ox -= max(0, tx - g.qx);
+      oy -= max(0, ty - g.qy);
+      oz -= max(0, tz - g.qz);
+      if (tx >= g.qx) ex = TE - 1;
+      if (ty >= g.qy) ey = TE - 1;
+      if (tz >= g.qz) ez = TE - 1;
+    }
+  }
+  __device__ __forceinline__ bool has(int x, int y, int z) const {
+    return !UNEVEN || (x < ex && y < ey && z < ez);
+  }
+};
 
 // One thread per (blob, dimension): xc = int(Y/DX); stencil start
 // xc - W/2 + 1; weight anorm*exp(-(xg*DX - Y)^2/anorm2), with sigma = a/sqrt(pi)
@@ -79,54 +135,14 @@ __global__ void k_set_up_gaussians(const double* __restrict__ Y, int n, int W, d
   }
 }
 
-// The same tables with one warp per (blob, dimension): lane i takes grid point
-// c0 + i of the blob's NCH * TE = 32-point chunk window (c0 = floor(base/8)*8),
-// evaluates its weight with the arithmetic above when it lies in the stencil
-// (s = c0 + i - base in [0, W)) and writes wc[i] and w[s]; every store is
-// coalesced and each weight is computed once (the window holds the stencil since
-// W <= 25 on tiled grids).  Without wc the lanes write w[i], i = lane, lane + 32, ...
-template <typename T>
-__global__ void __launch_bounds__(128) k_set_up_gaussians_warp(const double* __restrict__ Y, int n, int W, double dx,
-                                                               double anorm, double anorm2, int* __restrict__ base,
-                                                               T* __restrict__ w, T* __restrict__ wc,
-                                                               double* __restrict__ ypos) {
-  chain_begin();
-  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t >= 3LL * n) return;  // uniform over the warp
-  const double y = Y[t];
-  const int xc = (int)__ddiv_rn(y, dx);
-  const int b = xc - W / 2 + 1;
-  if (lane == 0) {
-    base[t] = b;
-    if (ypos) ypos[t] = y;
-  }
-  if (!wc) {
-    for (int i = lane; i < W; i += 32) {
-      const double xx = __dsub_rn(__dmul_rn((double)(b + i), dx), y);
-      w[t * W + i] = (T)(anorm * exp(__ddiv_rn(-__dmul_rn(xx, xx), anorm2)));
-    }
-    return;
-  }
-  const int c0 = floordiv(b, TE) * TE;  // first grid point of the window
-  const int g = c0 + lane, sidx = g - b;
-  T val = (T)0;
-  if (sidx >= 0 && sidx < W) {
-    const double xx = __dsub_rn(__dmul_rn((double)g, dx), y);
-    const double e = exp(__ddiv_rn(-__dmul_rn(xx, xx), anorm2));
-    val = (T)(anorm * e);
-    w[t * W + sidx] = val;
-  }
-  wc[t * NCH * TE + lane] = val;
-}
-
 // (blob, tile) overlaps of a blob: per dimension the tiles first..first+cnt-1.
 __device__ __forceinline__ void blob_tiles(const int* base, int b, const TileGeom& g, int f[3], int cnt[3]) {
+  const int n[3] = {g.nx, g.ny, g.nz}, nt[3] = {g.ntx, g.nty, g.ntz}, q[3] = {g.qx, g.qy, g.qz};
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const int lo = base[3 * b + d];
-    f[d] = floordiv(lo, TE);
-    cnt[d] = floordiv(lo + g.W - 1, TE) - f[d] + 1;
+    f[d] = tile_of(lo, n[d], nt[d], q[d]);
+    cnt[d] = tile_of(lo + g.W - 1, n[d], nt[d], q[d]) - f[d] + 1;
   }
 }
 
@@ -138,32 +154,101 @@ __device__ __forceinline__ unsigned half_mask(int lo, int W, int s) {
 
 // The tile of overlap (ox, oy, oz) of a blob whose first tile is f, periodic.
 __device__ __forceinline__ int overlap_tile(const TileGeom& g, const int f[3], int ox, int oy, int oz) {
-  return (wrap_index(f[0] + ox, g.ntx) * g.nty + wrap_index(f[1] + oy, g.nty)) * g.ntz + wrap_index(f[2] + oz, g.ntz);
+  const int x = f[0] + ox, y = f[1] + oy, z = f[2] + oz;
+  return ((x - period(x, g.ntx) * g.ntx) * g.nty + y - period(y, g.nty) * g.nty) * g.ntz + z -
+         period(z, g.ntz) * g.ntz;
 }
 
-// Overlaps per tile: one thread per (blob, candidate), the 4 x 4 x 4 candidate
-// tiles of a blob (a stencil of at most 25 points meets at most four per
-// dimension) beginning at its first tile.  A thread per blob walking its overlaps
-// waited for every atomic in turn: 34 us for the 192 blobs of a 64^3 grid and 58 us
-// for 12,288 at 256^3 in the fill, 12 us each in the count; one thread per candidate
-// takes 3-5 us each.
+// Overlap s of a blob with the 4 x 4 x 4 tiles beginning at its first one (a stencil of at
+// most 25 points meets at most four per dimension): its tile, or -1 where there is none.
+__device__ __forceinline__ int candidate_tile(const TileGeom& g, const int f[3], const int cnt[3], int s) {
+  const int ox = s >> 4, oy = (s >> 2) & 3, oz = s & 3;
+  if (ox >= cnt[0] || oy >= cnt[1] || oz >= cnt[2]) return -1;
+  const int tile = overlap_tile(g, f, ox, oy, oz);
+  return FCM_INB(tile, (long long)g.ntx * g.nty * g.ntz, BS_TILE) ? tile : -1;
+}
+
+// Overlaps per tile: one thread per (blob, candidate).  A thread per blob walking its
+// overlaps waited for every atomic in turn: 34 us for the 192 blobs of a 64^3 grid and 58 us
+// for 12,288 at 256^3 in the fill, 12 us each in the count.
 __global__ void __launch_bounds__(128) k_tile_count(const int* __restrict__ base, int n, TileGeom g,
                                                     int* __restrict__ count) {
   chain_begin();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int b = (int)(t >> 6), s = (int)(t & 63);
+  const int b = (int)(t >> 6);
   if (b >= n) return;
-  const int ox = s >> 4, oy = (s >> 2) & 3, oz = s & 3;
   int f[3], cnt[3];
   blob_tiles(base, b, g, f, cnt);
-  if (ox >= cnt[0] || oy >= cnt[1] || oz >= cnt[2]) return;
-  const int tile = overlap_tile(g, f, ox, oy, oz);
-  if (FCM_INB(tile, (long long)g.ntx * g.nty * g.ntz, BS_TILE)) atomicAdd(count + tile, 1);
+  const int tile = candidate_tile(g, f, cnt, (int)(t & 63));
+  if (tile >= 0) atomicAdd(count + tile, 1);
 }
 
-// The list entries, same threads: each takes the last free slot of its tile by
-// counting the tile's overlaps down again (the order within a tile is restored by
-// the sort).
+// The same tables with one warp per (blob, dimension), two blobs per CTA: lane i takes
+// grid point c0 + i of the blob's NCH * TE = 32-point chunk window (c0 = floor(base/8)*8),
+// evaluates its weight with the arithmetic above when it lies in the stencil
+// (s = c0 + i - base in [0, W)) and writes wc[i] and w[s]; every store is coalesced and
+// each weight is computed once (the window holds the stencil since W <= 25 on tiled grids).
+// On uneven tiles lane 8 k + i takes point i of tile k from the stencil's first one.  Then
+// 64 threads per blob count its overlaps (a launch of its own took 8 us for 12,288 blobs).
+// Without wc the lanes write w[i], i = lane, lane + 32, ...
+template <typename T>
+__global__ void __launch_bounds__(192) k_set_up_gaussians_warp(const double* __restrict__ Y, int n, int W, double dx,
+                                                               double anorm, double anorm2, int* __restrict__ base,
+                                                               T* __restrict__ w, T* __restrict__ wc,
+                                                               double* __restrict__ ypos, TileGeom tg,
+                                                               int* __restrict__ count) {
+  chain_begin();
+  __shared__ int sb[6];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long t = 6LL * blockIdx.x + wid;
+  if (t < 3LL * n) {  // uniform over the warp
+    const double y = Y[t];
+    const int xc = (int)__ddiv_rn(y, dx);
+    const int b = xc - W / 2 + 1;
+    if (lane == 0) {
+      base[t] = sb[wid] = b;
+      if (ypos) ypos[t] = y;
+    }
+    if (!wc) {
+      for (int i = lane; i < W; i += 32) {
+        const double xx = __dsub_rn(__dmul_rn((double)(b + i), dx), y);
+        w[t * W + i] = (T)(anorm * exp(__ddiv_rn(-__dmul_rn(xx, xx), anorm2)));
+      }
+      return;  // every warp of every CTA: wc is the launch's
+    }
+    const int d = wid % 3;
+    const int dn = d == 0 ? tg.nx : d == 1 ? tg.ny : tg.nz, dt = d == 0 ? tg.ntx : d == 1 ? tg.nty : tg.ntz;
+    const int dq = d == 0 ? tg.qx : d == 1 ? tg.qy : tg.qz;
+    int g = floordiv(b, TE) * TE + lane, next = g + 1;  // the lane's grid point, the first one not of its tile
+    if (dq != dt) {
+      const int k = tile_of(b, dn, dt, dq) + (lane >> 3);
+      g = tile_start(k, dn, dt, dq) + (lane & 7);
+      next = tile_start(k + 1, dn, dt, dq);
+    }
+    const int sidx = g - b;
+    T val = (T)0;
+    if (sidx >= 0 && sidx < W && g < next) {
+      const double xx = __dsub_rn(__dmul_rn((double)g, dx), y);
+      const double e = exp(__ddiv_rn(-__dmul_rn(xx, xx), anorm2));
+      val = (T)(anorm * e);
+      w[t * W + sidx] = val;
+    }
+    wc[t * NCH * TE + lane] = val;
+  }
+  if (!wc) return;
+  __syncthreads();
+  const int k = threadIdx.x >> 6;
+  if (k < 2 && 2LL * blockIdx.x + k < n) {
+    int f[3], cnt[3];
+    blob_tiles(sb, k, tg, f, cnt);
+    const int tile = candidate_tile(tg, f, cnt, threadIdx.x & 63);
+    if (tile >= 0) atomicAdd(count + tile, 1);
+  }
+}
+
+// The list entries, one thread per (blob, candidate): each takes the last free slot of its
+// tile by counting the tile's overlaps down again, so the counts end as zeros (the order
+// within a tile is restored by the sort).
 __global__ void __launch_bounds__(128) k_tile_fill(const int* __restrict__ base, int n, TileGeom g,
                                                    const int* __restrict__ offset, int* __restrict__ count,
                                                    unsigned long long* __restrict__ list) {
@@ -171,18 +256,17 @@ __global__ void __launch_bounds__(128) k_tile_fill(const int* __restrict__ base,
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int b = (int)(t >> 6), s = (int)(t & 63);
   if (b >= n) return;
-  const int ox = s >> 4, oy = (s >> 2) & 3, oz = s & 3;
   int f[3], cnt[3];
   blob_tiles(base, b, g, f, cnt);
-  if (ox >= cnt[0] || oy >= cnt[1] || oz >= cnt[2]) return;
-  const int tile = overlap_tile(g, f, ox, oy, oz);
-  if (!FCM_INB(tile, (long long)g.ntx * g.nty * g.ntz, BS_TILE)) return;
+  const int tile = candidate_tile(g, f, cnt, s);
+  if (tile < 0) return;
+  const int slot = offset[tile] + atomicSub(count + tile, 1) - 1;
+  const int ox = s >> 4, oy = (s >> 2) & 3, oz = s & 3;
   const unsigned j = (unsigned)((ox * cnt[1] + oy) * cnt[2] + oz);
   const unsigned lo = (unsigned)ox | ((unsigned)oy << 2) | ((unsigned)oz << 4) | (j << EJ) |
-                      (half_mask(base[3 * b], g.W, (f[0] + ox) * TE) << EXM) |
-                      (half_mask(base[3 * b + 1], g.W, (f[1] + oy) * TE) << EYM) |
-                      (half_mask(base[3 * b + 2], g.W, (f[2] + oz) * TE) << EZM);
-  const int slot = offset[tile] + atomicSub(count + tile, 1) - 1;
+                      (half_mask(base[3 * b], g.W, tile_start(f[0] + ox, g.nx, g.ntx, g.qx)) << EXM) |
+                      (half_mask(base[3 * b + 1], g.W, tile_start(f[1] + oy, g.ny, g.nty, g.qy)) << EYM) |
+                      (half_mask(base[3 * b + 2], g.W, tile_start(f[2] + oz, g.nz, g.ntz, g.qz)) << EZM);
   if (FCM_INB(slot - offset[tile], (long long)offset[tile + 1] - offset[tile], BS_LIST) &&
       FCM_INB(slot, g.list_cap, BS_LIST))
     list[slot] = ((unsigned long long)b << 32) | lo;
@@ -206,55 +290,63 @@ __global__ void k_tile_sort(const int* __restrict__ offset, int ntiles, unsigned
   }
 }
 
-// The same order, one warp per tile: the tile's entries (all distinct) are
-// loaded into a shared buffer padded to a power of two with all-ones keys and
-// bitonic-sorted by the warp; tiles with more than TSORT entries are sorted by
-// lane 0 in place as k_tile_sort does.  128 threads = four tiles per CTA.
+// The same order, one warp per tile: E entries per lane, each placed by its rank, the number
+// of smaller blob ids in the tile (read four at a time from shared memory, padded with
+// ids above all others).  No step waits for another, as those of a bitonic sort did: the
+// lists of 2048 rods at 256^3 (15 entries) take 9.9 us instead of 20, those of 24,000 blobs
+// in 12,831 tiles (80 entries) 17.5 us instead of 41.
+template <int E>
+__device__ __forceinline__ void sort_by_rank(unsigned long long* __restrict__ list, int n, unsigned* keys) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long e[E];
+  int r[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    e[i] = lane + 32 * i < n ? list[lane + 32 * i] : ~0ull;
+    keys[lane + 32 * i] = (unsigned)(e[i] >> 32);
+    r[i] = 0;
+  }
+  __syncwarp();  // every entry read before the first is written
+  for (int k = 0; k < n; k += 4) {
+    const uint4 o = *reinterpret_cast<const uint4*>(keys + k);
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const unsigned key = (unsigned)(e[i] >> 32);
+      r[i] += (o.x < key) + (o.y < key) + (o.z < key) + (o.w < key);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < E; ++i)
+    if (lane + 32 * i < n) list[r[i]] = e[i];
+}
+
+// 128 threads = four tiles per CTA; tiles with more than TSORT entries are sorted by lane 0
+// in place as k_tile_sort does.
 constexpr int TSORT = 256;
 __global__ void __launch_bounds__(128) k_tile_sort_warp(const int* __restrict__ offset, int ntiles,
                                                         unsigned long long* __restrict__ list, long long cap) {
   chain_begin();
-  __shared__ unsigned long long buf[4][TSORT];
+  __shared__ __align__(16) unsigned keys[4][TSORT];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + w;
   if (t >= ntiles) return;  // uniform over the warp
   const int b = offset[t], e = offset[t + 1], n = e - b;
   if (!FCM_INB(b, (long long)e + 1, BS_LIST) || !FCM_INB(e, cap + 1, BS_LIST)) return;  // uniform over the warp
   if (n < 2) return;
-  if (n > TSORT) {
-    if (lane == 0)
-      for (int i = b + 1; i < e; ++i) {
-        const unsigned long long v = list[i];
-        int j = i - 1;
-        while (j >= b && list[j] > v) {
-          list[j + 1] = list[j];
-          --j;
-        }
-        list[j + 1] = v;
+  if (n <= 32) return sort_by_rank<1>(list + b, n, keys[w]);
+  if (n <= 64) return sort_by_rank<2>(list + b, n, keys[w]);
+  if (n <= 128) return sort_by_rank<4>(list + b, n, keys[w]);
+  if (n <= TSORT) return sort_by_rank<8>(list + b, n, keys[w]);
+  if (lane == 0)
+    for (int i = b + 1; i < e; ++i) {
+      const unsigned long long v = list[i];
+      int j = i - 1;
+      while (j >= b && list[j] > v) {
+        list[j + 1] = list[j];
+        --j;
       }
-    return;
-  }
-  int P = 2;
-  while (P < n) P <<= 1;
-  unsigned long long* a = buf[w];
-  for (int i = lane; i < P; i += 32) a[i] = i < n ? list[b + i] : ~0ull;
-  __syncwarp();
-  for (int k = 2; k <= P; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < P; i += 32) {
-        const int l = i ^ j;
-        if (l > i) {
-          const unsigned long long x = a[i], y = a[l];
-          const bool up = (i & k) == 0;
-          if ((x > y) == up) {
-            a[i] = y;
-            a[l] = x;
-          }
-        }
-      }
-      __syncwarp();
+      list[j + 1] = v;
     }
-  for (int i = lane; i < n; i += 32) list[b + i] = a[i];
 }
 
 // Eight consecutive T from global (aligned to 8*sizeof(T)) to shared memory.
@@ -491,7 +583,7 @@ __global__ void __launch_bounds__(64) k_spread_tiled(const T* __restrict__ wc, c
 // blob are read once for both rows.  Every point sums its blobs in ascending order
 // with the products of k_spread_tiled (f_c = F_c wy wz, then f_c wx), so the grid
 // is the same bit for bit.
-template <typename T>
+template <typename T, bool UNEVEN>
 __global__ void __launch_bounds__(32) k_spread_warp(const T* __restrict__ wc, const double* __restrict__ F,
                                                     TileGeom g, const int* __restrict__ offset,
                                                     const unsigned long long* __restrict__ list, long long G,
@@ -504,7 +596,7 @@ __global__ void __launch_bounds__(32) k_spread_warp(const T* __restrict__ wc, co
   if (!FCM_INB(tile, (long long)g.ntx * g.nty * g.ntz, BS_TILE)) return;  // uniform over the warp
   int b0, b1;
   tile_range(offset, tile, g, b0, b1);
-  const int tz = tile % g.ntz, ty = (tile / g.ntz) % g.nty, tx = tile / (g.ntz * g.nty);
+  const TileBox<UNEVEN> box(g, tile);
   const int lane = threadIdx.x, z = lane & 7, yq = lane >> 3;
   constexpr int XA = sizeof(T) == 4 ? TE / 2 : TE;  // x accumulators per row (pairs in FP32)
   using A = typename std::conditional<sizeof(T) == 4, float2, T>::type;
@@ -573,11 +665,11 @@ __global__ void __launch_bounds__(32) k_spread_warp(const T* __restrict__ wc, co
   }
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    const int ox = tx * TE, oy = ty * TE + yq + 4 * r, oz = tz * TE + z;
+    const int oy = box.oy + yq + 4 * r, oz = box.oz + z;
 #pragma unroll
     for (int x = 0; x < TE; ++x) {
-      const long long idx = ((long long)(ox + x) * g.ny + oy) * g.nz + oz;
-      if (!FCM_INB(idx, G, BS_GRID)) continue;
+      const long long idx = ((long long)(box.ox + x) * g.ny + oy) * g.nz + oz;
+      if (!box.has(x, yq + 4 * r, z) || !FCM_INB(idx, G, BS_GRID)) continue;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         if constexpr (sizeof(T) == 4)
@@ -1089,7 +1181,7 @@ __global__ void __launch_bounds__(64 / R) k_interp_rows(const T* __restrict__ wc
 // lanes 2i write value i straight to partial[blob][j][c].  Against the 64-thread
 // kernel this halves the reductions per (blob, tile) pair and needs no CTA
 // barrier or shared-memory sum: only the staged weights pass through shared memory.
-template <typename T>
+template <typename T, bool UNEVEN>
 __global__ void __launch_bounds__(32) k_interp_warp(const T* __restrict__ wc, const T* __restrict__ grid,
                                                     TileGeom g, const int* __restrict__ offset,
                                                     const unsigned long long* __restrict__ list, long long G,
@@ -1102,17 +1194,17 @@ __global__ void __launch_bounds__(32) k_interp_warp(const T* __restrict__ wc, co
   int b0, b1;
   tile_range(offset, tile, g, b0, b1);
   if (b0 == b1) return;  // no blob meets this tile
-  const int tz = tile % g.ntz, ty = (tile / g.ntz) % g.nty, tx = tile / (g.ntz * g.nty);
+  const TileBox<UNEVEN> box(g, tile);
   const int lane = threadIdx.x, z = lane & 7, yq = lane >> 3;
   XColumn<T> col[2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    const int ox = tx * TE, oy = ty * TE + yq + 4 * r, oz = tz * TE + z;
+    const int oy = box.oy + yq + 4 * r, oz = box.oz + z;
     const bool live = oy < g.ycut;  // rows at or above the slip channel's upper wall read as 0
 #pragma unroll
     for (int x = 0; x < TE; ++x) {
-      const long long idx = ((long long)(ox + x) * g.ny + oy) * g.nz + oz;
-      const bool in = live && FCM_INB(idx, G, BS_GRID);
+      const long long idx = ((long long)(box.ox + x) * g.ny + oy) * g.nz + oz;
+      const bool in = live && box.has(x, yq + 4 * r, z) && FCM_INB(idx, G, BS_GRID);
       col[r].set(x, in ? grid[idx] : (T)0, in ? grid[G + idx] : (T)0, in ? grid[2 * G + idx] : (T)0);
     }
   }
@@ -1575,6 +1667,7 @@ __device__ __forceinline__ void stage_part64(double* sw, double* sF, const doubl
 // kernel 24 (283 us at 256^3 with 57.7 blobs per tile, 2048 rods 111 us; the 64-thread
 // pipelined FMA kernel took 362 and 126 us).  Two warps per tile (a y-half each, twice
 // the warps per SM) measured level, so the chip is not short of warps here.
+template <bool UNEVEN>
 __global__ void __launch_bounds__(32) k_spread_mma64(const double* __restrict__ wc, const double* __restrict__ F,
                                                      TileGeom g, const int* __restrict__ offset,
                                                      const unsigned long long* __restrict__ list, long long G,
@@ -1628,9 +1721,9 @@ __global__ void __launch_bounds__(32) k_spread_mma64(const double* __restrict__ 
       }
     }
     if (cur.last) {  // the tile is complete: every point written once
-      const int tz = cur.tile % g.ntz, ty = (cur.tile / g.ntz) % g.nty, tx = cur.tile / (g.ntz * g.nty);
+      const TileBox<UNEVEN> box(g, cur.tile);
       const long long xs = (long long)g.ny * g.nz;
-      const long long i0 = ((long long)(tx * TE + 2 * tq) * g.ny + ty * TE) * g.nz + tz * TE + gq;
+      const long long i0 = ((long long)(box.ox + 2 * tq) * g.ny + box.oy) * g.nz + box.oz + gq;
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -1638,7 +1731,7 @@ __global__ void __launch_bounds__(32) k_spread_mma64(const double* __restrict__ 
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const long long idx = i0 + h * xs + (long long)y * g.nz;
-            if (FCM_INB(idx, G, BS_GRID)) grid[c * G + idx] = acc[c][y][h];
+            if (box.has(2 * tq + h, y, gq) && FCM_INB(idx, G, BS_GRID)) grid[c * G + idx] = acc[c][y][h];
             acc[c][y][h] = 0.0;
           }
     }
@@ -1663,12 +1756,28 @@ __global__ void __launch_bounds__(32) k_spread_mma64(const double* __restrict__ 
 // contiguous ranges of tiles with equal shares of the list entries 360 us.
 constexpr int SGX64 = TE * TE + 4;  // padded x-plane: the fragment reads fall in different banks
 
+template <bool UNEVEN>
 __device__ __forceinline__ void grid_tile_async64(const double* __restrict__ grid, const TileGeom& g, long long G,
                                                   int tile, double* sg) {
-  const int tz = tile % g.ntz, ty = (tile / g.ntz) % g.nty, tx = tile / (g.ntz * g.nty);
-  const int y = threadIdx.x >> 2, part = threadIdx.x & 3;  // row y of every (component, x), a quarter of its 64 bytes
-  const long long i0 = ((long long)(tx * TE) * g.ny + ty * TE + y) * g.nz + tz * TE + 2 * part;
+  const TileBox<UNEVEN> box(g, tile);
   const long long xs = (long long)g.ny * g.nz;
+  if constexpr (UNEVEN) {  // point z of rows y and y + 4; what is not the tile's reads as 0
+    const int y = threadIdx.x >> 3, z = threadIdx.x & 7;
+    const long long i0 = ((long long)box.ox * g.ny + box.oy + y) * g.nz + box.oz + z;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int x = 0; x < TE; ++x)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const long long idx = i0 + x * xs + 4 * h * g.nz;
+          const bool live = box.has(x, y + 4 * h, z) && FCM_INB(idx, G, BS_GRID);
+          cp_async8_or_zero(sg + (c * TE + x) * SGX64 + (y + 4 * h) * TE + z, grid + (live ? c * G + idx : 0), live);
+        }
+    return;
+  }
+  const int y = threadIdx.x >> 2, part = threadIdx.x & 3;  // row y of every (component, x), a quarter of its 64 bytes
+  const long long i0 = ((long long)box.ox * g.ny + box.oy + y) * g.nz + box.oz + 2 * part;
   double* d0 = sg + y * TE + 2 * part;
 #pragma unroll
   for (int c = 0; c < 3; ++c)
@@ -1679,6 +1788,7 @@ __device__ __forceinline__ void grid_tile_async64(const double* __restrict__ gri
     }
 }
 
+template <bool UNEVEN>
 __global__ void __launch_bounds__(32) k_interp_mma64(const double* __restrict__ wc, const double* __restrict__ grid,
                                                      TileGeom g, const int* __restrict__ offset,
                                                      const unsigned long long* __restrict__ list, long long G,
@@ -1707,7 +1817,7 @@ __global__ void __launch_bounds__(32) k_interp_mma64(const double* __restrict__ 
       if (tq == 3) sent[b][k] = e[i];
     }
   };
-  grid_tile_async64(grid, g, G, cur.tile, sg);
+  grid_tile_async64<UNEVEN>(grid, g, G, cur.tile, sg);
   entries(cur, e1);
   stage(0, cur, e1);
   cp_async_commit();
@@ -1719,19 +1829,19 @@ __global__ void __launch_bounds__(32) k_interp_mma64(const double* __restrict__ 
     cp_async_wait_all();
     __syncwarp();
     if (first) {
-      const int ty = (cur.tile / g.ntz) % g.nty;
+      const int oy = TileBox<UNEVEN>(g, cur.tile).oy;
 #pragma unroll
       for (int j = 0; j < 2 * TE; ++j)
 #pragma unroll
         for (int c = 0; c < 3; ++c) u[j][c] = sg[(c * TE + gq) * SGX64 + 4 * j + tq];
-      if (ty * TE + TE > g.ycut) {  // rows at or above the slip channel's upper wall read as 0
+      if (oy + TE > g.ycut) {  // rows at or above the slip channel's upper wall read as 0
 #pragma unroll
         for (int j = 0; j < 2 * TE; ++j)
-          if (ty * TE + (j >> 1) >= g.ycut) u[j][0] = u[j][1] = u[j][2] = 0.0;
+          if (oy + (j >> 1) >= g.ycut) u[j][0] = u[j][1] = u[j][2] = 0.0;
       }
       __syncwarp();  // every lane has its fragments: the buffer takes the next tile
       const int nt = cur.tile + (int)gridDim.x;
-      if (nt < ntiles) grid_tile_async64(grid, g, G, nt, sg);
+      if (nt < ntiles) grid_tile_async64<UNEVEN>(grid, g, G, nt, sg);
     }
     bool v2 = false;
     TileItem nx2{0, 0, 0, 0};
@@ -1990,7 +2100,9 @@ __global__ void __launch_bounds__(NT) k_interp_block(const int* __restrict__ bas
 }  // namespace
 
 TileGeom tile_geom(const GridDims& g, int W, int nblobs, long long list_cap) {
-  return TileGeom{g.nx / TE, g.ny / TE, g.nz / TE, g.nx, g.ny, g.nz, W, g.ny, nblobs, list_cap};
+  const int tx = (g.nx + TE - 1) / TE, ty = (g.ny + TE - 1) / TE, tz = (g.nz + TE - 1) / TE;
+  return TileGeom{tx,     ty,       tz,           g.nx,           g.ny,           g.nz, W, g.ny,
+                  nblobs, list_cap, g.nx - 7 * tx, g.ny - 7 * ty, g.nz - 7 * tz};
 }
 
 // CTAs of a persistent kernel: as many as fit on the device at once
@@ -2014,7 +2126,7 @@ int persistent_ctas(K kernel, int threads, int device) {
   return n;
 }
 
-// CTAs of k_tile_count and k_tile_fill: 64 candidate tiles per blob, 128 threads.
+// CTAs of k_tile_count and k_tile_fill (64 candidate tiles per blob, 128 threads).
 static unsigned tile_bin_ctas(int n) { return (unsigned)(((long long)n + 1) / 2); }
 
 template <typename T>
@@ -2026,18 +2138,22 @@ int blob_table_alloc(BlobTable<T>& t, int n, int W, const GridDims& g) {
   FCM_CUDA(cudaMalloc(&t.base, sizeof(int) * 3 * (size_t)(n > 0 ? n : 1)));
   FCM_CUDA(cudaMalloc(&t.w, sizeof(T) * 3 * (size_t)W * (n > 0 ? n : 1)));
   FCM_CUDA(cudaMalloc(&t.ypos, sizeof(double) * 3 * (size_t)(n > 0 ? n : 1)));
-  const bool ok = g.nx % TE == 0 && g.ny % TE == 0 && g.nz % TE == 0 && W + TE <= g.nx && W + TE <= g.ny &&
-                  W + TE <= g.nz && W <= MAXW && n < (1 << 30);
-  if (ok) {
-    t.tiled = true;
-    t.ntx = g.nx / TE;
-    t.nty = g.ny / TE;
-    t.ntz = g.nz / TE;
+  const bool fits = W + TE <= g.nx && W + TE <= g.ny && W + TE <= g.nz && W <= MAXW && n < (1 << 30);
+  const TileGeom tg = tile_geom(g, W, n, 0);
+  t.tiled = fits && g.nx % TE == 0 && g.ny % TE == 0 && g.nz % TE == 0;
+  t.uneven = fits && !t.tiled && W <= MAXW_UNEVEN && tg.qx >= 0 && tg.qy >= 0 && tg.qz >= 0;
+  if (t.binned()) {
+    t.ntx = tg.ntx;
+    t.nty = tg.nty;
+    t.ntz = tg.ntz;
     t.ntiles = t.ntx * t.nty * t.ntz;
-    const long long per = (long long)((W + TE - 2) / TE + 1);
+    const int te = t.tiled ? TE : TE - 1;  // the smallest tile
+    const long long per = (long long)((W + te - 2) / te + 1);
     t.tile_cap = (long long)(n > 0 ? n : 1) * per * per * per;
     FCM_CUDA(cudaMalloc(&t.wc, sizeof(T) * 3 * NCH * TE * (size_t)(n > 0 ? n : 1)));
     FCM_CUDA(cudaMalloc(&t.tile_count, sizeof(int) * (size_t)t.ntiles));
+    FCM_CUDA(cudaMemset(t.tile_count, 0, sizeof(int) * (size_t)t.ntiles));
+    FCM_CUDA(cudaStreamSynchronize(nullptr));
     FCM_CUDA(cudaMalloc(&t.tile_offset, sizeof(int) * ((size_t)t.ntiles + 1)));
     FCM_CUDA(cudaMalloc(&t.tile_list, sizeof(unsigned long long) * (size_t)t.tile_cap));
     FCM_CUDA(cudaMalloc(&t.partial, sizeof(T) * 64 * 3 * (size_t)(n > 0 ? n : 1)));
@@ -2068,16 +2184,17 @@ int launch_set_up_gaussians(const Ctx& c, BlobTable<T>& t, const double* dY, cud
   const double a = c.p.blob_radius;
   const double anorm = 1.0 / (sqrt(2.0) * a);
   const double anorm2 = 2.0 * a * a / PI;
-  const int nt = 3 * t.n;
-  if (t.tiled) FCM_CUDA(cudaMemsetAsync(t.tile_count, 0, sizeof(int) * (size_t)t.ntiles, s));
-  FCM_TRY(launch_chained(k_set_up_gaussians_warp<T>, dim3((unsigned)((32LL * nt + 127) / 128)), dim3(128), 0, s, dY,
-                         t.n, t.W, c.g.dx, anorm, anorm2, t.base, t.w, t.tiled ? t.wc : nullptr, t.ypos));
-  if (t.tiled) {
-    const TileGeom g = tile_geom(c.g, t);
-    FCM_TRY(launch_chained(k_tile_count, dim3(tile_bin_ctas(t.n)), dim3(128), 0, s, t.base, t.n, g, t.tile_count));
+  const TileGeom g = tile_geom(c.g, t);
+  // the fill leaves the counts at zero; a set-up that failed half-way does not
+  if (t.binned() && t.counts_dirty) FCM_CUDA(cudaMemsetAsync(t.tile_count, 0, sizeof(int) * (size_t)t.ntiles, s));
+  t.counts_dirty = true;
+  FCM_TRY(launch_chained(k_set_up_gaussians_warp<T>, dim3((unsigned)((t.n + 1) / 2)), dim3(192), 0, s, dY, t.n, t.W,
+                         c.g.dx, anorm, anorm2, t.base, t.w, t.binned() ? t.wc : nullptr, t.ypos, g, t.tile_count));
+  if (t.binned()) {
     FCM_TRY(launch_exclusive_scan(t.tile_count, t.tile_offset, t.ntiles, s));
     FCM_TRY(launch_chained(k_tile_fill, dim3(tile_bin_ctas(t.n)), dim3(128), 0, s, t.base, t.n, g, t.tile_offset,
                            t.tile_count, t.tile_list));
+    t.counts_dirty = false;
     FCM_TRY(launch_chained(k_tile_sort_warp, dim3((t.ntiles + 3) / 4), dim3(128), 0, s, t.tile_offset, t.ntiles,
                            t.tile_list, t.tile_cap));
   }
@@ -2094,8 +2211,8 @@ int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid
     const TileGeom tg = tile_geom(c.g, t);
     if (v == 0) {
       if constexpr (sizeof(T) == 8) {
-        const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_mma64, 32, c.device));
-        return launch_chained(k_spread_mma64, dim3(ctas), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
+        const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_mma64<false>, 32, c.device));
+        return launch_chained(k_spread_mma64<false>, dim3(ctas), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
                               c.g.G,
                               grid, t.ntiles);
       } else {
@@ -2107,7 +2224,7 @@ int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid
     } else if (v == 3) {
       k_spread_tiled<T, 32><<<t.ntiles, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid);
     } else if (v == 4) {
-      return launch_chained(k_spread_warp<T>, dim3(t.ntiles), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
+      return launch_chained(k_spread_warp<T, false>, dim3(t.ntiles), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
                             c.g.G, grid);
     } else if (v == 5 && sizeof(T) == 4) {
       if constexpr (sizeof(T) == 4)
@@ -2118,6 +2235,17 @@ int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid
     }
     FCM_LAUNCH_CHECK();
     return FCM_OK;
+  }
+  if (t.uneven) {  // the default kernels whatever the variants, which are those of whole tiles
+    const TileGeom tg = tile_geom(c.g, t);
+    if constexpr (sizeof(T) == 8) {
+      const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_mma64<true>, 32, c.device));
+      return launch_chained(k_spread_mma64<true>, dim3(ctas), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
+                            c.g.G, grid, t.ntiles);
+    } else {
+      return launch_chained(k_spread_warp<T, true>, dim3(t.ntiles), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset,
+                            t.tile_list, c.g.G, grid);
+    }
   }
   FCM_CUDA(cudaMemsetAsync(grid, 0, sizeof(T) * 3 * (size_t)c.g.G, s));
   if (t.n == 0) return FCM_OK;
@@ -2131,6 +2259,15 @@ template <typename T>
 static int launch_interp_tiles(const Ctx& c, const BlobTable<T>& t, const T* grid, TileGeom& g, cudaStream_t s) {
   g = tile_geom(c.g, t);
   g.ycut = c.p.slip_channel ? c.g.ny / 2 : c.g.ny;  // fcm_fluid_solver.cpp:387-389
+  if (t.uneven) {
+    if constexpr (sizeof(T) == 8)
+      return launch_chained(k_interp_mma64<true>,
+                            dim3(std::min(t.ntiles, persistent_ctas(k_interp_mma64<true>, 32, c.device))), dim3(32), 0,
+                            s, t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles);
+    else
+      return launch_chained(k_interp_warp<T, true>, dim3(t.ntiles), dim3(32), 0, s, t.wc, grid, g, t.tile_offset,
+                            t.tile_list, c.g.G, t.partial);
+  }
   const int v = c.interp_variant[sizeof(T) == 8 ? 0 : 1];
   // the tensor-core kernels copy 16-byte parts of the grid's rows (every caller's grid is
   // an allocation of its own, so aligned; otherwise the 64-thread kernel)
@@ -2142,7 +2279,7 @@ static int launch_interp_tiles(const Ctx& c, const BlobTable<T>& t, const T* gri
   }
   if constexpr (sizeof(T) == 8) {
     if (v == 1 && aligned) {
-      FCM_TRY(launch_chained(k_interp_mma64, dim3(std::min(t.ntiles, persistent_ctas(k_interp_mma64, 32, c.device))),
+      FCM_TRY(launch_chained(k_interp_mma64<false>, dim3(std::min(t.ntiles, persistent_ctas(k_interp_mma64<false>, 32, c.device))),
                              dim3(32), 0, s, t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial, t.ntiles));
       return FCM_OK;
     }
@@ -2153,7 +2290,7 @@ static int launch_interp_tiles(const Ctx& c, const BlobTable<T>& t, const T* gri
       return FCM_OK;
     }
     if (v == 1) {
-      FCM_TRY(launch_chained(k_interp_warp<T>, dim3(t.ntiles), dim3(32), 0, s, t.wc, grid, g, t.tile_offset,
+      FCM_TRY(launch_chained(k_interp_warp<T, false>, dim3(t.ntiles), dim3(32), 0, s, t.wc, grid, g, t.tile_offset,
                              t.tile_list, c.g.G, t.partial));
       return FCM_OK;
     }
@@ -2167,7 +2304,11 @@ template <typename T>
 int launch_interp(const Ctx& c, const BlobTable<T>& t, const T* grid, double* dV, cudaStream_t s) {
   if (t.n == 0) return FCM_OK;
   const double dx3 = c.g.dx * c.g.dx * c.g.dx;
-  if (t.tiled) {
+  // few blobs in FP32 on an uneven grid: a CTA per blob, at two per SM still faster than
+  // the tiles' longest list (60 blobs 6.2 against 8.4 us, 240 in a 42^3 grid 6.4 against
+  // 12.3, 360 level, 1500 level, 4200 22.8 against 17.8)
+  const bool few = sizeof(T) == 4 && t.uneven && t.n <= 300;
+  if (t.binned() && !few) {
     TileGeom g;
     FCM_TRY(launch_interp_tiles<T>(c, t, grid, g, s));
     FCM_TRY(launch_chained(k_interp_reduce8<T>, dim3((t.n + 15) / 16), dim3(128), 0, s, t.base, t.partial, t.n, g, dx3,
@@ -2183,7 +2324,7 @@ int launch_interp(const Ctx& c, const BlobTable<T>& t, const T* grid, double* dV
 template <typename T>
 int launch_saddle_end(const Ctx& c, const BlobTable<T>& t, const T* grid, const double* qm, const double* in,
                       double* out, cudaStream_t s) {
-  if (t.n == 0 || !t.tiled) {
+  if (t.n == 0 || !t.binned()) {
     FCM_TRY(launch_interp<T>(c, t, grid, out, s));
     FCM_TRY(launch_multiply_K(c, qm, in + 3 * (size_t)c.Nb, out, 1.0, s));
     return launch_multiply_KT(c, qm, in, out + 3 * (size_t)c.Nb, -1.0, nullptr, 0.0, s);
@@ -2749,7 +2890,7 @@ extern "C" int fcm_interp_noalloc(int32_t nx, int32_t ny, int32_t nz, double dx,
   const double PI = 3.14159265358979323846264338327950288;
   const double anorm = 1.0 / (sqrt(2.0) * blob_radius);
   const double anorm2 = 2.0 * blob_radius * blob_radius / PI;
-  const TileGeom g{nx / TE, ny / TE, nz / TE, nx, ny, nz, W, ny, n, (long long)cap};
+  const TileGeom g{nx / TE, ny / TE, nz / TE, nx, ny, nz, W, ny, n, (long long)cap, nx / TE, ny / TE, nz / TE};
   const long long G = (long long)nx * ny * nz;
   // the array keeps the previous call's contents: counters start at zero
   FCM_CUDA(cudaMemsetAsync(s_count, 0, sizeof(int) * (size_t)ntiles, s));

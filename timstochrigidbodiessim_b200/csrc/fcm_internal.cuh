@@ -196,9 +196,13 @@ struct BlobTable {
   // Usable when every grid dimension is a multiple of the tile edge and
   // W + tile edge <= n (a stencil never meets the same tile twice).
   bool tiled = false;
+  // The same binning on grids with other dimensions, by uneven tiles of 8 and 7 points.
+  bool uneven = false;
+  bool binned() const { return tiled || uneven; }
   int ntx = 0, nty = 0, ntz = 0, ntiles = 0;
   T* wc = nullptr;                // [n][3][4][8] weights on the 8-aligned grid chunks a stencil meets
-  int* tile_count = nullptr;      // [ntiles]
+  int* tile_count = nullptr;      // [ntiles], zero between set-ups
+  bool counts_dirty = false;      // a set-up ended before its fill
   int* tile_offset = nullptr;     // [ntiles+1] exclusive offsets
   unsigned long long* tile_list = nullptr;  // [cap] (blob << 32) | chunk indices, j and half masks
   long long tile_cap = 0;
@@ -234,6 +238,7 @@ struct TileGeom {
   int ycut;            // interpolation reads rows y < ycut only (ny, or ny/2 in a slip channel)
   int nblobs;          // blobs of the tables
   long long list_cap;  // capacity of the tile list (entries)
+  int qx, qy, qz;      // tiles of 8 points per direction (the first ones); the others have 7
 };
 
 // k-space geometry of the projection (fcm_kspace.cu).
