@@ -501,8 +501,7 @@ int set_stream_all(Ctx* c) {
 // ------------------------------------------------------------------ FCM pieces
 // Gaussian tables of all blobs from Y (device), FP64 always, FP32 for precision 1.
 int set_up_gaussians_dev(Ctx* c, const double* dY) {
-  FCM_TRY(launch_set_up_gaussians<double>(*c, c->g64.blobs, dY, c->stream));
-  if (c->p.precision == 1) FCM_TRY(launch_set_up_gaussians<float>(*c, c->g32.blobs, dY, c->stream));
+  FCM_TRY(launch_set_up_gaussians(*c, c->g64.blobs, c->p.precision == 1 ? &c->g32.blobs : nullptr, dY, c->stream));
   c->gauss_ready = true;
   return FCM_OK;
 }
@@ -1190,7 +1189,7 @@ int reference_matrices_dev(Ctx* c) {
   std::vector<double> Mb((size_t)n3 * n3);
   do {
     if ((st = copy_in(c, dY, Y.data(), sizeof(double) * 3 * nb)) != FCM_OK) break;
-    if ((st = launch_set_up_gaussians<double>(*c, c->g64.ref_blobs, dY, c->stream)) != FCM_OK) break;
+    if ((st = launch_set_up_gaussians(*c, c->g64.ref_blobs, nullptr, dY, c->stream)) != FCM_OK) break;
     std::vector<double> e(n3, 0.0);
     for (int n = 0; n < n3 && st == FCM_OK; ++n) {
       std::fill(e.begin(), e.end(), 0.0);

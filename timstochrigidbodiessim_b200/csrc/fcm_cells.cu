@@ -180,8 +180,14 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_chunks(const int* __restrict__ 
 // 32,768 tile counts of a 256^3 grid take 6 us; chunks of 8192 by four CTAs took 9.8, one
 // CTA 11.7 us for 12,831 entries.
 constexpr int SCAN_DIRECT = 64 * 1024;
-__global__ void __launch_bounds__(SCAN_T) k_scan_direct(const int* __restrict__ in, int* __restrict__ out, int n) {
+// blockIdx.y = 1 scans a second input of the same length.
+__global__ void __launch_bounds__(SCAN_T) k_scan_direct(const int* __restrict__ in, int* __restrict__ out, int n,
+                                                        const int* __restrict__ in2, int* __restrict__ out2) {
   chain_begin();
+  if (blockIdx.y) {
+    in = in2;
+    out = out2;
+  }
   __shared__ int warp_sums[32];
   const int c0 = blockIdx.x * SCAN_T, i = c0 + threadIdx.x;
   const int4* in4 = reinterpret_cast<const int4*>(in);
@@ -471,10 +477,12 @@ PairArgs pair_args(const Ctx& c) {
 
 }  // namespace
 
-int launch_exclusive_scan(const int* in, int* out, int n, cudaStream_t s) {
-  const bool aligned = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
+int launch_exclusive_scan(const int* in, int* out, int n, cudaStream_t s, const int* in2, int* out2) {
+  const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(in2)) & 15u) == 0;
   if (n <= SCAN_DIRECT && aligned)
-    return launch_chained(k_scan_direct, dim3(std::max(1, (n + SCAN_T - 1) / SCAN_T)), dim3(SCAN_T), 0, s, in, out, n);
+    return launch_chained(k_scan_direct, dim3(std::max(1, (n + SCAN_T - 1) / SCAN_T), in2 ? 2 : 1), dim3(SCAN_T), 0, s,
+                          in, out, n, in2, out2);
+  if (in2) FCM_TRY(launch_exclusive_scan(in2, out2, n, s, nullptr, nullptr));
   const int nchunks = (n + SCAN_CH - 1) / SCAN_CH;
   k_scan_chunk_sums<<<nchunks, SCAN_T, 0, s>>>(in, out, n);
   FCM_LAUNCH_CHECK();

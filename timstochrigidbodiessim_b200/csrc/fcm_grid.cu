@@ -192,13 +192,21 @@ __global__ void __launch_bounds__(128) k_tile_count(const int* __restrict__ base
 // 64 threads per blob count its overlaps (a launch of its own took 8 us for 12,288 blobs).
 // Without wc the lanes write w[i], i = lane, lane + 32, ...
 template <typename T>
-__global__ void __launch_bounds__(192) k_set_up_gaussians_warp(const double* __restrict__ Y, int n, int W, double dx,
-                                                               double anorm, double anorm2, int* __restrict__ base,
-                                                               T* __restrict__ w, T* __restrict__ wc,
-                                                               double* __restrict__ ypos, TileGeom tg,
-                                                               int* __restrict__ count) {
-  chain_begin();
-  __shared__ int sb[6];
+struct GaussTable {
+  int* base;
+  T *w, *wc;
+  double* ypos;
+  TileGeom g;
+  int* count;
+};
+template <typename T>
+__device__ __forceinline__ void set_up_gaussians_cta(const double* __restrict__ Y, int n, double dx, double anorm,
+                                                     double anorm2, const GaussTable<T>& tab, int* sb) {
+  const TileGeom& tg = tab.g;
+  const int W = tg.W;
+  int* __restrict__ base = tab.base;
+  T* __restrict__ w = tab.w;
+  T* __restrict__ wc = tab.wc;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long t = 6LL * blockIdx.x + wid;
   if (t < 3LL * n) {  // uniform over the warp
@@ -207,14 +215,14 @@ __global__ void __launch_bounds__(192) k_set_up_gaussians_warp(const double* __r
     const int b = xc - W / 2 + 1;
     if (lane == 0) {
       base[t] = sb[wid] = b;
-      if (ypos) ypos[t] = y;
+      if (tab.ypos) tab.ypos[t] = y;
     }
     if (!wc) {
       for (int i = lane; i < W; i += 32) {
         const double xx = __dsub_rn(__dmul_rn((double)(b + i), dx), y);
         w[t * W + i] = (T)(anorm * exp(__ddiv_rn(-__dmul_rn(xx, xx), anorm2)));
       }
-      return;  // every warp of every CTA: wc is the launch's
+      return;  // every warp of the CTA: wc is the table's
     }
     const int d = wid % 3;
     const int dn = d == 0 ? tg.nx : d == 1 ? tg.ny : tg.nz, dt = d == 0 ? tg.ntx : d == 1 ? tg.nty : tg.ntz;
@@ -242,17 +250,45 @@ __global__ void __launch_bounds__(192) k_set_up_gaussians_warp(const double* __r
     int f[3], cnt[3];
     blob_tiles(sb, k, tg, f, cnt);
     const int tile = candidate_tile(tg, f, cnt, threadIdx.x & 63);
-    if (tile >= 0) atomicAdd(count + tile, 1);
+    if (tile >= 0) atomicAdd(tab.count + tile, 1);
   }
 }
+
+// The FP64 tables and, in blockIdx.y = 1, the FP32 ones of the same positions.  The kernels
+// of a small set-up are bound by their launches and loads in turn, so both precisions share
+// them here and below: set-up of a mixed context, 192 blobs at 64^3, 13 us (23.5 one after
+// the other), 12,288 blobs at 256^3 56 us (63).
+__global__ void __launch_bounds__(192) k_set_up_gaussians_both(const double* __restrict__ Y, int n, double dx,
+                                                               double anorm, double anorm2, GaussTable<double> a,
+                                                               GaussTable<float> b) {
+  chain_begin();
+  __shared__ int sb[6];
+  if (blockIdx.y == 0)
+    set_up_gaussians_cta<double>(Y, n, dx, anorm, anorm2, a, sb);
+  else
+    set_up_gaussians_cta<float>(Y, n, dx, anorm, anorm2, b, sb);
+}
+
+// Tile lists of one or two tables, by blockIdx.y.
+struct BinTables {
+  const int* base[2];
+  TileGeom g[2];
+  int* count[2];
+  int* offset[2];
+  unsigned long long* list[2];
+};
 
 // The list entries, one thread per (blob, candidate): each takes the last free slot of its
 // tile by counting the tile's overlaps down again, so the counts end as zeros (the order
 // within a tile is restored by the sort).
-__global__ void __launch_bounds__(128) k_tile_fill(const int* __restrict__ base, int n, TileGeom g,
-                                                   const int* __restrict__ offset, int* __restrict__ count,
-                                                   unsigned long long* __restrict__ list) {
+__global__ void __launch_bounds__(128) k_tile_fill(BinTables bt, int n) {
   chain_begin();
+  const bool second = blockIdx.y != 0;
+  const TileGeom& g = second ? bt.g[1] : bt.g[0];
+  const int* __restrict__ base = second ? bt.base[1] : bt.base[0];
+  const int* __restrict__ offset = second ? bt.offset[1] : bt.offset[0];
+  int* __restrict__ count = second ? bt.count[1] : bt.count[0];
+  unsigned long long* __restrict__ list = second ? bt.list[1] : bt.list[0];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int b = (int)(t >> 6), s = (int)(t & 63);
   if (b >= n) return;
@@ -323,9 +359,12 @@ __device__ __forceinline__ void sort_by_rank(unsigned long long* __restrict__ li
 // 128 threads = four tiles per CTA; tiles with more than TSORT entries are sorted by lane 0
 // in place as k_tile_sort does.
 constexpr int TSORT = 256;
-__global__ void __launch_bounds__(128) k_tile_sort_warp(const int* __restrict__ offset, int ntiles,
-                                                        unsigned long long* __restrict__ list, long long cap) {
+__global__ void __launch_bounds__(128) k_tile_sort_warp(BinTables bt, int ntiles) {
   chain_begin();
+  const bool second = blockIdx.y != 0;
+  const int* __restrict__ offset = second ? bt.offset[1] : bt.offset[0];
+  unsigned long long* __restrict__ list = second ? bt.list[1] : bt.list[0];
+  const long long cap = second ? bt.g[1].list_cap : bt.g[0].list_cap;
   __shared__ __align__(16) unsigned keys[4][TSORT];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + w;
@@ -573,6 +612,7 @@ __global__ void __launch_bounds__(64) k_spread_tiled(const T* __restrict__ wc, c
                                                      TileGeom g, const int* __restrict__ offset,
                                                      const unsigned long long* __restrict__ list, long long G,
                                                      T* __restrict__ grid) {
+  chain_begin();
   spread_tile<T, NB>(wc, F, g, offset, list, G, grid, blockIdx.x);
 }
 
@@ -759,6 +799,7 @@ __global__ void __launch_bounds__(64) k_spread_pipe(const T* __restrict__ wc, co
                                                     const int* __restrict__ offset,
                                                     const unsigned long long* __restrict__ list, long long G,
                                                     T* __restrict__ grid, int ntiles) {
+  chain_begin();
   __shared__ __align__(16) T sw[2][SCB][3][TE];
   __shared__ __align__(16) T sF[2][SCB][4];
   __shared__ unsigned sflag[2][SCB];
@@ -1028,6 +1069,7 @@ __global__ void __launch_bounds__(64) k_interp_tiled(const T* __restrict__ wc, c
                                                      TileGeom g, const int* __restrict__ offset,
                                                      const unsigned long long* __restrict__ list, long long G,
                                                      T* __restrict__ partial) {
+  chain_begin();
   interp_tile<T>(wc, grid, g, offset, list, G, partial, blockIdx.x);
 }
 
@@ -1049,6 +1091,7 @@ __global__ void __launch_bounds__(64 / R) k_interp_rows(const T* __restrict__ wc
                                                         TileGeom g, const int* __restrict__ offset,
                                                         const unsigned long long* __restrict__ list, long long G,
                                                         T* __restrict__ partial) {
+  chain_begin();
   constexpr int NT = 64 / R;                    // threads per tile
   constexpr int RS = NT + 16 / (int)sizeof(T);  // padded reduction row
   constexpr int YS = TE / R;                    // row step between a thread's rows
@@ -2178,27 +2221,44 @@ void blob_table_free(BlobTable<T>& t) {
 }
 
 template <typename T>
-int launch_set_up_gaussians(const Ctx& c, BlobTable<T>& t, const double* dY, cudaStream_t s) {
-  if (t.n == 0) return FCM_OK;
+static GaussTable<T> gauss_table(const Ctx& c, const BlobTable<T>& t) {
+  return GaussTable<T>{t.base, t.w, t.binned() ? t.wc : nullptr, t.ypos, tile_geom(c.g, t), t.tile_count};
+}
+
+int launch_set_up_gaussians(const Ctx& c, BlobTable<double>& t64, BlobTable<float>* t32, const double* dY,
+                            cudaStream_t s) {
+  const int n = t64.n;
+  if (n == 0) return FCM_OK;
   const double PI = 3.14159265358979323846264338327950288;
   const double a = c.p.blob_radius;
   const double anorm = 1.0 / (sqrt(2.0) * a);
   const double anorm2 = 2.0 * a * a / PI;
-  const TileGeom g = tile_geom(c.g, t);
-  // the fill leaves the counts at zero; a set-up that failed half-way does not
-  if (t.binned() && t.counts_dirty) FCM_CUDA(cudaMemsetAsync(t.tile_count, 0, sizeof(int) * (size_t)t.ntiles, s));
-  t.counts_dirty = true;
-  FCM_TRY(launch_chained(k_set_up_gaussians_warp<T>, dim3((unsigned)((t.n + 1) / 2)), dim3(192), 0, s, dY, t.n, t.W,
-                         c.g.dx, anorm, anorm2, t.base, t.w, t.binned() ? t.wc : nullptr, t.ypos, g, t.tile_count));
-  if (t.binned()) {
-    FCM_TRY(launch_exclusive_scan(t.tile_count, t.tile_offset, t.ntiles, s));
-    FCM_TRY(launch_chained(k_tile_fill, dim3(tile_bin_ctas(t.n)), dim3(128), 0, s, t.base, t.n, g, t.tile_offset,
-                           t.tile_count, t.tile_list));
-    t.counts_dirty = false;
-    FCM_TRY(launch_chained(k_tile_sort_warp, dim3((t.ntiles + 3) / 4), dim3(128), 0, s, t.tile_offset, t.ntiles,
-                           t.tile_list, t.tile_cap));
-  }
-  return FCM_OK;
+  BinTables bt{};
+  int nbin = 0, ntiles = 0;
+  auto add = [&](auto& t) -> int {
+    if (!t.binned()) return FCM_OK;
+    // the fill leaves the counts at zero; a set-up that failed half-way does not
+    if (t.counts_dirty) FCM_CUDA(cudaMemsetAsync(t.tile_count, 0, sizeof(int) * (size_t)t.ntiles, s));
+    t.counts_dirty = true;
+    bt.base[nbin] = t.base;
+    bt.g[nbin] = tile_geom(c.g, t);
+    bt.count[nbin] = t.tile_count;
+    bt.offset[nbin] = t.tile_offset;
+    bt.list[nbin] = t.tile_list;
+    ntiles = t.ntiles;  // the grid's, in either precision
+    ++nbin;
+    return FCM_OK;
+  };
+  FCM_TRY(add(t64));
+  if (t32) FCM_TRY(add(*t32));
+  FCM_TRY(launch_chained(k_set_up_gaussians_both, dim3((unsigned)((n + 1) / 2), t32 ? 2 : 1), dim3(192), 0, s, dY, n,
+                         c.g.dx, anorm, anorm2, gauss_table(c, t64), t32 ? gauss_table(c, *t32) : GaussTable<float>{}));
+  if (nbin == 0) return FCM_OK;
+  FCM_TRY(launch_exclusive_scan(bt.count[0], bt.offset[0], ntiles, s, bt.count[1], bt.offset[1]));
+  FCM_TRY(launch_chained(k_tile_fill, dim3(tile_bin_ctas(n), nbin), dim3(128), 0, s, bt, n));
+  t64.counts_dirty = false;
+  if (t32) t32->counts_dirty = false;
+  return launch_chained(k_tile_sort_warp, dim3((ntiles + 3) / 4, nbin), dim3(128), 0, s, bt, ntiles);
 }
 
 template <typename T>
@@ -2212,17 +2272,19 @@ int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid
     if (v == 0) {
       if constexpr (sizeof(T) == 8) {
         const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_mma64<false>, 32, c.device));
-        return launch_chained(k_spread_mma64<false>, dim3(ctas), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
-                              c.g.G,
-                              grid, t.ntiles);
+        return launch_chained(k_spread_mma64<false>, dim3(ctas), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset,
+                              t.tile_list, c.g.G, grid, t.ntiles);
       } else {
         const int ctas = std::min(t.ntiles, persistent_ctas(k_spread_pipe<T>, 64, c.device));
-        k_spread_pipe<T><<<ctas, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid, t.ntiles);
+        return launch_chained(k_spread_pipe<T>, dim3(ctas), dim3(64), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
+                              c.g.G, grid, t.ntiles);
       }
     } else if (v == 2) {
-      k_spread_tiled<T, 8><<<t.ntiles, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid);
+      return launch_chained(k_spread_tiled<T, 8>, dim3(t.ntiles), dim3(64), 0, s, t.wc, dF, tg, t.tile_offset,
+                            t.tile_list, c.g.G, grid);
     } else if (v == 3) {
-      k_spread_tiled<T, 32><<<t.ntiles, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid);
+      return launch_chained(k_spread_tiled<T, 32>, dim3(t.ntiles), dim3(64), 0, s, t.wc, dF, tg, t.tile_offset,
+                            t.tile_list, c.g.G, grid);
     } else if (v == 4) {
       return launch_chained(k_spread_warp<T, false>, dim3(t.ntiles), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
                             c.g.G, grid);
@@ -2230,11 +2292,9 @@ int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid
       if constexpr (sizeof(T) == 4)
         return launch_chained(k_spread_mma, dim3(t.ntiles), dim3(32), 0, s, t.wc, dF, tg, t.tile_offset, t.tile_list,
                               c.g.G, grid);
-    } else {
-      k_spread_tiled<T, 16><<<t.ntiles, 64, 0, s>>>(t.wc, dF, tg, t.tile_offset, t.tile_list, c.g.G, grid);
     }
-    FCM_LAUNCH_CHECK();
-    return FCM_OK;
+    return launch_chained(k_spread_tiled<T, 16>, dim3(t.ntiles), dim3(64), 0, s, t.wc, dF, tg, t.tile_offset,
+                          t.tile_list, c.g.G, grid);
   }
   if (t.uneven) {  // the default kernels whatever the variants, which are those of whole tiles
     const TileGeom tg = tile_geom(c.g, t);
@@ -2273,9 +2333,8 @@ static int launch_interp_tiles(const Ctx& c, const BlobTable<T>& t, const T* gri
   // an allocation of its own, so aligned; otherwise the 64-thread kernel)
   const bool aligned = (reinterpret_cast<uintptr_t>(grid) & 15u) == 0;
   if (v == 2) {
-    k_interp_rows<T, 2><<<t.ntiles, 32, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
-    FCM_LAUNCH_CHECK();
-    return FCM_OK;
+    return launch_chained(k_interp_rows<T, 2>, dim3(t.ntiles), dim3(32), 0, s, t.wc, grid, g, t.tile_offset, t.tile_list,
+                          c.g.G, t.partial);
   }
   if constexpr (sizeof(T) == 8) {
     if (v == 1 && aligned) {
@@ -2295,9 +2354,8 @@ static int launch_interp_tiles(const Ctx& c, const BlobTable<T>& t, const T* gri
       return FCM_OK;
     }
   }
-  k_interp_tiled<T><<<t.ntiles, 64, 0, s>>>(t.wc, grid, g, t.tile_offset, t.tile_list, c.g.G, t.partial);
-  FCM_LAUNCH_CHECK();
-  return FCM_OK;
+  return launch_chained(k_interp_tiled<T>, dim3(t.ntiles), dim3(64), 0, s, t.wc, grid, g, t.tile_offset, t.tile_list,
+                        c.g.G, t.partial);
 }
 
 template <typename T>
@@ -2373,8 +2431,6 @@ template int blob_table_alloc<double>(BlobTable<double>&, int, int, const GridDi
 template int blob_table_alloc<float>(BlobTable<float>&, int, int, const GridDims&);
 template void blob_table_free<double>(BlobTable<double>&);
 template void blob_table_free<float>(BlobTable<float>&);
-template int launch_set_up_gaussians<double>(const Ctx&, BlobTable<double>&, const double*, cudaStream_t);
-template int launch_set_up_gaussians<float>(const Ctx&, BlobTable<float>&, const double*, cudaStream_t);
 template int launch_spread<double>(const Ctx&, const BlobTable<double>&, const double*, double*, cudaStream_t);
 template int launch_spread<float>(const Ctx&, const BlobTable<float>&, const double*, float*, cudaStream_t);
 template int launch_saddle_end<double>(const Ctx&, const BlobTable<double>&, const double*, const double*,
@@ -2899,8 +2955,8 @@ extern "C" int fcm_interp_noalloc(int32_t nx, int32_t ny, int32_t nz, double dx,
   FCM_LAUNCH_CHECK();
   FCM_TRY(launch_chained(k_tile_count, dim3(tile_bin_ctas(n)), dim3(128), 0, s, s_base, n, g, s_count));
   FCM_TRY(launch_exclusive_scan(s_count, s_offset, (int)ntiles, s));
-  FCM_TRY(launch_chained(k_tile_fill, dim3(tile_bin_ctas(n)), dim3(128), 0, s, s_base, n, g, s_offset, s_count,
-                         s_list));
+  FCM_TRY(launch_chained(k_tile_fill, dim3(tile_bin_ctas(n)), dim3(128), 0, s,
+                         BinTables{{s_base}, {g}, {s_count}, {s_offset}, {s_list}}, n));
   k_tile_sort<<<(unsigned)((ntiles + 127) / 128), 128, 0, s>>>(s_offset, (int)ntiles, s_list, (long long)cap);
   FCM_LAUNCH_CHECK();
   k_interp_tiled<double><<<(unsigned)ntiles, 64, 0, s>>>(s_wc, grid, g, s_offset, s_list, G, s_partial);

@@ -380,14 +380,16 @@ struct Ctx {
   // what the grids allow (fcm_autotune chooses within it): the fused x-transform per
   // precision (its (y, z) plans exist)
   bool xfft_cap[2] = {false, false};
-  // spread kernel per precision: 0 the persistent software-pipelined one (FP64
-  // default), 1 / 2 / 3 one CTA per tile staging 16 / 8 / 32 blobs per round, 4
-  // one warp per tile (FP32 default); all sum every point's blobs in the same order
+  // spread kernel per precision: 0 in FP64 the FP64 tensor-core tile kernel (the
+  // default), in FP32 the persistent software-pipelined one, 1 / 2 / 3 one CTA per tile
+  // staging 16 / 8 / 32 blobs per round, 4 one warp per tile (FP32 default), 5 the FP32
+  // tensor-core kernel; all but 5 sum every point's blobs in the same order
   int spread_variant[2] = {0, 4};
   // interpolation kernel per precision: 0 the 64-thread shuffle-reduced tile
-  // kernel (k_interp_tiled), 1 one warp per tile with two y-rows per lane and the
-  // shuffle reduction (k_interp_warp, the default), 2 the shared-memory reduced
-  // kernel with two y-rows per thread (k_interp_rows, 32 threads per tile)
+  // kernel (k_interp_tiled), 1 (the default) in FP64 the FP64 tensor-core kernel
+  // (k_interp_mma64), in FP32 one warp per tile with two y-rows per lane and the shuffle
+  // reduction (k_interp_warp), 2 the shared-memory reduced kernel with two y-rows per
+  // thread (k_interp_rows, 32 threads per tile), 3 the FP32 tensor-core kernel
   int interp_variant[2] = {1, 1};
   void* d_ytw32 = nullptr;
   void* d_ztw32 = nullptr;
@@ -569,8 +571,8 @@ template <typename T>
 int blob_table_alloc(BlobTable<T>& t, int n, int W, const GridDims& g);
 template <typename T>
 void blob_table_free(BlobTable<T>& t);
-template <typename T>
-int launch_set_up_gaussians(const Ctx& c, BlobTable<T>& t, const double* dY, cudaStream_t s);
+int launch_set_up_gaussians(const Ctx& c, BlobTable<double>& t64, BlobTable<float>* t32, const double* dY,
+                            cudaStream_t s);
 template <typename T>
 int launch_spread(const Ctx& c, const BlobTable<T>& t, const double* dF, T* grid, cudaStream_t s);
 template <typename T>
@@ -648,7 +650,8 @@ int launch_body_update_uniform(const Ctx& c, double* x, double* q, const double*
 int launch_mcmc_propose(const Ctx& c, const McmcDev* st, cudaStream_t s);
 int launch_mcmc_restore(const Ctx& c, const McmcDev* st, cudaStream_t s);
 int launch_divU_accumulate(const Ctx& c, const double* U6, const double* U0, int component, double delta, double* acc, cudaStream_t s);
-int launch_exclusive_scan(const int* in, int* out, int n, cudaStream_t s);
+int launch_exclusive_scan(const int* in, int* out, int n, cudaStream_t s, const int* in2 = nullptr,
+                          int* out2 = nullptr);
 // cells (fcm_cells.cu)
 int cells_build(Ctx& c, cudaStream_t s);
 // with_walls adds a slip channel's wall forces (collection_of_rigid_bodies.cpp:640-662)
