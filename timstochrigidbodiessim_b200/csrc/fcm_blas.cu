@@ -352,6 +352,11 @@ constexpr int AC = 8, AT = 512, AW = AT / 32;
 constexpr long long GM_CLUSTER_MAX_N = 4LL * AC * AT;
 constexpr int GM_CLUSTER_MAX_COLS = 256;
 constexpr size_t gm_cluster_smem(int hn) { return sizeof(double) * ((size_t)(AW + 2 + 1 + 2) * hn + 1 + AW); }
+// With the static arrays (h_all, nred, nsum) the largest launch stays within the 48 KB that
+// every kernel may take: no limit has to be raised, which another thread's smaller context
+// could lower again before the launch.
+static_assert(gm_cluster_smem(GM_CLUSTER_MAX_COLS) + sizeof(double) * (GM_CLUSTER_MAX_COLS + AW + 1) <= 48 * 1024,
+              "k_gm_arnoldi's shared memory fits the default limit");
 
 template <int AE>
 __global__ void __cluster_dims__(AC, 1, 1) __launch_bounds__(AT)
@@ -545,8 +550,6 @@ int gm_arnoldi(const Ctx& c, const double* w, cudaStream_t s, cudaGraphCondition
   const int hn = c.maxit_alloc + 1;
   auto kern = n <= per ? k_gm_arnoldi<1> : n <= 2 * per ? k_gm_arnoldi<2> : k_gm_arnoldi<4>;
   const size_t smem = gm_cluster_smem(hn);
-  if (smem > 40 * 1024)  // not a stream operation: allowed while capturing
-    FCM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   return launch_chained(kern, dim3(AC), dim3(AT), smem, s, c.gm, c.d_Qm, n, w, c.d_Hd, hn, c.d_beta, c.d_CS, c.d_SN,
                         handle, sd, limit);
 }
