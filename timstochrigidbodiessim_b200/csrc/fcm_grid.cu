@@ -278,9 +278,10 @@ struct BinTables {
   unsigned long long* list[2];
 };
 
-// The list entries, one thread per (blob, candidate): each takes the last free slot of its
-// tile by counting the tile's overlaps down again, so the counts end as zeros (the order
-// within a tile is restored by the sort).
+// The list entries, one thread per (blob, candidate): each takes the first free slot of its
+// tile by counting the tile's overlaps down, so the counts end as zeros and the lists nearly
+// in blob order, which the serial sorts need (filled from the last slot down, a list of
+// thousands took them the square of its length).
 __global__ void __launch_bounds__(128) k_tile_fill(BinTables bt, int n) {
   chain_begin();
   const bool second = blockIdx.y != 0;
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(128) k_tile_fill(BinTables bt, int n) {
   blob_tiles(base, b, g, f, cnt);
   const int tile = candidate_tile(g, f, cnt, s);
   if (tile < 0) return;
-  const int slot = offset[tile] + atomicSub(count + tile, 1) - 1;
+  const int slot = offset[tile + 1] - atomicSub(count + tile, 1);
   const int ox = s >> 4, oy = (s >> 2) & 3, oz = s & 3;
   const unsigned j = (unsigned)((ox * cnt[1] + oy) * cnt[2] + oz);
   const unsigned lo = (unsigned)ox | ((unsigned)oy << 2) | ((unsigned)oz << 4) | (j << EJ) |
@@ -326,23 +327,26 @@ __global__ void k_tile_sort(const int* __restrict__ offset, int ntiles, unsigned
   }
 }
 
-// The same order, one warp per tile: E entries per lane, each placed by its rank, the number
-// of smaller blob ids in the tile (read four at a time from shared memory, padded with
-// ids above all others).  No step waits for another, as those of a bitonic sort did: the
-// lists of 2048 rods at 256^3 (15 entries) take 9.9 us instead of 20, those of 24,000 blobs
-// in 12,831 tiles (80 entries) 17.5 us instead of 41.
-template <int E>
-__device__ __forceinline__ void sort_by_rank(unsigned long long* __restrict__ list, int n, unsigned* keys) {
-  const int lane = threadIdx.x & 31;
+// The same order, by T threads (a warp or a CTA of 128): E entries per thread, each placed by
+// its rank, the number of smaller blob ids in the tile (read four at a time from shared
+// memory, padded with ids above all others).  No step waits for another, as those of a
+// bitonic sort do: the lists of 2048 rods at 256^3 (15 entries) take 9.9 us instead of 20,
+// those of 24,000 blobs in 12,831 tiles (80 entries) 17.5 us instead of 41.
+template <int E, int T>
+__device__ __forceinline__ void sort_by_rank(unsigned long long* list, int n, unsigned* keys) {
+  const int lane = threadIdx.x & (T - 1);
   unsigned long long e[E];
   int r[E];
 #pragma unroll
   for (int i = 0; i < E; ++i) {
-    e[i] = lane + 32 * i < n ? list[lane + 32 * i] : ~0ull;
-    keys[lane + 32 * i] = (unsigned)(e[i] >> 32);
+    e[i] = lane + T * i < n ? list[lane + T * i] : ~0ull;
+    keys[lane + T * i] = (unsigned)(e[i] >> 32);
     r[i] = 0;
   }
-  __syncwarp();  // every entry read before the first is written
+  if constexpr (T == 32)  // every entry read before the first is written
+    __syncwarp();
+  else
+    __syncthreads();
   for (int k = 0; k < n; k += 4) {
     const uint4 o = *reinterpret_cast<const uint4*>(keys + k);
 #pragma unroll
@@ -353,39 +357,65 @@ __device__ __forceinline__ void sort_by_rank(unsigned long long* __restrict__ li
   }
 #pragma unroll
   for (int i = 0; i < E; ++i)
-    if (lane + 32 * i < n) list[r[i]] = e[i];
+    if (lane + T * i < n) list[r[i]] = e[i];
 }
 
-// 128 threads = four tiles per CTA; tiles with more than TSORT entries are sorted by lane 0
-// in place as k_tile_sort does.
+// Lists of any length, in place by a CTA of 128: a bitonic sort whose comparators all point
+// upwards (the first of each merge pairs i with its mirror image), so that the places past
+// the end, larger than all entries, never move and need not exist.
+__device__ __forceinline__ void sort_bitonic(unsigned long long* list, int n) {
+  for (long long k = 2; k < 2LL * n; k <<= 1)
+    for (long long j = k >> 1; j > 0; j >>= 1) {
+      const int x = (int)(2 * j == k ? k - 1 : j);
+      for (int i = threadIdx.x; i < n; i += 128) {
+        const int l = i ^ x;
+        if (l > i && l < n) {
+          const unsigned long long u = list[i], v = list[l];
+          if (u > v) {
+            list[i] = v;
+            list[l] = u;
+          }
+        }
+      }
+      __syncthreads();
+    }
+}
+
+// A warp per tile, four tiles per CTA, for lists of up to TSORT entries; longer ones (dense
+// suspensions on coarse grids) by the CTA, one after the other: set-up of 3000 blobs in a
+// 64^3 grid (up to 700 entries) 45 us, 1340 us by an insertion sort in one lane.
 constexpr int TSORT = 256;
 __global__ void __launch_bounds__(128) k_tile_sort_warp(BinTables bt, int ntiles) {
   chain_begin();
   const bool second = blockIdx.y != 0;
   const int* __restrict__ offset = second ? bt.offset[1] : bt.offset[0];
-  unsigned long long* __restrict__ list = second ? bt.list[1] : bt.list[0];
+  unsigned long long* list = second ? bt.list[1] : bt.list[0];
   const long long cap = second ? bt.g[1].list_cap : bt.g[0].list_cap;
   __shared__ __align__(16) unsigned keys[4][TSORT];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * 4 + w;
-  if (t >= ntiles) return;  // uniform over the warp
-  const int b = offset[t], e = offset[t + 1], n = e - b;
-  if (!FCM_INB(b, (long long)e + 1, BS_LIST) || !FCM_INB(e, cap + 1, BS_LIST)) return;  // uniform over the warp
-  if (n < 2) return;
-  if (n <= 32) return sort_by_rank<1>(list + b, n, keys[w]);
-  if (n <= 64) return sort_by_rank<2>(list + b, n, keys[w]);
-  if (n <= 128) return sort_by_rank<4>(list + b, n, keys[w]);
-  if (n <= TSORT) return sort_by_rank<8>(list + b, n, keys[w]);
-  if (lane == 0)
-    for (int i = b + 1; i < e; ++i) {
-      const unsigned long long v = list[i];
-      int j = i - 1;
-      while (j >= b && list[j] > v) {
-        list[j + 1] = list[j];
-        --j;
-      }
-      list[j + 1] = v;
-    }
+  auto range = [&](int t, int& b) -> int {  // entries of tile t from b on
+    b = 0;
+    if (t >= ntiles) return 0;
+    b = offset[t];
+    const int e = offset[t + 1];
+    return FCM_INB(b, (long long)e + 1, BS_LIST) && FCM_INB(e, cap + 1, BS_LIST) ? e - b : 0;
+  };
+  const int w = threadIdx.x >> 5, t0 = blockIdx.x * 4;
+  int b;
+  int n = range(t0 + w, b);
+  if (n > 1 && n <= 32) sort_by_rank<1, 32>(list + b, n, keys[w]);
+  else if (n > 32 && n <= 64) sort_by_rank<2, 32>(list + b, n, keys[w]);
+  else if (n > 64 && n <= 128) sort_by_rank<4, 32>(list + b, n, keys[w]);
+  else if (n > 128 && n <= TSORT) sort_by_rank<8, 32>(list + b, n, keys[w]);
+  if (!__syncthreads_or(n > TSORT)) return;
+  for (int i = 0; i < 4; ++i) {  // uniform over the CTA
+    n = range(t0 + i, b);
+    if (n <= TSORT) continue;
+    if (n <= 4 * TSORT)
+      sort_by_rank<8, 128>(list + b, n, keys[0]);
+    else
+      sort_bitonic(list + b, n);
+    __syncthreads();  // the keys are used again
+  }
 }
 
 // Eight consecutive T from global (aligned to 8*sizeof(T)) to shared memory.
