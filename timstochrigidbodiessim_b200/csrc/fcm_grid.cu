@@ -135,14 +135,17 @@ __global__ void k_set_up_gaussians(const double* __restrict__ Y, int n, int W, d
   }
 }
 
-// (blob, tile) overlaps of a blob: per dimension the tiles first..first+cnt-1.
+// (blob, tile) overlaps of a blob: per dimension the tiles first..first+cnt-1, at most NCH.
+// A position that is infinite or 2^31 grid points away saturates: its stencil's last point is
+// past the largest int, and the counts (as the weights there) are zero, whatever the
+// wrapped-around sum is.
 __device__ __forceinline__ void blob_tiles(const int* base, int b, const TileGeom& g, int f[3], int cnt[3]) {
   const int n[3] = {g.nx, g.ny, g.nz}, nt[3] = {g.ntx, g.nty, g.ntz}, q[3] = {g.qx, g.qy, g.qz};
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const int lo = base[3 * b + d];
     f[d] = tile_of(lo, n[d], nt[d], q[d]);
-    cnt[d] = tile_of(lo + g.W - 1, n[d], nt[d], q[d]) - f[d] + 1;
+    cnt[d] = min(max(tile_of((int)((unsigned)lo + g.W - 1u), n[d], nt[d], q[d]) - f[d] + 1, 0), NCH);
   }
 }
 
@@ -2007,7 +2010,7 @@ __device__ __forceinline__ void interp_reduce_one(const int* __restrict__ base, 
   int f[3], cnt[3];
   blob_tiles(base, b, g, f, cnt);
   int nj = cnt[0] * cnt[1] * cnt[2];
-  if (!FCM_INB(nj - 1, 64, BS_PARTIAL)) nj = 0;
+  if (!FCM_INB(nj, 65, BS_PARTIAL)) nj = 0;
   double s0 = 0, s1 = 0, s2 = 0;
   const T* p = partial + (size_t)b * 64 * 3;
   for (int j = 0; j < nj; ++j) {
@@ -2041,7 +2044,7 @@ __device__ __forceinline__ void interp_reduce8(const int* __restrict__ base, con
     int f[3], cnt[3];
     blob_tiles(base, b, g, f, cnt);
     int nj = cnt[0] * cnt[1] * cnt[2];
-    if (!FCM_INB(nj - 1, 64, BS_PARTIAL)) nj = 0;
+    if (!FCM_INB(nj, 65, BS_PARTIAL)) nj = 0;
     const T* p = partial + (size_t)b * 64 * 3;
     for (int j = k; j < nj; j += 8) {
       s0 += (double)p[3 * j];
@@ -2712,7 +2715,7 @@ __global__ void k_interp_dipole_reduce(const int* __restrict__ base, const T* __
   int f[3], cnt[3];
   blob_tiles(base, b, g, f, cnt);
   int nj = cnt[0] * cnt[1] * cnt[2];
-  if (!FCM_INB(nj - 1, 64, BS_PARTIAL)) nj = 0;
+  if (!FCM_INB(nj, 65, BS_PARTIAL)) nj = 0;
   double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   const T* p = partial9 + (size_t)b * 64 * 9;
   for (int j = 0; j < nj; ++j)
