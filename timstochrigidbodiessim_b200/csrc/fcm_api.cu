@@ -2165,17 +2165,16 @@ int build_batch_graph(Batch* B) {
 // Whether a solve of precision P projects inside its x-transform kernel.
 bool projects_in_x(const Ctx& c, int P) { return c.xfft[P] || use_packed(c, P); }
 
-// Member i's spectrum in the batched kernels: its own part of the group's array, or, on
-// the packed half spectrum (all of a group's grids transformed as one array), its share
-// of that.
+// Member i's spectrum in the batched kernels, which transform all of a group's grids as one
+// array: its share of that, as long as the transforms make it (a member's own spectrum,
+// for what it does alone, starts every spectrum_size values instead, the larger layout's).
 template <typename T>
-void* batch_spec(const Batch* B, Ctx* c, int i) {
+void* batch_spec(const Batch* B, const Ctx* c, int i) {
   constexpr int P = sizeof(T) == 8 ? 0 : 1;
-  if (!use_packed(*c, P)) return grid_of<T>(c).c;
+  const size_t len = use_packed(*c, P) ? (size_t)packed_spectrum_size<T>(*c) : 3 * (size_t)c->g.Gc;
   for (const BatchGroup& g : B->groups)
     for (size_t j = 0; j < g.idx.size(); ++j)
-      if (g.idx[j] == i)
-        return (typename cplx_t<T>::type*)g.c[P] + j * (size_t)packed_spectrum_size<T>(*c);
+      if (g.idx[j] == i) return (typename cplx_t<T>::type*)g.c[P] + j * len;
   return nullptr;
 }
 
