@@ -2215,6 +2215,21 @@ int persistent_ctas(K kernel, int threads, int device) {
 // CTAs of k_tile_count and k_tile_fill (64 candidate tiles per blob, 128 threads).
 static unsigned tile_bin_ctas(int n) { return (unsigned)(((long long)n + 1) / 2); }
 
+// Few blobs on an uneven grid beyond the L2 (126 MB): the tiles write every row in pieces that
+// end inside 32-byte sectors, which memory has to complete, unless the rows are whole sectors
+// and only the last tiles of each are 7 points long.  The per-blob kernels (a fill and the
+// atomics of each blob) are then faster, up to about one blob per 32 tiles in FP64 and 14 in
+// FP32 (us, spread + interpolation, per blob / tiles: FP64 1000 blobs at 250^3 233 / 273, 2000
+// 375 / 286, 450 at 186^3 99 / 107; FP32 1500 at 250^3 109 / 160, 3000 175 / 167, 600 at 210^3
+// 47 / 64, 1500 at 230^3 95 / 122).  Where the rows are whole sectors a small margin is left
+// to set-up, which has no lists to make (60 blobs at 300^3 in FP64 129 / 180, 450 192 / 232).
+template <typename T>
+static bool per_blob(int n, long long ntiles, const GridDims& g) {
+  if (3 * g.G * (long long)sizeof(T) < 105'000'000) return false;
+  const bool sectors = g.nz * sizeof(T) % 32 == 0;
+  return (sectors ? 200LL : sizeof(T) == 8 ? 32LL : 14LL) * n < ntiles;
+}
+
 template <typename T>
 int blob_table_alloc(BlobTable<T>& t, int n, int W, const GridDims& g) {
   if (t.n == n && t.W == W && t.base) return FCM_OK;
@@ -2227,7 +2242,8 @@ int blob_table_alloc(BlobTable<T>& t, int n, int W, const GridDims& g) {
   const bool fits = W + TE <= g.nx && W + TE <= g.ny && W + TE <= g.nz && W <= MAXW && n < (1 << 30);
   const TileGeom tg = tile_geom(g, W, n, 0);
   t.tiled = fits && g.nx % TE == 0 && g.ny % TE == 0 && g.nz % TE == 0;
-  t.uneven = fits && !t.tiled && W <= MAXW_UNEVEN && tg.qx >= 0 && tg.qy >= 0 && tg.qz >= 0;
+  t.uneven = fits && !t.tiled && W <= MAXW_UNEVEN && tg.qx >= 0 && tg.qy >= 0 && tg.qz >= 0 &&
+             !per_blob<T>(n, (long long)tg.ntx * tg.nty * tg.ntz, g);
   if (t.binned()) {
     t.ntx = tg.ntx;
     t.nty = tg.nty;
@@ -2400,15 +2416,22 @@ static int launch_interp_tiles(const Ctx& c, const BlobTable<T>& t, const T* gri
                         c.g.G, t.partial);
 }
 
+// Few blobs on an uneven grid: a CTA per blob is faster than the tiles' longest list and the
+// walk over the tiles without blobs (us, per blob / tiles: FP32 60 blobs 6.2 / 8.4, 240 in a
+// 42^3 grid 6.4 / 12.3, 450 at 62^3 8 / 12, 600 at 90^3 10 / 10, 1000 at 150^3 13 / 16, 2000 at
+// 186^3 24 / 27, 3000 at 250^3 46 / 52, 4500 65 / 56; FP64, from 16^3 tiles on, 60 at 126^3 13 /
+// 16, 450 at 162^3 26 / 35, 1000 at 210^3 60 / 69, 1500 at 250^3 93 / 104, 3000 160 / 113).
+template <typename T>
+static bool few_on_uneven(const BlobTable<T>& t) {
+  if (!t.uneven) return false;
+  return sizeof(T) == 4 ? 12LL * (t.n - 600) < t.ntiles : t.ntiles >= 4096 && 16LL * t.n < t.ntiles;
+}
+
 template <typename T>
 int launch_interp(const Ctx& c, const BlobTable<T>& t, const T* grid, double* dV, cudaStream_t s) {
   if (t.n == 0) return FCM_OK;
   const double dx3 = c.g.dx * c.g.dx * c.g.dx;
-  // few blobs in FP32 on an uneven grid: a CTA per blob, at two per SM still faster than
-  // the tiles' longest list (60 blobs 6.2 against 8.4 us, 240 in a 42^3 grid 6.4 against
-  // 12.3, 360 level, 1500 level, 4200 22.8 against 17.8)
-  const bool few = sizeof(T) == 4 && t.uneven && t.n <= 300;
-  if (t.binned() && !few) {
+  if (t.binned() && !few_on_uneven(t)) {
     TileGeom g;
     FCM_TRY(launch_interp_tiles<T>(c, t, grid, g, s));
     FCM_TRY(launch_chained(k_interp_reduce8<T>, dim3((t.n + 15) / 16), dim3(128), 0, s, t.base, t.partial, t.n, g, dx3,
@@ -2424,7 +2447,9 @@ int launch_interp(const Ctx& c, const BlobTable<T>& t, const T* grid, double* dV
 template <typename T>
 int launch_saddle_end(const Ctx& c, const BlobTable<T>& t, const T* grid, const double* qm, const double* in,
                       double* out, cudaStream_t s) {
-  if (t.n == 0 || !t.binned()) {
+  // (two launches more than the tiles' end: a mixed step of 40 rods at 42^3 1000 -> 983 us, 75 at
+  // 62^3 1535 -> 1512, 100 at 126^3 2775 -> 2756)
+  if (t.n == 0 || !t.binned() || few_on_uneven(t)) {
     FCM_TRY(launch_interp<T>(c, t, grid, out, s));
     FCM_TRY(launch_multiply_K(c, qm, in + 3 * (size_t)c.Nb, out, 1.0, s));
     return launch_multiply_KT(c, qm, in, out + 3 * (size_t)c.Nb, -1.0, nullptr, 0.0, s);
