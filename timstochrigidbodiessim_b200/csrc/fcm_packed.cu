@@ -72,6 +72,8 @@ __global__ void __launch_bounds__(NT) k_packed_z(C* __restrict__ real, C* __rest
     return real + (((long long)mc * t.nxb * XB + XB * xb + p % XB) * t.ny + line_y(p)) * H;
   };
   auto spec_line = [&](int p) { return spec + t.row(mc, XB * xb + p % XB, line_y(p)); };
+  [[maybe_unused]] const long long comps = gridDim.x / ((unsigned)nyb * t.nxb);  // components of all members
+  [[maybe_unused]] const long long nreal = comps * t.nxb * XB * t.ny * H, nspec = comps / 3 * t.size();
   for (int i = threadIdx.x; i < Q * Z2; i += NT) {
     int p = i / Z2, n2 = i % Z2;
     if (INV) tile_item<TKB, Q, Z2>(i, p, n2);
@@ -81,11 +83,13 @@ __global__ void __launch_bounds__(NT) k_packed_z(C* __restrict__ real, C* __rest
       const C* src = spec_line(p);
       const ColRun<C, XB, Z2, Z1> col(t, n2);
 #pragma unroll
-      for (int j = 0; j < Z1; ++j) a[j] = ldt<T>(src[col.at(j)]);
+      for (int j = 0; j < Z1; ++j)
+        a[j] = FCM_INB(src + col.at(j) - spec, nspec, BS_SPECTRUM) ? ldt<T>(src[col.at(j)]) : V2<T>{(T)0, (T)0};
     } else {
       const C* src = real_line(p) + n2;
 #pragma unroll
-      for (int j = 0; j < Z1; ++j) a[j] = ldt<T>(src[j * Z2]);
+      for (int j = 0; j < Z1; ++j)
+        a[j] = FCM_INB(src + j * Z2 - real, nreal, BS_GRID) ? ldt<T>(src[j * Z2]) : V2<T>{(T)0, (T)0};
     }
     dft<T, Z1, INV>(a);
 #pragma unroll
@@ -112,7 +116,8 @@ __global__ void __launch_bounds__(NT) k_packed_z(C* __restrict__ real, C* __rest
       C o;
       o.x = b[j].x;
       o.y = b[j].y;
-      dst[INV ? (long long)(Z1 * j) : col.at(j)] = o;
+      const long long at = INV ? (long long)(Z1 * j) : col.at(j);
+      if (INV ? FCM_INB(dst + at - real, nreal, BS_GRID) : FCM_INB(dst + at - spec, nspec, BS_SPECTRUM)) dst[at] = o;
     }
   }
 }
@@ -121,17 +126,22 @@ __global__ void __launch_bounds__(NT) k_packed_z(C* __restrict__ real, C* __rest
 // Transforms along y in place: one CTA per tile column, XB x times TKB columns at once in
 // a contiguous run of 128 ny bytes, the two steps as above.
 template <typename T, typename C, int Y1, int Y2, int NT, bool INV>
-__global__ void __launch_bounds__(NT) k_packed_y(C* __restrict__ spec, const C* __restrict__ tw) {
+__global__ void __launch_bounds__(NT) k_packed_y(C* __restrict__ spec, const C* __restrict__ tw,
+                                                 [[maybe_unused]] long long nspec) {
   chain_begin();
   constexpr int TK = 128 / (int)sizeof(C);  // values per tile
   extern __shared__ __align__(16) unsigned char packed_smem[];
   V2<T>* s = reinterpret_cast<V2<T>*>(packed_smem);  // [Y1 Y2][TK]
   C* base = spec + (long long)blockIdx.x * (Y1 * Y2 * TK);
+  auto in = [&](int i) { return FCM_INB(base + i - spec, nspec, BS_SPECTRUM); };
   for (int i = threadIdx.x; i < Y2 * TK; i += NT) {
     const int kzl = i % TK, n2 = i / TK;
     V2<T> a[Y1];
 #pragma unroll
-    for (int j = 0; j < Y1; ++j) a[j] = ldt<T>(base[(j * Y2 + n2) * TK + kzl]);
+    for (int j = 0; j < Y1; ++j) {
+      const int at = (j * Y2 + n2) * TK + kzl;
+      a[j] = in(at) ? ldt<T>(base[at]) : V2<T>{(T)0, (T)0};
+    }
     dft<T, Y1, INV>(a);
 #pragma unroll
     for (int j = 1; j < Y1; ++j) {
@@ -153,7 +163,7 @@ __global__ void __launch_bounds__(NT) k_packed_y(C* __restrict__ spec, const C* 
       C o;
       o.x = b[j].x;
       o.y = b[j].y;
-      base[(k1 + Y1 * j) * TK + kzl] = o;
+      if (in((k1 + Y1 * j) * TK + kzl)) base[(k1 + Y1 * j) * TK + kzl] = o;
     }
   }
 }
@@ -174,12 +184,16 @@ __global__ void __launch_bounds__(NT) k_packed_plane(C* __restrict__ real, C* __
   const int nx = XB * t.nxb;
   C* sp = spec + t.row(blockIdx.x / nx, blockIdx.x % nx, 0);
   constexpr int TS = Tiles<C, XB>::TS;  // values from one y to the next
+  [[maybe_unused]] const long long nreal = (long long)gridDim.x * N * H, nspec = gridDim.x / (3u * nx) * t.size();
   if constexpr (!INV) {
     for (int i = threadIdx.x; i < N * Z2; i += NT) {
       const int y = i / Z2, n2 = i % Z2;
       V2<T> a[Z1];
 #pragma unroll
-      for (int j = 0; j < Z1; ++j) a[j] = ldt<T>(plane[y * H + j * Z2 + n2]);
+      for (int j = 0; j < Z1; ++j) {
+        const int at = y * H + j * Z2 + n2;
+        a[j] = FCM_INB(plane + at - real, nreal, BS_GRID) ? ldt<T>(plane[at]) : V2<T>{(T)0, (T)0};
+      }
       dft<T, Z1, false>(a);
 #pragma unroll
       for (int j = 1; j < Z1; ++j) a[j] = cmul(a[j], ldt<T>(__ldg(&twz[2 * n2 * j])));
@@ -222,7 +236,7 @@ __global__ void __launch_bounds__(NT) k_packed_plane(C* __restrict__ real, C* __
         C o;
         o.x = b[j].x;
         o.y = b[j].y;
-        dst[(k1 + Y1 * j) * TS] = o;
+        if (FCM_INB(dst + (k1 + Y1 * j) * TS - spec, nspec, BS_SPECTRUM)) dst[(k1 + Y1 * j) * TS] = o;
       }
     }
   } else {
@@ -231,7 +245,10 @@ __global__ void __launch_bounds__(NT) k_packed_plane(C* __restrict__ real, C* __
       const C* src = sp + t.col(kz);
       V2<T> a[Y1];
 #pragma unroll
-      for (int j = 0; j < Y1; ++j) a[j] = ldt<T>(src[(j * Y2 + n2) * TS]);
+      for (int j = 0; j < Y1; ++j) {
+        const int at = (j * Y2 + n2) * TS;
+        a[j] = FCM_INB(src + at - spec, nspec, BS_SPECTRUM) ? ldt<T>(src[at]) : V2<T>{(T)0, (T)0};
+      }
       dft<T, Y1, true>(a);
 #pragma unroll
       for (int j = 1; j < Y1; ++j) a[j] = cmulc(a[j], ldt<T>(__ldg(&twy[n2 * j])));
@@ -273,7 +290,7 @@ __global__ void __launch_bounds__(NT) k_packed_plane(C* __restrict__ real, C* __
         C o;
         o.x = b[j].x;
         o.y = b[j].y;
-        plane[y * H + k1 + Z1 * j] = o;
+        if (FCM_INB(plane + y * H + k1 + Z1 * j - real, nreal, BS_GRID)) plane[y * H + k1 + Z1 * j] = o;
       }
     }
   }
@@ -318,7 +335,8 @@ int packed_y(const Ctx& c, typename cplx_t<T>::type* spec, int members, cudaStre
     auto kern = k_packed_y<T, C, Y1, Y2, NT, INV>;
     FCM_TRY(smem_attr_once(kern, smem));
     const long long per = packed_spectrum_size<T>(c) / ((long long)Y1 * Y2 * (128 / (int)sizeof(C)));  // tile columns
-    return launch_chained(kern, dim3((unsigned)(per * members)), dim3(NT), smem, s, spec, ytw<T>(c));
+    return launch_chained(kern, dim3((unsigned)(per * members)), dim3(NT), smem, s, spec, ytw<T>(c),
+                          (long long)members * packed_spectrum_size<T>(c));
   });
 }
 
