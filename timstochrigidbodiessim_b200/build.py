@@ -31,12 +31,27 @@ CFLAGS = GENCODE + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O3",
                     "-I" + os.path.join(ROOT, "include")]
 
 
-def _sources():
-    return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
+# The packed transforms' kernels, an object (and so a module, loaded on its own) per precision
+# and class of lengths: see fcm_packed.cuh.
+_PACKED = [("f%d_%d" % (8 * size, c), ["-DFCM_PACKED_T=" + t, "-DFCM_PACKED_CLASS=%d" % c])
+           for t, size in (("double", 8), ("float", 4)) for c in range(3)]
+INSTANCES = {
+    "fcm_packed_zy.cu": _PACKED,
+    "fcm_packed_x.cu": [(tag, defs + (["-DFCM_PACKED_NOISE"] if tag.startswith("f64") else [])) for tag, defs in _PACKED]
+    + [("batch_" + tag, defs + ["-DFCM_PACKED_BATCH=1"]) for tag, defs in _PACKED],
+}
 
 
-def _compile(src, extra, out_dir=BUILD):
-    obj = os.path.join(out_dir, os.path.basename(src) + ".o")
+def _units():
+    """(source, tag, defines) of every object, the long compilations first."""
+    units = []
+    for src in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        units += [(src, tag, defs) for tag, defs in INSTANCES.get(os.path.basename(src), [("", [])])]
+    return sorted(units, key=lambda u: not u[1])
+
+
+def _compile(src, tag, extra, out_dir=BUILD):
+    obj = os.path.join(out_dir, os.path.basename(src) + ("." + tag if tag else "") + ".o")
     if (os.path.exists(obj) and os.path.getmtime(obj) > os.path.getmtime(src)
             and all(os.path.getmtime(obj) > os.path.getmtime(h)
                     for h in glob.glob(os.path.join(CSRC, "*.cuh")) + [os.path.join(ROOT, "include", "fcm_b200.h")])):
@@ -50,9 +65,9 @@ def _compile(src, extra, out_dir=BUILD):
 
 def _build_lib(lib, out_dir, extra, verbose):
     os.makedirs(out_dir, exist_ok=True)
-    srcs = _sources()
-    with cf.ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
-        results = list(ex.map(lambda s: _compile(s, extra, out_dir), srcs))
+    units = _units()
+    with cf.ThreadPoolExecutor(max_workers=8) as ex:
+        results = list(ex.map(lambda u: _compile(u[0], u[1], extra + u[2], out_dir), units))
     objs = [o for o, _ in results]
     if verbose:
         for _, log in results:
@@ -72,7 +87,7 @@ def build(verbose=False, ptxas_info=False, bounds_check=True):
     extra = ["-Xptxas", "-v"] if ptxas_info else []
     _build_lib(LIB, BUILD, extra, verbose)
     if bounds_check:
-        _build_lib(DEBUG_LIB, DEBUG_BUILD, extra + ["-DFCM_BOUNDS_CHECK"], verbose)
+        _build_lib(DEBUG_LIB, DEBUG_BUILD, extra + ["-DFCM_BOUNDS_CHECK", "-Xfatbin=-compress-all"], verbose)
     _build_host()
     return LIB
 

@@ -398,8 +398,9 @@ int setup_xfft(Ctx* c) {
   c->packed_cap = packed_lengths(c->g.nx, c->g.ny, c->g.nz);
   c->packed_variant = c->packed_cap && ok && xfft_factor(c->g.ny, &n1, &n2) && xfft_factor(c->g.nz, &n1, &n2);
   c->packed32 = c->packed_variant;
-  if (ok) FCM_TRY(xfft_tables_init());
-  if (c->packed_cap) FCM_TRY(packed_tables_init());
+  // (FP64 never takes the fused x-transform where it has the packed solve)
+  if (ok && (!c->packed_cap || c->p.precision == 1)) FCM_TRY(xfft_tables_init());
+  if (c->packed_cap) FCM_TRY(packed_tables_init(*c));
   const double PI = 3.14159265358979323846264338327950288;
   const int sides[3] = {c->g.nx, c->g.ny, c->g.nz};
   void** const d64[3] = {&c->d_xtw64, &c->d_ytw64, &c->d_ztw64};
@@ -2209,6 +2210,7 @@ int rehome_grids(Batch* B, int P) {
     FCM_CUFFT(cufftPlanMany(&grp.r2c[P], 3, nn, nullptr, 1, (int)G, nullptr, 1, (int)Gc, r2c_type<T>(), (int)(3 * k)));
     FCM_CUFFT(cufftPlanMany(&grp.c2r[P], 3, nn, nullptr, 1, (int)Gc, nullptr, 1, (int)G, c2r_type<T>(), (int)(3 * k)));
     const bool packed = use_packed(*c0, P);
+    if (packed) FCM_TRY(b_packed_init<T>(*c0));
     if (c0->xfft[P] && !packed) {
       int n2[2] = {grp.ny, grp.nz};
       const int pz = grp.ny * grp.nz, pc = grp.ny * (grp.nz / 2 + 1), planes = (int)(3 * grp.nx * k);
@@ -2700,7 +2702,7 @@ int fcm_debug_bounds(int32_t* checked, int64_t* count, int32_t* site, int64_t* i
     const int on = 0;
 #endif
     int (*readers[])(BoundsRecord*, int) = {bounds_read_grid, bounds_read_cells, bounds_read_kspace,
-                                            bounds_read_packed, bounds_read_packed_x, bounds_read_blas};
+                                            bounds_read_packed, bounds_read_blas};
     unsigned long long total = 0;
     BoundsRecord first{};
     for (auto rd : readers) {

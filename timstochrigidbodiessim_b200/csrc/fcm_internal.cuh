@@ -161,8 +161,7 @@ static __device__ __forceinline__ bool fcm_inb(long long i, long long n, int sit
 int bounds_read_grid(BoundsRecord* out, int reset);
 int bounds_read_cells(BoundsRecord* out, int reset);
 int bounds_read_kspace(BoundsRecord* out, int reset);
-int bounds_read_packed(BoundsRecord* out, int reset);
-int bounds_read_packed_x(BoundsRecord* out, int reset);
+int bounds_read_packed(BoundsRecord* out, int reset);  // all modules of the packed passes
 int bounds_read_blas(BoundsRecord* out, int reset);
 
 template <typename T>
@@ -606,8 +605,9 @@ template <typename T>
 int launch_xfft_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s);
 // the packed half-spectrum solve (fcm_packed.cu) of `members` consecutive grids of c's
 // shape: (y, z) transforms, x transforms with the projection, inverse (y, z) transforms
-int packed_tables_init();
-int packed_zy_tables_init();  // by packed_tables_init
+int packed_tables_init(const Ctx& c);  // of the modules that c's passes are in
+template <typename T>
+int b_packed_init(const Ctx& c0);  // of the module of a batch group's x pass
 bool packed_lengths(int nx, int ny, int nz);  // whether the packed solve takes this grid
 template <typename T>
 long long packed_spectrum_size(const Ctx& c);  // complex values of one grid's spectrum

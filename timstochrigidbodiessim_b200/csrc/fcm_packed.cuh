@@ -1,5 +1,6 @@
 // fcm_packed.cuh -- layout, lengths and launch helpers of the Stokes solve on a packed half
-// spectrum (fcm_packed.cu: z and y passes, fcm_packed_x.cu: x passes).
+// spectrum (fcm_packed_zy.cu: z and y passes, fcm_packed_x.cu: x passes, fcm_packed.cu: the
+// choice among them).
 //
 // A real line of nz points is transformed along z as H = nz/2 complex points (even
 // samples the real, odd ones the imaginary parts) and nothing else is done to it:
@@ -25,7 +26,7 @@
 // writes one contiguous run of 128 ny bytes, and the z passes write whole tiles, XB x of
 // a row per CTA.  The columns j < H/2 fill the blocks 0..nkb - 1 in order, H/2 (where it is a
 // whole number) the first place of block nkb and H - j (0 < j < H/2) place j from there: the
-// two columns of a pair lie nkb blocks apart.  Lengths: those of with_length.
+// two columns of a pair lie nkb blocks apart.  Lengths: PACKED_LENGTHS.
 //
 // Measured per solve against the separate passes on nz/2 + 1 columns with cuFFT's 3D or
 // (y, z) plans in FP64 (us, FP64 / FP32): 64^3 29 / 20 (43 / 25), 96^3 60 / 35 (101 / 43),
@@ -43,6 +44,44 @@
 #include "fcm_internal.cuh"
 
 namespace fcm {
+
+// The sources of the passes are compiled once per precision and class of lengths (build.py):
+// each object is a module of its own, which the driver loads when a context first needs it.
+// As one module per source the first context of a process took 100 ms at 64^3 in FP64 and
+// 110 ms at 256^3 in mixed precision instead of 15 and 40, and the library 79 s to build
+// instead of 54.
+constexpr int PACKED_CLASSES = 3;
+constexpr int length_class(int n) { return n <= 96 ? 0 : n <= 216 ? 1 : 2; }
+
+template <typename T, int CL>
+int packed_zy_init();  // the tables of the module, before its first launch
+template <typename T, int CL>
+int packed_z_pass(const Ctx& c, typename cplx_t<T>::type* real, typename cplx_t<T>::type* spec, int members,
+                  bool inverse, cudaStream_t s);
+template <typename T, int CL>
+int packed_y_pass(const Ctx& c, typename cplx_t<T>::type* spec, int members, bool inverse, cudaStream_t s);
+template <typename T>
+int packed_plane_pass(const Ctx& c, typename cplx_t<T>::type* real, typename cplx_t<T>::type* spec, int members,
+                      bool inverse, cudaStream_t s);  // class 0
+template <typename T, int CL>
+int packed_x_init();
+template <typename T, int CL>
+int packed_x_pass(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s);
+template <int CL>
+int packed_noise_pass(const Ctx& c, cufftDoubleComplex* spec, uint64_t seed, uint64_t counter, const uint64_t* d_args,
+                      cudaStream_t s);
+template <typename T, int CL>
+int b_packed_x_init();
+template <typename T, int CL>
+int b_packed_x_pass(const BatchGeom& b, const Ctx& c0, const int* gidx, int nm, int mask, cudaStream_t s);
+
+// The bounds records of the modules, by 2 * class + (1 in FP32).
+template <int ID>
+int bounds_read_packed_zy(BoundsRecord* out, int reset);
+template <int ID>
+int bounds_read_packed_x(BoundsRecord* out, int reset);
+template <int ID>
+int bounds_read_b_packed_x(BoundsRecord* out, int reset);
 
 namespace {
 
@@ -75,144 +114,40 @@ struct Tiles {
 // 258 us), 4 else (32-byte sectors in the z passes).
 __host__ __device__ constexpr int tile_x(int nx) { return nx >= 256 ? 8 : 4; }
 
-// Calls f(integral_constant<N1>, integral_constant<N2>) with the two register DFT sizes of
-// length n along y: the even numbers with factors 2, 3, 5 and 7 from 32 to 320 whose
-// register sizes stay within 20 points, and a few smaller and longer ones.
-template <typename F>
-int with_length(int n, F&& f) {
-  using std::integral_constant;
-  switch (n) {
-    case 8: return f(integral_constant<int, 2>{}, integral_constant<int, 4>{});
-    case 12: return f(integral_constant<int, 3>{}, integral_constant<int, 4>{});
-    case 16: return f(integral_constant<int, 4>{}, integral_constant<int, 4>{});
-    case 24: return f(integral_constant<int, 4>{}, integral_constant<int, 6>{});
-    case 32: return f(integral_constant<int, 4>{}, integral_constant<int, 8>{});
-    case 36: return f(integral_constant<int, 6>{}, integral_constant<int, 6>{});
-    case 40: return f(integral_constant<int, 5>{}, integral_constant<int, 8>{});
-    case 42: return f(integral_constant<int, 6>{}, integral_constant<int, 7>{});
-    case 48: return f(integral_constant<int, 6>{}, integral_constant<int, 8>{});
-    case 50: return f(integral_constant<int, 5>{}, integral_constant<int, 10>{});
-    case 54: return f(integral_constant<int, 6>{}, integral_constant<int, 9>{});
-    case 56: return f(integral_constant<int, 7>{}, integral_constant<int, 8>{});
-    case 60: return f(integral_constant<int, 6>{}, integral_constant<int, 10>{});
-    case 64: return f(integral_constant<int, 8>{}, integral_constant<int, 8>{});
-    case 70: return f(integral_constant<int, 7>{}, integral_constant<int, 10>{});
-    case 72: return f(integral_constant<int, 8>{}, integral_constant<int, 9>{});
-    case 80: return f(integral_constant<int, 8>{}, integral_constant<int, 10>{});
-    case 84: return f(integral_constant<int, 7>{}, integral_constant<int, 12>{});
-    case 90: return f(integral_constant<int, 9>{}, integral_constant<int, 10>{});
-    case 96: return f(integral_constant<int, 8>{}, integral_constant<int, 12>{});
-    case 98: return f(integral_constant<int, 7>{}, integral_constant<int, 14>{});
-    case 100: return f(integral_constant<int, 10>{}, integral_constant<int, 10>{});
-    case 108: return f(integral_constant<int, 9>{}, integral_constant<int, 12>{});
-    case 112: return f(integral_constant<int, 8>{}, integral_constant<int, 14>{});
-    case 120: return f(integral_constant<int, 10>{}, integral_constant<int, 12>{});
-    case 126: return f(integral_constant<int, 9>{}, integral_constant<int, 14>{});
-    case 128: return f(integral_constant<int, 8>{}, integral_constant<int, 16>{});
-    case 140: return f(integral_constant<int, 10>{}, integral_constant<int, 14>{});
-    case 144: return f(integral_constant<int, 12>{}, integral_constant<int, 12>{});
-    case 150: return f(integral_constant<int, 10>{}, integral_constant<int, 15>{});
-    case 160: return f(integral_constant<int, 10>{}, integral_constant<int, 16>{});
-    case 162: return f(integral_constant<int, 9>{}, integral_constant<int, 18>{});
-    case 168: return f(integral_constant<int, 12>{}, integral_constant<int, 14>{});
-    case 180: return f(integral_constant<int, 12>{}, integral_constant<int, 15>{});
-    case 192: return f(integral_constant<int, 12>{}, integral_constant<int, 16>{});
-    case 196: return f(integral_constant<int, 14>{}, integral_constant<int, 14>{});
-    case 200: return f(integral_constant<int, 10>{}, integral_constant<int, 20>{});
-    case 210: return f(integral_constant<int, 14>{}, integral_constant<int, 15>{});
-    case 216: return f(integral_constant<int, 12>{}, integral_constant<int, 18>{});
-    case 224: return f(integral_constant<int, 14>{}, integral_constant<int, 16>{});
-    case 240: return f(integral_constant<int, 15>{}, integral_constant<int, 16>{});
-    case 252: return f(integral_constant<int, 14>{}, integral_constant<int, 18>{});
-    case 256: return f(integral_constant<int, 16>{}, integral_constant<int, 16>{});
-    case 270: return f(integral_constant<int, 15>{}, integral_constant<int, 18>{});
-    case 280: return f(integral_constant<int, 14>{}, integral_constant<int, 20>{});
-    case 288: return f(integral_constant<int, 16>{}, integral_constant<int, 18>{});
-    case 300: return f(integral_constant<int, 15>{}, integral_constant<int, 20>{});
-    case 320: return f(integral_constant<int, 16>{}, integral_constant<int, 20>{});
-    case 384: return f(integral_constant<int, 16>{}, integral_constant<int, 24>{});
-    case 400: return f(integral_constant<int, 20>{}, integral_constant<int, 20>{});
-    case 480: return f(integral_constant<int, 20>{}, integral_constant<int, 24>{});
-    case 512: return f(integral_constant<int, 16>{}, integral_constant<int, 32>{});
-    default: break;
-  }
-  set_error("packed transforms: unsupported length " + std::to_string(n));
-  return FCM_ERR_INVALID;
-}
-// The same along x: whole tiles.
+// The lengths: the even numbers with factors 2, 3, 5 and 7 from 32 to 320 whose register DFT
+// sizes stay within 20 points, and a few smaller and longer ones.  n1 n2 = n along x (whole
+// tiles only) and y, h1 h2 = n / 2 along z.
+struct PackedLength {
+  int n, n1, n2, h1, h2;
+};
+constexpr PackedLength PACKED_LENGTHS[] = {
+    {8, 2, 4, 2, 2}, {12, 3, 4, 2, 3}, {16, 4, 4, 2, 4}, {24, 4, 6, 3, 4}, {32, 4, 8, 4, 4}, {36, 6, 6, 3, 6},
+    {40, 5, 8, 4, 5}, {42, 6, 7, 3, 7}, {48, 6, 8, 4, 6}, {50, 5, 10, 5, 5}, {54, 6, 9, 3, 9}, {56, 7, 8, 4, 7},
+    {60, 6, 10, 5, 6}, {64, 8, 8, 4, 8}, {70, 7, 10, 5, 7}, {72, 8, 9, 6, 6}, {80, 8, 10, 5, 8}, {84, 7, 12, 6, 7},
+    {90, 9, 10, 5, 9}, {96, 8, 12, 6, 8}, {98, 7, 14, 7, 7}, {100, 10, 10, 5, 10}, {108, 9, 12, 6, 9},
+    {112, 8, 14, 7, 8}, {120, 10, 12, 6, 10}, {126, 9, 14, 7, 9}, {128, 8, 16, 8, 8}, {140, 10, 14, 7, 10},
+    {144, 12, 12, 8, 9}, {150, 10, 15, 5, 15}, {160, 10, 16, 8, 10}, {162, 9, 18, 9, 9}, {168, 12, 14, 7, 12},
+    {180, 12, 15, 9, 10}, {192, 12, 16, 8, 12}, {196, 14, 14, 7, 14}, {200, 10, 20, 10, 10}, {210, 14, 15, 7, 15},
+    {216, 12, 18, 9, 12}, {224, 14, 16, 8, 14}, {240, 15, 16, 10, 12}, {252, 14, 18, 9, 14}, {256, 16, 16, 8, 16},
+    {270, 15, 18, 9, 15}, {280, 14, 20, 10, 14}, {288, 16, 18, 12, 12}, {300, 15, 20, 10, 15},
+    {320, 16, 20, 10, 16}, {384, 16, 24, 12, 16}, {400, 20, 20, 10, 20}, {480, 20, 24, 15, 16},
+    {512, 16, 32, 16, 16}};
+constexpr int NUM_PACKED_LENGTHS = sizeof(PACKED_LENGTHS) / sizeof(PACKED_LENGTHS[0]);
+
+// Whether a length is taken along x: whole tiles.
 constexpr bool x_length(int n) { return n % tile_x(n) == 0; }
-template <typename F>
-int with_length_x(int n, F&& f) {
-  return with_length(n, [&](auto a, auto b) -> int {
-    if constexpr (x_length(decltype(a)::value * decltype(b)::value)) {
-      return f(a, b);
-    } else {
-      set_error("packed transforms: unsupported length along x");
-      return FCM_ERR_INVALID;
-    }
-  });
-}
-// The same for half a length (the z transforms).
-template <typename F>
-int with_half_length(int h, F&& f) {
-  using std::integral_constant;
-  switch (h) {
-    case 4: return f(integral_constant<int, 2>{}, integral_constant<int, 2>{});
-    case 6: return f(integral_constant<int, 2>{}, integral_constant<int, 3>{});
-    case 8: return f(integral_constant<int, 2>{}, integral_constant<int, 4>{});
-    case 12: return f(integral_constant<int, 3>{}, integral_constant<int, 4>{});
-    case 16: return f(integral_constant<int, 4>{}, integral_constant<int, 4>{});
-    case 18: return f(integral_constant<int, 3>{}, integral_constant<int, 6>{});
-    case 20: return f(integral_constant<int, 4>{}, integral_constant<int, 5>{});
-    case 21: return f(integral_constant<int, 3>{}, integral_constant<int, 7>{});
-    case 24: return f(integral_constant<int, 4>{}, integral_constant<int, 6>{});
-    case 25: return f(integral_constant<int, 5>{}, integral_constant<int, 5>{});
-    case 27: return f(integral_constant<int, 3>{}, integral_constant<int, 9>{});
-    case 28: return f(integral_constant<int, 4>{}, integral_constant<int, 7>{});
-    case 30: return f(integral_constant<int, 5>{}, integral_constant<int, 6>{});
-    case 32: return f(integral_constant<int, 4>{}, integral_constant<int, 8>{});
-    case 35: return f(integral_constant<int, 5>{}, integral_constant<int, 7>{});
-    case 36: return f(integral_constant<int, 6>{}, integral_constant<int, 6>{});
-    case 40: return f(integral_constant<int, 5>{}, integral_constant<int, 8>{});
-    case 42: return f(integral_constant<int, 6>{}, integral_constant<int, 7>{});
-    case 45: return f(integral_constant<int, 5>{}, integral_constant<int, 9>{});
-    case 48: return f(integral_constant<int, 6>{}, integral_constant<int, 8>{});
-    case 49: return f(integral_constant<int, 7>{}, integral_constant<int, 7>{});
-    case 50: return f(integral_constant<int, 5>{}, integral_constant<int, 10>{});
-    case 54: return f(integral_constant<int, 6>{}, integral_constant<int, 9>{});
-    case 56: return f(integral_constant<int, 7>{}, integral_constant<int, 8>{});
-    case 60: return f(integral_constant<int, 6>{}, integral_constant<int, 10>{});
-    case 63: return f(integral_constant<int, 7>{}, integral_constant<int, 9>{});
-    case 64: return f(integral_constant<int, 8>{}, integral_constant<int, 8>{});
-    case 70: return f(integral_constant<int, 7>{}, integral_constant<int, 10>{});
-    case 72: return f(integral_constant<int, 8>{}, integral_constant<int, 9>{});
-    case 75: return f(integral_constant<int, 5>{}, integral_constant<int, 15>{});
-    case 80: return f(integral_constant<int, 8>{}, integral_constant<int, 10>{});
-    case 81: return f(integral_constant<int, 9>{}, integral_constant<int, 9>{});
-    case 84: return f(integral_constant<int, 7>{}, integral_constant<int, 12>{});
-    case 90: return f(integral_constant<int, 9>{}, integral_constant<int, 10>{});
-    case 96: return f(integral_constant<int, 8>{}, integral_constant<int, 12>{});
-    case 98: return f(integral_constant<int, 7>{}, integral_constant<int, 14>{});
-    case 100: return f(integral_constant<int, 10>{}, integral_constant<int, 10>{});
-    case 105: return f(integral_constant<int, 7>{}, integral_constant<int, 15>{});
-    case 108: return f(integral_constant<int, 9>{}, integral_constant<int, 12>{});
-    case 112: return f(integral_constant<int, 8>{}, integral_constant<int, 14>{});
-    case 120: return f(integral_constant<int, 10>{}, integral_constant<int, 12>{});
-    case 126: return f(integral_constant<int, 9>{}, integral_constant<int, 14>{});
-    case 128: return f(integral_constant<int, 8>{}, integral_constant<int, 16>{});
-    case 135: return f(integral_constant<int, 9>{}, integral_constant<int, 15>{});
-    case 140: return f(integral_constant<int, 10>{}, integral_constant<int, 14>{});
-    case 144: return f(integral_constant<int, 12>{}, integral_constant<int, 12>{});
-    case 150: return f(integral_constant<int, 10>{}, integral_constant<int, 15>{});
-    case 160: return f(integral_constant<int, 10>{}, integral_constant<int, 16>{});
-    case 192: return f(integral_constant<int, 12>{}, integral_constant<int, 16>{});
-    case 200: return f(integral_constant<int, 10>{}, integral_constant<int, 20>{});
-    case 240: return f(integral_constant<int, 15>{}, integral_constant<int, 16>{});
-    case 256: return f(integral_constant<int, 16>{}, integral_constant<int, 16>{});
-    default: break;
+
+// Calls f(integral_constant<I>) for the entry I of length n among those of class CL.
+template <int CL, int I = 0, typename F>
+int with_length(int n, F&& f) {
+  if constexpr (I == NUM_PACKED_LENGTHS) {
+    set_error("packed transforms: unsupported length " + std::to_string(n));
+    return FCM_ERR_INVALID;
+  } else {
+    if constexpr (length_class(PACKED_LENGTHS[I].n) == CL)
+      if (n == PACKED_LENGTHS[I].n) return f(std::integral_constant<int, I>{});
+    return with_length<CL, I + 1>(n, f);
   }
-  set_error("packed transforms: unsupported half length " + std::to_string(h));
-  return FCM_ERR_INVALID;
 }
 
 // Dynamic shared memory above the default 48 KB for `kernel`, set once per kernel

@@ -1,7 +1,17 @@
 // fcm_packed_x.cu -- x passes of the Stokes solve on a packed half spectrum: forward
-// transform, projection and inverse transform, and the draw of the fluctuating field.
+// transform, projection and inverse transform, and the draw of the fluctuating field, for
+// one precision and class of lengths per object (build.py), a batch's kernels in objects of
+// their own.
 #include "fcm_fluct.cuh"
 #include "fcm_packed.cuh"
+
+#ifndef FCM_PACKED_T
+#define FCM_PACKED_T double
+#define FCM_PACKED_CLASS 0
+#endif
+#ifndef FCM_PACKED_BATCH
+#define FCM_PACKED_BATCH 0
+#endif
 
 namespace fcm {
 
@@ -311,70 +321,91 @@ constexpr int px_min() {
   return N <= 128 || (sizeof(T) == 8 && N <= 216) ? 4 : N == 256 ? (sizeof(T) == 4 ? 8 : 5) : sizeof(T) == 4 ? 4 : N <= 256 ? 3 : 4;
 }
 
-template <typename T>
-int packed_x(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s, const BatchGeom* b, const int* gidx, int nm,
-             int mask) {
-  using C = typename cplx_t<T>::type;
-  constexpr int P = sizeof(T) == 8 ? 0 : 1;
-  return with_length_x(c.g.nx, [&](auto a, auto d) -> int {
-    constexpr int N1 = decltype(a)::value, N2 = decltype(d)::value, N = N1 * N2;
-    constexpr int TK = px_tk<T, N>(), NT = px_threads<T, N>(), MB = px_min<T, N>();
-    constexpr size_t smem = XShape<C, N1, N2, TK>::SMEM;
-    const int pairs = (c.g.nz / 2 + 1) / 2;
-    const dim3 grid((unsigned)((pairs + TK - 1) / TK), (unsigned)c.g.ny, (unsigned)(b ? nm : 1));
-    if (b) {
-      auto kern = k_b_packed_x<T, C, P, N1, N2, TK, NT, MB>;
-      FCM_TRY(smem_attr_once(kern, smem));
-      return launch_chained(kern, grid, dim3(NT), smem, s, b->mem, gidx, mask, xtw<T>(c), ztw<T>(c));
+using Real = FCM_PACKED_T;
+using Cplx = cplx_t<Real>::type;
+constexpr int CLASS = FCM_PACKED_CLASS;
+
+// Calls f(kernel of this length's sizes, threads, shared memory, grid of nm members).
+template <typename F>
+int with_x_length(const Ctx& c, int nm, F&& f) {
+  return with_length<CLASS>(c.g.nx, [&](auto l) -> int {
+    constexpr PackedLength L = PACKED_LENGTHS[decltype(l)::value];
+    if constexpr (x_length(L.n)) {
+      constexpr int TK = px_tk<Real, L.n>();
+      const int pairs = (c.g.nz / 2 + 1) / 2;
+      return f(l, XShape<Cplx, L.n1, L.n2, TK>::SMEM,
+               dim3((unsigned)((pairs + TK - 1) / TK), (unsigned)c.g.ny, (unsigned)nm));
     } else {
-      auto kern = k_packed_x<T, C, N1, N2, TK, NT, MB>;
-      FCM_TRY(smem_attr_once(kern, smem));
-      return launch_chained(kern, grid, dim3(NT), smem, s, spec, make_kparams(c), xtw<T>(c), ztw<T>(c));
+      set_error("packed transforms: unsupported length along x");
+      return FCM_ERR_INVALID;
     }
   });
 }
 
 }  // namespace
 
-int packed_tables_init() {
-  FCM_TRY(packed_zy_tables_init());
+#if FCM_PACKED_BATCH
+
+template <>
+int b_packed_x_init<Real, CLASS>() {
   return roots_upload();
 }
-
-template <typename T>
-int launch_packed_project(const Ctx& c, typename cplx_t<T>::type* spec, cudaStream_t s) {
-  return packed_x<T>(c, spec, s, nullptr, nullptr, 0, 0);
+template <>
+int b_packed_x_pass<Real, CLASS>(const BatchGeom& b, const Ctx& c0, const int* gidx, int nm, int mask,
+                                 cudaStream_t s) {
+  return with_x_length(c0, nm, [&](auto l, size_t smem, dim3 grid) -> int {
+    constexpr PackedLength L = PACKED_LENGTHS[decltype(l)::value];
+    constexpr int NT = px_threads<Real, L.n>();
+    auto kern = k_b_packed_x<Real, Cplx, sizeof(Real) == 8 ? 0 : 1, L.n1, L.n2, px_tk<Real, L.n>(), NT,
+                             px_min<Real, L.n>()>;
+    FCM_TRY(smem_attr_once(kern, smem));
+    return launch_chained(kern, grid, dim3(NT), smem, s, b.mem, gidx, mask, xtw<Real>(c0), ztw<Real>(c0));
+  });
 }
 
-// The fluctuating velocity field of (seed, counter), or d_args[0..1] where given, into r.
-int launch_packed_noise(const Ctx& c, cufftDoubleComplex* spec, double* r, uint64_t seed, uint64_t counter,
-                        const uint64_t* d_args, cudaStream_t s) {
-  using T = double;
-  using C = cufftDoubleComplex;
+template <>
+FCM_BOUNDS_READER(bounds_read_b_packed_x<2 * CLASS + (sizeof(Real) == 4)>)
+
+#else
+
+template <>
+int packed_x_init<Real, CLASS>() {
+  return roots_upload();
+}
+template <>
+int packed_x_pass<Real, CLASS>(const Ctx& c, Cplx* spec, cudaStream_t s) {
+  return with_x_length(c, 1, [&](auto l, size_t smem, dim3 grid) -> int {
+    constexpr PackedLength L = PACKED_LENGTHS[decltype(l)::value];
+    constexpr int NT = px_threads<Real, L.n>();
+    auto kern = k_packed_x<Real, Cplx, L.n1, L.n2, px_tk<Real, L.n>(), NT, px_min<Real, L.n>()>;
+    FCM_TRY(smem_attr_once(kern, smem));
+    return launch_chained(kern, grid, dim3(NT), smem, s, spec, make_kparams(c), xtw<Real>(c), ztw<Real>(c));
+  });
+}
+
+// FP64 only: the spectrum of the fluctuating velocity field.
+template <int CL>
+int packed_noise_pass(const Ctx& c, cufftDoubleComplex* spec, uint64_t seed, uint64_t counter, const uint64_t* d_args,
+                      cudaStream_t s) {
   NoiseArgs na{seed, counter, d_args, 0.0, 0.0};
   stress_amplitudes(c, na.amp_diag, na.amp_off);
-  FCM_TRY(with_length_x(c.g.nx, [&](auto a, auto d) -> int {
-    constexpr int N1 = decltype(a)::value, N2 = decltype(d)::value, N = N1 * N2;
-    constexpr int TK = px_tk<T, N>(), NT = px_threads<T, N>(), MB = px_min<T, N>();
-    constexpr size_t smem = XShape<C, N1, N2, TK>::SMEM;
-    const dim3 grid((unsigned)(((c.g.nz / 2 + 1) / 2 + TK - 1) / TK), (unsigned)c.g.ny);
-    auto kern = k_packed_noise<T, C, N1, N2, TK, NT, MB>;
+  return with_x_length(c, 1, [&](auto l, size_t smem, dim3 grid) -> int {
+    constexpr PackedLength L = PACKED_LENGTHS[decltype(l)::value];
+    constexpr int NT = px_threads<double, L.n>();
+    auto kern = k_packed_noise<double, cufftDoubleComplex, L.n1, L.n2, px_tk<double, L.n>(), NT,
+                               px_min<double, L.n>()>;
     FCM_TRY(smem_attr_once(kern, smem));
-    return launch_chained(kern, grid, dim3(NT), smem, s, spec, make_kparams(c), xtw<T>(c), ztw<T>(c), na);
-  }));
-  return launch_packed_inverse<T>(c, spec, r, 1, s);
+    return launch_chained(kern, grid, dim3(NT), smem, s, spec, make_kparams(c), xtw<double>(c), ztw<double>(c), na);
+  });
 }
+#ifdef FCM_PACKED_NOISE
+template int packed_noise_pass<CLASS>(const Ctx&, cufftDoubleComplex*, uint64_t, uint64_t, const uint64_t*,
+                                      cudaStream_t);
+#endif
 
-template <typename T>
-int b_packed_project(const BatchGeom& b, const Ctx& c0, const int* gidx, int nm, int mask, cudaStream_t s) {
-  return packed_x<T>(c0, nullptr, s, &b, gidx, nm, mask);
-}
+template <>
+FCM_BOUNDS_READER(bounds_read_packed_x<2 * CLASS + (sizeof(Real) == 4)>)
 
-template int launch_packed_project<double>(const Ctx&, cufftDoubleComplex*, cudaStream_t);
-template int launch_packed_project<float>(const Ctx&, cufftComplex*, cudaStream_t);
-template int b_packed_project<double>(const BatchGeom&, const Ctx&, const int*, int, int, cudaStream_t);
-template int b_packed_project<float>(const BatchGeom&, const Ctx&, const int*, int, int, cudaStream_t);
-
-FCM_BOUNDS_READER(bounds_read_packed_x)
+#endif
 
 }  // namespace fcm
