@@ -426,12 +426,36 @@ int setup_xfft(Ctx* c) {
 }
 
 // Complex values of a grid's spectrum: cuFFT's three half spectra or the packed layout,
-// whichever is larger (the packed one for 8 and 12 points along z, padded to whole tiles).
+// whichever is larger (the packed one where nz/2 columns are far from whole tiles: 8, 12, 36,
+// 42, 50 points along z and others).
 template <typename T>
 size_t spectrum_size(const Ctx& c) {
   const size_t n = 3 * (size_t)c.g.Gc;
   return c.packed_cap ? std::max(n, (size_t)packed_spectrum_size<T>(c)) : n;
 }
+
+// cuFFT's 3D transforms of the grid's three components, each when first asked for (not while
+// a stream is captured).
+template <typename T>
+int ensure_r2c(Ctx* c) {
+  GridBufs<T>& gb = grid_of<T>(c);
+  if (gb.r2c) return FCM_OK;
+  int n[3] = {c->g.nx, c->g.ny, c->g.nz};
+  FCM_CUFFT(cufftPlanMany(&gb.r2c, 3, n, nullptr, 1, (int)c->g.G, nullptr, 1, (int)c->g.Gc, r2c_type<T>(), 3));
+  FCM_CUFFT(cufftSetStream(gb.r2c, c->stream));
+  return FCM_OK;
+}
+template <typename T>
+int ensure_c2r(Ctx* c) {
+  GridBufs<T>& gb = grid_of<T>(c);
+  if (gb.c2r) return FCM_OK;
+  int n[3] = {c->g.nx, c->g.ny, c->g.nz};
+  FCM_CUFFT(cufftPlanMany(&gb.c2r, 3, n, nullptr, 1, (int)c->g.Gc, nullptr, 1, (int)c->g.G, c2r_type<T>(), 3));
+  FCM_CUFFT(cufftSetStream(gb.c2r, c->stream));
+  return FCM_OK;
+}
+
+int noise_precision(const Ctx* c);
 
 template <typename T>
 int ensure_grid(Ctx* c) {
@@ -441,14 +465,14 @@ int ensure_grid(Ctx* c) {
   FCM_TRY(dev_alloc(&gb.c, spectrum_size<T>(*c)));
   FCM_TRY(dev_alloc(&gb.urand, 3 * (size_t)c->g.G));
   FCM_CUDA(cudaMemsetAsync(gb.urand, 0, sizeof(T) * 3 * (size_t)c->g.G, c->stream));
-  int n[3] = {c->g.nx, c->g.ny, c->g.nz};
-  FCM_CUFFT(cufftPlanMany(&gb.r2c, 3, n, nullptr, 1, (int)c->g.G, nullptr, 1, (int)c->g.Gc, r2c_type<T>(), 3));
-  FCM_CUFFT(cufftPlanMany(&gb.c2r, 3, n, nullptr, 1, (int)c->g.Gc, nullptr, 1, (int)c->g.G, c2r_type<T>(), 3));
-  FCM_CUFFT(cufftSetStream(gb.r2c, c->stream));
-  FCM_CUFFT(cufftSetStream(gb.c2r, c->stream));
+  // The 3D transforms (their work areas take 6.5 GB at 512^3 in FP64) where a solve variant runs
+  // them; the inverse also for the FP32 noise (injected stress asks for it by itself).
+  constexpr int P = sizeof(T) == 8 ? 0 : 1;
+  if (!packed_always(*c, P)) FCM_TRY(ensure_r2c<T>(c));
+  if (!packed_always(*c, P) || (P == 1 && noise_precision(c) == 1)) FCM_TRY(ensure_c2r<T>(c));
   // cuFFT's (y, z) transforms of the 3 nx planes, for the fused x-transform on grids
   // without the packed solve and for FP32 variant 1 beside it
-  if (c->xfft_cap[sizeof(T) == 8 ? 0 : 1] && (!c->packed_cap || (sizeof(T) == 4 && c->packed_variant))) {
+  if (c->xfft_cap[P] && (!c->packed_cap || (P == 1 && c->packed_variant))) {
     int n2[2] = {c->g.ny, c->g.nz};
     const int planes = 3 * c->g.nx;
     FCM_CUFFT(cufftPlanMany(&gb.r2c2d, 2, n2, nullptr, 1, c->g.ny * c->g.nz, nullptr, 1, c->g.ny * c->g.nzh,
@@ -484,14 +508,14 @@ void free_grid(GridBufs<T>& gb) {
 
 int set_stream_all(Ctx* c) {
   if (c->g64.ready) {
-    FCM_CUFFT(cufftSetStream(c->g64.r2c, c->stream));
-    FCM_CUFFT(cufftSetStream(c->g64.c2r, c->stream));
+    if (c->g64.r2c) FCM_CUFFT(cufftSetStream(c->g64.r2c, c->stream));
+    if (c->g64.c2r) FCM_CUFFT(cufftSetStream(c->g64.c2r, c->stream));
     if (c->g64.r2c2d) FCM_CUFFT(cufftSetStream(c->g64.r2c2d, c->stream));
     if (c->g64.c2r2d) FCM_CUFFT(cufftSetStream(c->g64.c2r2d, c->stream));
   }
   if (c->g32.ready) {
-    FCM_CUFFT(cufftSetStream(c->g32.r2c, c->stream));
-    FCM_CUFFT(cufftSetStream(c->g32.c2r, c->stream));
+    if (c->g32.r2c) FCM_CUFFT(cufftSetStream(c->g32.r2c, c->stream));
+    if (c->g32.c2r) FCM_CUFFT(cufftSetStream(c->g32.c2r, c->stream));
     if (c->g32.r2c2d) FCM_CUFFT(cufftSetStream(c->g32.r2c2d, c->stream));
     if (c->g32.c2r2d) FCM_CUFFT(cufftSetStream(c->g32.c2r2d, c->stream));
   }
@@ -592,6 +616,8 @@ int noise_dev(Ctx* c, uint64_t seed, uint64_t counter, const uint64_t* d_args = 
   return FCM_OK;
 }
 
+// Condition of a GMRES while-loop: go on while the solve is not done, for at
+// most `limit` iterations of this loop.
 __global__ void k_gm_loop_cond(cudaGraphConditionalHandle h, const GmState* __restrict__ gm, StepRecord* sd,
                                int enter, int limit) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
@@ -862,8 +888,6 @@ int divU_dev(Ctx* c, double* out) {
 // The per-step inputs (noise seed and step index) are read from device memory.
 // Built once per context, after a host-driven step has allocated every buffer.
 
-// Condition of a GMRES while-loop: go on while the solve is not done, for at
-// most `limit` iterations of this loop.
 __global__ void k_step_begin(StepRecord* sd) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   sd->iters = 0;
@@ -2161,8 +2185,6 @@ int build_batch_graph(Batch* B) {
   return st;
 }
 
-// The members' grids of precision T moved into one contiguous array per group
-// of equal grids, with one cuFFT plan per group over all of them.
 // Whether a solve of precision P projects inside its x-transform kernel.
 bool projects_in_x(const Ctx& c, int P) { return c.xfft[P] || use_packed(c, P); }
 
@@ -2179,6 +2201,8 @@ void* batch_spec(const Batch* B, const Ctx* c, int i) {
   return nullptr;
 }
 
+// The members' grids of precision T moved into one contiguous array per group
+// of equal grids, with one cuFFT plan per group over all of them where its solve uses cuFFT.
 template <typename T>
 int rehome_grids(Batch* B, int P) {
   for (BatchGroup& grp : B->groups) {
@@ -2207,11 +2231,13 @@ int rehome_grids(Batch* B, int P) {
       gb.borrowed = true;
     }
     int nn[3] = {grp.nx, grp.ny, grp.nz};
-    FCM_CUFFT(cufftPlanMany(&grp.r2c[P], 3, nn, nullptr, 1, (int)G, nullptr, 1, (int)Gc, r2c_type<T>(), (int)(3 * k)));
-    FCM_CUFFT(cufftPlanMany(&grp.c2r[P], 3, nn, nullptr, 1, (int)Gc, nullptr, 1, (int)G, c2r_type<T>(), (int)(3 * k)));
     const bool packed = use_packed(*c0, P);
-    if (packed) FCM_TRY(b_packed_init<T>(*c0));
-    if (c0->xfft[P] && !packed) {
+    if (packed) {
+      FCM_TRY(b_packed_init<T>(*c0));
+    } else if (!c0->xfft[P]) {
+      FCM_CUFFT(cufftPlanMany(&grp.r2c[P], 3, nn, nullptr, 1, (int)G, nullptr, 1, (int)Gc, r2c_type<T>(), (int)(3 * k)));
+      FCM_CUFFT(cufftPlanMany(&grp.c2r[P], 3, nn, nullptr, 1, (int)Gc, nullptr, 1, (int)G, c2r_type<T>(), (int)(3 * k)));
+    } else {
       int n2[2] = {grp.ny, grp.nz};
       const int pz = grp.ny * grp.nz, pc = grp.ny * (grp.nz / 2 + 1), planes = (int)(3 * grp.nx * k);
       FCM_CUFFT(cufftPlanMany(&grp.r2c2d[P], 2, n2, nullptr, 1, pz, nullptr, 1, pc, r2c_type<T>(), planes));
@@ -3030,6 +3056,7 @@ int fcm_inject_random_stress(fcm_ctx* ctx, const double* sxx, const double* syy,
         set_error("null stress array");
         return (int)FCM_ERR_INVALID;
       }
+    FCM_TRY(ensure_c2r<double>(c));
     if (!c->d_stress) {
       FCM_TRY(dev_alloc(&c->d_stress, 6 * (size_t)c->g.G));
       FCM_TRY(dev_alloc(&c->d_stress_c, 6 * (size_t)c->g.Gc));

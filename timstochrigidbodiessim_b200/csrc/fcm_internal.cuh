@@ -435,6 +435,9 @@ inline bool use_packed(const Ctx& c, int P) {
   return c.xfft[0] || c.g.nx > 256;
 }
 
+// Whether it does in every solve variant the grid allows, so that no variant needs cuFFT.
+inline bool packed_always(const Ctx& c, int P) { return c.packed_cap && (!c.xfft_cap[P] || (P == 0 && c.g.nx > 256)); }
+
 // ------------------------------------------------------------------ batches
 // One member suspension of a batch as the batched kernels see it (a device
 // array, one entry per member; blockIdx.y or .z selects the member).
