@@ -1,6 +1,7 @@
 """Grids whose solve is the packed one in every variant (an x length of its own, or FP64 beyond
 256 points along x): no cuFFT plan is made for them (its work areas doubled the memory of
-the spectrum), injected stress, which needs one, makes it when it comes."""
+the spectrum), injected stress, which needs one, makes it when it comes, and the autotuner
+times the one path once and keeps variant 0."""
 import numpy as np
 import pytest
 import torch
@@ -58,3 +59,14 @@ def test_injected_stress(gpu, n):
             i[d] = n[d] // 2
             A[tuple(i)] = B[tuple(i)] = 0
         assert rel_err(np.stack([A.real, A.imag]), np.stack([B.real, B.imag])) < 1e-11
+
+
+@pytest.mark.parametrize("n, P", [((384, 16, 16), 0), ((40, 48, 48), 0), ((40, 48, 48), 1)])
+def test_autotune_times_one_path_once(gpu, n, P):
+    g = Suspension(_params(n, precision=1), [0, 0, 0])
+    g.set_up_gaussians(np.linspace(0.0, 15.0, 30))
+    for _ in range(3):
+        v, us = g.autotune(reps=3)
+        t = us[16 * P + 6:16 * P + 9]
+        assert v[2 * P + 1] == 0 and t[0] > 0
+        assert all(x in (-1.0, t[0]) for x in t[1:])

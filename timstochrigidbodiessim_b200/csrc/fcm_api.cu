@@ -2663,6 +2663,10 @@ static int tune_precision(Ctx* c, int reps, double* t) {
   FCM_CUDA(cudaMemsetAsync(gb.r, 0, sizeof(T) * 3 * (size_t)c->g.G, c->stream));
   for (int v = 0; v < 3; ++v) {
     if ((v >= 1 && !c->xfft_cap[P]) || (v == 2 && (P == 0 || !c->packed_variant))) continue;
+    if (v > 0 && packed_always(*c, P)) {  // the path of variant 0, timed once: ties go to it
+      t[6 + v] = t[6];
+      continue;
+    }
     c->xfft[P] = v >= 1;
     if (P == 1) c->packed32 = v == 2;
     FCM_TRY(time_calls(c, reps, [&] { return stokes_t<T>(c); }, &t[6 + v]));
