@@ -307,18 +307,31 @@ __global__ void __launch_bounds__(NT, MINB) k_b_packed_x(const BMember* __restri
 // only other CTAs fill the gaps (49 KB of pencils and four CTAs at 512 points).  In FP64
 // 192 threads leave 96 registers, which spill: 128 threads up to 216 points (solve at 200
 // points 426 -> 402 us, 160 195 -> 186), above which five of their CTAs no longer fit (240
-// points 671 -> 708 us).
+// points 671 -> 708 us).  From 256 points on, where a CTA has half the columns: us of a solve
+// with 256 x 256 points along y and z, by 96 threads (FP64 five CTAs, FP32 eight), 128 (four,
+// six) and beyond that 96 in FP64 (four CTAs) and 192 in FP32 (four):
+//   FP64  256 758 763 771   280 873 865 877   288 905 889 902   320 1041 969 987   384 1200 1173 1142
+//   FP32  256 380 381 377   280 454 444 454   288 462 449 460   320 507 492 508    384 595 585 577
+// (400, 480 and 512 as 384), so the first below 280 points, the second to 320.
 template <typename T, int N>
 constexpr int px_tk() {
   return 64 / (int)sizeof(T) / tile_x(N);
 }
 template <typename T, int N>
 constexpr int px_threads() {
-  return N <= 128 || (sizeof(T) == 8 && N <= 216) ? 128 : N < 256 ? 192 : N == 256 ? 96 : sizeof(T) == 4 ? 192 : 96;
+  if (N <= 128 || (sizeof(T) == 8 && N <= 216)) return 128;
+  if (N < 256) return 192;
+  if (N < 280) return 96;
+  if (N <= 320) return 128;
+  return sizeof(T) == 4 ? 192 : 96;
 }
 template <typename T, int N>
 constexpr int px_min() {
-  return N <= 128 || (sizeof(T) == 8 && N <= 216) ? 4 : N == 256 ? (sizeof(T) == 4 ? 8 : 5) : sizeof(T) == 4 ? 4 : N <= 256 ? 3 : 4;
+  if (N <= 128 || (sizeof(T) == 8 && N <= 216)) return 4;
+  if (N < 256) return sizeof(T) == 4 ? 4 : 3;
+  if (N < 280) return sizeof(T) == 4 ? 8 : 5;
+  if (N <= 320) return sizeof(T) == 4 ? 6 : 4;
+  return 4;
 }
 
 using Real = FCM_PACKED_T;
