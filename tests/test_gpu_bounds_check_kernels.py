@@ -16,7 +16,7 @@ from timstochrigidbodiessim_b200 import capi
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SUITES = ["tests/test_gpu_uneven_tiles.py", "tests/test_gpu_tensor_tiles_fp64.py", "tests/test_gpu_long_tile_lists.py",
           "tests/test_gpu_sparse_interpolation.py", "tests/test_gpu_sparse_uneven.py", "tests/test_gpu_far_positions.py", "tests/test_gpu_packed_solve.py",
-          "tests/test_gpu_small_gmres.py", "tests/test_gpu_gmres_columns.py", "tests/test_gpu_batch_unpacked.py"]
+          "tests/test_gpu_slender_noise.py", "tests/test_gpu_small_gmres.py", "tests/test_gpu_gmres_columns.py", "tests/test_gpu_batch_unpacked.py"]
 
 
 def test_sources_with_a_bounds_record_check_something():

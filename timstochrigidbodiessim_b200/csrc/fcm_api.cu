@@ -466,10 +466,11 @@ int ensure_grid(Ctx* c) {
   FCM_TRY(dev_alloc(&gb.urand, 3 * (size_t)c->g.G));
   FCM_CUDA(cudaMemsetAsync(gb.urand, 0, sizeof(T) * 3 * (size_t)c->g.G, c->stream));
   // The 3D transforms (their work areas take 6.5 GB at 512^3 in FP64) where a solve variant runs
-  // them; the inverse also for the FP32 noise (injected stress asks for it by itself).
+  // them; the inverse also for the noise that it transforms (injected stress asks for it by itself).
   constexpr int P = sizeof(T) == 8 ? 0 : 1;
   if (!packed_always(*c, P)) FCM_TRY(ensure_r2c<T>(c));
-  if (!packed_always(*c, P) || (P == 1 && noise_precision(c) == 1)) FCM_TRY(ensure_c2r<T>(c));
+  const bool noise = noise_precision(c) == P && !(P == 0 && packed_noise(*c));
+  if (!packed_always(*c, P) || noise) FCM_TRY(ensure_c2r<T>(c));
   // cuFFT's (y, z) transforms of the 3 nx planes, for the fused x-transform on grids
   // without the packed solve and for FP32 variant 1 beside it
   if (c->xfft_cap[P] && (!c->packed_cap || (P == 1 && c->packed_variant))) {
@@ -600,7 +601,7 @@ int noise_dev(Ctx* c, uint64_t seed, uint64_t counter, const uint64_t* d_args = 
   // FP64: drawn inside the x pass of the packed spectrum (256^3 617 against 762 us). The
   // FP32 field of a mixed step keeps cuFFT's transform: its roundings are the only FP32
   // ones that no refinement removes, and once a step it is 2% of the time.
-  if (c->packed_cap && noise_precision(c) == 0) {
+  if (packed_noise(*c) && noise_precision(c) == 0) {
     FCM_TRY(launch_packed_noise(*c, c->g64.c, c->g64.urand, seed, counter, d_args, c->stream));
     c->urand_prec = 0;
   } else if (noise_precision(c) == 1) {

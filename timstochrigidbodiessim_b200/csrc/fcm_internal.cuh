@@ -612,6 +612,7 @@ int packed_tables_init(const Ctx& c);  // of the modules that c's passes are in
 template <typename T>
 int b_packed_init(const Ctx& c0);  // of the module of a batch group's x pass
 bool packed_lengths(int nx, int ny, int nz);  // whether the packed solve takes this grid
+bool packed_noise(const Ctx& c);              // and the FP64 fluctuating field, see there
 template <typename T>
 long long packed_spectrum_size(const Ctx& c);  // complex values of one grid's spectrum
 template <typename T>

@@ -53,6 +53,19 @@ bool packed_lengths(int nx, int ny, int nz) {
   return listed(nx) && listed(ny) && listed(nz);
 }
 
+// Whether the FP64 fluctuating field is drawn in the x pass of the packed spectrum.  From 140
+// points along x on, a CTA's draws take 25-45 us however few CTAs there are (a tile's
+// columns of one row each), so slender boxes of less than one and a half CTAs per SM draw the
+// whole half spectrum and take cuFFT's transform (us of a field, cuFFT / packed: 512 x 8 x 8 23
+// / 43, 400 x 24 x 24 29 / 42, 200 x 24 x 24 24 / 30; 240 x 32 x 32 (128 CTAs) 30 / 32, 320 x 32 x 32 (256)
+// 35 / 31, 160 x 42 x 42 (252) 30 / 29, 256 x 40 x 40 (400) 38 / 26).
+bool packed_noise(const Ctx& c) {
+  if (!c.packed_cap) return false;
+  const int tk = 8 / tile_x(c.g.nx), pairs = (c.g.nz / 2 + 1) / 2;
+  const long long ctas = (long long)((pairs + tk - 1) / tk) * c.g.ny;
+  return c.g.nx < 140 || 2 * ctas >= 3 * 148;
+}
+
 int packed_tables_init(const Ctx& c) {
   FCM_TRY(tables_init<double>(c));
   return c.p.precision == 1 ? tables_init<float>(c) : (int)FCM_OK;

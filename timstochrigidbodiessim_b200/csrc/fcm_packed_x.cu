@@ -404,9 +404,12 @@ int packed_noise_pass(const Ctx& c, cufftDoubleComplex* spec, uint64_t seed, uin
   stress_amplitudes(c, na.amp_diag, na.amp_off);
   return with_x_length(c, 1, [&](auto l, size_t smem, dim3 grid) -> int {
     constexpr PackedLength L = PACKED_LENGTHS[decltype(l)::value];
-    constexpr int NT = px_threads<double, L.n>();
+    // the draws need more threads than the transforms (field at 256 x 128 x 128 153 -> 145 us, 512
+    // 366 -> 352)
+    constexpr bool LONG = L.n >= 256;
+    constexpr int NT = LONG ? 128 : px_threads<double, L.n>();
     auto kern = k_packed_noise<double, cufftDoubleComplex, L.n1, L.n2, px_tk<double, L.n>(), NT,
-                               px_min<double, L.n>()>;
+                               LONG ? 4 : px_min<double, L.n>()>;
     FCM_TRY(smem_attr_once(kern, smem));
     return launch_chained(kern, grid, dim3(NT), smem, s, spec, make_kparams(c), xtw<double>(c), ztw<double>(c), na);
   });
