@@ -298,30 +298,33 @@ int fcm_interp(fcm_ctx* ctx, int32_t precision, double* V);
 /* Kernel variants of the grid stages (no reference counterpart).
  * variants[FCM_NUM_VARIANTS]:
  *   [0] FP64 spread, [2] FP32 spread: 0 = the persistent software-pipelined tile
- *       kernel (FP64: by one warp on the FP64 tensor cores, FP32: FMAs), 1 / 2 / 3 = one CTA per 8^3 tile staging 16 / 8 / 32 blobs per
- *       round, 4 = one warp per tile staging 16 blobs per round, two y-rows per
+ *       kernel (FP64: by one warp on the FP64 tensor cores, FP32: FMAs), 1 / 2 / 3 =
+ *       one CTA per 8^3 tile staging 16 / 8 / 32 blobs per round, 4 = one warp per tile staging 16 blobs per round, two y-rows per
  *       lane.  All sum every grid point's blobs in the same order with the same
  *       products, so the grids are the same bit for bit.  FP32 only: 5 = one warp
  *       per tile on the tensor cores (mma.sync with TF32 operands split in two,
  *       3xTF32, FP32 accumulators), equal to the others to FP32 rounding.
  *   [1] FP64 Stokes solve, [3] FP32 Stokes solve: 0 = cuFFT 3D transforms and the
- *       projection kernel (FP64 beyond 256 points along x with three supported lengths:
- *       the library's transforms of variant 1), 1 = the projection fused into the
- *       x-transform, in FP64 with the library's own transforms where all three lengths
- *       are supported, else between cuFFT (y, z) transforms, 2 = the library's own
- *       transforms in FP32.  FP64 defaults to 0 beyond 256 points along x.  The solves
- *       agree within rounding.
+ *       projection kernel, 1 = the projection fused into the x-transform, between cuFFT
+ *       (y, z) transforms or, in FP64 where all three lengths have them, the library's
+ *       own (a packed half spectrum), 2 = the library's own transforms in FP32.
+ *       The library's own also stand in for cuFFT's where they have the three lengths and
+ *       are faster than the variant: for variant 0 in FP64 beyond 256 points along x
+ *       and, in either precision, on grids whose x length the fused x-transform lacks (those
+ *       with factors 5, 7 or 9); for FP32 variant 1 where it lacks the y or z length.
+ *       FP64 reports variant 0 by default beyond 256 points along x.  The solves agree
+ *       within rounding.
  *   [4] FP64 interpolation, [5] FP32 interpolation: 0 = 64 threads per 8^3 tile
  *       with a warp shuffle reduction, 1 = one warp per tile (FP64: on the FP64
  *       tensor cores; FP32: two y-rows per lane, added in the lane, with the shuffle
- *       reduction), 2 = one warp per tile
- *       (two y-rows per thread) with a shared-memory reduction; FP32 only: 3 = one
- *       warp per tile on the tensor cores (3xTF32).  They agree within rounding.
+ *       reduction), 2 = one warp per tile (two y-rows per thread) with a shared-memory
+ *       reduction; FP32 only: 3 = one warp per tile on the tensor cores (3xTF32).
+ *       They agree within rounding.
  * Defaults: spread 0 (FP64) and 4 (FP32), solve 1 (FP64 up to 256 points along
  * x, else 0) and 2 (FP32, where the grid allows, else 1 or 0), interpolation 1.
  * A variant the grid does not allow (solve 1 and 2 need supported lengths, 2 also
  * nz <= 512) or out of range is refused with FCM_ERR_INVALID; the spread and
- * interpolation entries have no effect where the grid is not tiled, the FP32
+ * interpolation entries have no effect where the grid is not cut into whole 8^3 tiles, the FP32
  * entries none in a context without an FP32 grid (they are still range-checked).
  * Step graphs are rebuilt on the next step.  Refused for a context owned by a
  * batch. */
@@ -334,7 +337,8 @@ int fcm_set_variants(fcm_ctx* ctx, const int32_t* variants);
  * FCM_NUM_TUNE_TIMES doubles, [16 P + v] for precision P (0 FP64, 1 FP32): v = 0..5
  * the spread variants, v = 6, 7, 8 the solve variants 0, 1, 2, v = 9..12 the
  * interpolation variants 0..3, in microseconds per call, -1 where not available
- * (FP64 v = 5 and 12, v = 13..15 always); variants (may be NULL) receives the
+ * (FP64 v = 5 and 12, v = 13..15 always); solve variants that run the same transforms
+ * get one time, and the first of them; variants (may be NULL) receives the
  * choice as fcm_get_variants does.
  * Needs set_up_gaussians first; overwrites the grid work arrays, so call it
  * between steps. */

@@ -382,17 +382,16 @@ int fp32_stencil(const Ctx* c) {
   return std::min(c->p.ngauss, std::max(2, 2 * half));
 }
 
-// The fused x-transform path of the Stokes solve (stokes_t) when nx has a kernel
-// and nz is even -- for FP64 only up to 256 points, where it measured faster than
-// the 3D transforms (at 512^3 FP64 it was slower) -- and the twiddles
-// exp(-2 pi i j / nx) of both precisions.
-// The packed half-spectrum solve when its lengths include all three, with the twiddles
-// along y and z.
+// The solve that the grid allows (use_packed says which runs).  The fused x-transform when
+// nx has a kernel and nz is even, in FP64 by default only up to 256 points: beyond, where the
+// grid is not packed, the 3D transforms measured faster.  The packed half-spectrum solve when
+// its lengths include all three.  The twiddles exp(-2 pi i j / n) of both precisions along
+// x, for the packed solve along y and z too.
 int setup_xfft(Ctx* c) {
   int n1 = 0, n2 = 0;
   const bool ok = xfft_factor(c->g.nx, &n1, &n2) && c->g.nz % 2 == 0;
   c->xfft[1] = ok;
-  c->xfft[0] = ok && c->g.nx <= 256;  // FP64 beyond 256 points: the 3D transforms unless tuned
+  c->xfft[0] = ok && c->g.nx <= 256;  // beyond 256 points: variant 0 unless tuned
   c->xfft_cap[0] = ok;
   c->xfft_cap[1] = c->xfft[1];
   c->packed_cap = packed_lengths(c->g.nx, c->g.ny, c->g.nz);

@@ -1,5 +1,5 @@
 // fcm_dft.cuh -- complex pairs, wavenumbers and the in-register DFTs of the transform
-// kernels (fcm_kspace.cu, fcm_packed.cu).
+// kernels (fcm_kspace.cu, fcm_packed_zy.cu, fcm_packed_x.cu).
 #pragma once
 #include <cmath>
 #include <mutex>

@@ -1,5 +1,5 @@
 // fcm_fluct.cuh -- the fluctuating stress drawn in Fourier space and its velocity, one mode
-// at a time (fcm_kspace.cu, fcm_packed.cu).
+// at a time (fcm_kspace.cu, fcm_packed_x.cu).
 #pragma once
 #include "fcm_dft.cuh"
 #include "fcm_internal.cuh"

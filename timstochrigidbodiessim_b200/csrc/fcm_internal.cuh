@@ -117,7 +117,7 @@ enum BoundsSite : int {
   BS_LIST = 4,      // tile-list or cell-list slot against its range or capacity
   BS_PARTIAL = 5,   // per-(blob, tile) partial against its table
   BS_CELL = 6,      // cell id against the cell count
-  BS_SPECTRUM = 7,  // spectrum index against the spectrum's 3 Gc values
+  BS_SPECTRUM = 7,  // spectrum index against the spectrum's values (3 Gc, or the packed layout's)
   BS_KRYLOV = 8,    // Krylov column (GMRES iteration) against the columns allocated
 };
 struct BoundsRecord {
@@ -366,8 +366,9 @@ struct Ctx {
   // shear forcing (fcm_fluid_solver.hpp SHEARING_FORCES fields), allocated when
   // the imposed flow is produced: u_shear 3G (the grid layout of g64.r), Vshear 3Nb
   // fused x-transform of the Stokes solve, per grid precision ([0] FP64, [1] FP32):
-  // on when nx is a supported length and nz is even (FP64 up to 256 points, beyond
-  // which the 3D transforms are faster); twiddles exp(-2 pi i j / nx), j < nx
+  // on when nx is a supported length and nz is even (FP64 by default up to 256 points:
+  // beyond, unpacked grids are faster by the 3D transforms); twiddles exp(-2 pi i j / nx),
+  // j < nx
   bool xfft[2] = {false, false};
   // the packed half-spectrum solve (fcm_packed.cuh): all three lengths among its own;
   // packed_variant where they are among those of the fused x-transform too and solve

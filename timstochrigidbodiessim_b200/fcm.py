@@ -326,15 +326,15 @@ class Suspension:
         return V
 
     # kernel variants: [FP64 spread, FP64 solve, FP32 spread, FP32 solve, FP64
-    # interp, FP32 interp]; spread 0 = persistent pipelined, 1 / 2 / 3 = one CTA
-    # per tile staging 16 / 8 / 32 blobs per round, 4 = one warp per tile (two
-    # y-rows per lane), 5 = one warp per tile on the tensor cores (FP32 only);
-    # solve 0 = cuFFT 3D, 1 = the projection fused into the x-transform, 2 = the
-    # threads per tile, 1 =
-
-    # one warp per tile (two y-rows per lane) with the shuffle reduction, 2 = one
-    # warp per tile with a shared-memory reduction, 3 = one warp per tile on the
-    # tensor cores (FP32 only)
+    # interp, FP32 interp]; spread 0 = persistent pipelined (FP64: one warp per tile
+    # on the FP64 tensor cores), 1 / 2 / 3 = one CTA per tile staging 16 / 8 / 32
+    # blobs per round, 4 = one warp per tile (two y-rows per lane), 5 = one warp per
+    # tile on the tensor cores (FP32 only); solve 0 = cuFFT 3D, 1 = the projection
+    # fused into the x-transform (FP64: the library's own transforms where it has the
+    # lengths), 2 = the library's own transforms (FP32 only); interp 0 = 64 threads
+    # per tile, 1 = one warp per tile (FP64: on the FP64 tensor cores; FP32: two
+    # y-rows per lane, shuffle reduction), 2 = one warp per tile with a shared-memory
+    # reduction, 3 = one warp per tile on the tensor cores (FP32 only)
     NUM_VARIANTS = 6
     NUM_TUNE_TIMES = 32
 
@@ -351,7 +351,8 @@ class Suspension:
         """Time every variant the grids allow and keep the fastest.  Returns
         (variants, us): us[16 P + v] microseconds per call for precision P, v = 0-5
         spread variants, 6, 7, 8 solve variants, 9-12 interpolation variants
-        (-1 where not available; v = 13-15 unused)."""
+        (-1 where not available; v = 13-15 unused; solve variants that run the same
+        transforms have the same time)."""
         us, pu = _out(None, self.NUM_TUNE_TIMES)
         v, pv = _out(None, self.NUM_VARIANTS, np.int32)
         self._c(self.L.fcm_autotune(self.h, reps, pu, pv), "fcm_autotune")
