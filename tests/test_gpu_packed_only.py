@@ -2,6 +2,8 @@
 256 points along x): no cuFFT plan is made for them (its work areas doubled the memory of
 the spectrum), injected stress, which needs one, makes it when it comes, and the autotuner
 times the one path once and keeps variant 0."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -21,6 +23,7 @@ def _params(n, **kw):
 @pytest.mark.parametrize("n", [(512, 128, 128), (200, 200, 200)])
 def test_memory(gpu, n):
     Suspension(_params((64, 64, 64)), [0, 0, 0]).close()
+    gc.collect()  # contexts of earlier tests give their memory back now, not in between
     torch.cuda.empty_cache()
     free = torch.cuda.mem_get_info()[0]
     s = Suspension(_params(n), [0, 0, 0])
